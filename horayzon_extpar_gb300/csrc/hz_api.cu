@@ -135,6 +135,13 @@ struct Buffers {
   Node4* nodes4;     // wide traversal only
   Tri* tris;
   BvhScratch bvh;
+  // profile sweep
+  SweepBuffers sweep;
+  float* cell_f32;
+  int16_t* codes;
+  float* tan_m;
+  int tri_base, cell_base;   // of the domain in the call's arrays (SweepAll)
+  unsigned ref_base;
   // search
   void* order_scratch;
   unsigned* cell_bounds;
@@ -152,7 +159,8 @@ int trace_variant(const hz_options& opt) {
 
 Buffers carve_domain(Carver& c, long long ncell, long long nvert, long long nhori,
                      int grid_type, bool host_io, bool precise = false, bool learned = false,
-                     long long L = 0, bool wide = false, long long svf_part_len = 0) {
+                     long long L = 0, bool wide = false, long long svf_part_len = 0,
+                     bool sweep = false) {
   Buffers b;
   std::memset(&b, 0, sizeof(b));
   const long long max_tri = (grid_type == 0 ? 4 : 6) * nvert;
@@ -180,16 +188,13 @@ Buffers carve_domain(Carver& c, long long ncell, long long nvert, long long nhor
   b.origin_sum = c.take<double>(4);
   b.vert32 = c.take<float>(3 * max_mv);
   b.cell_enu = c.take<double>(3 * ncell);
-  b.cell_frame = c.take<double>(9 * ncell);
-  b.cell_origin = c.take<float>(6 * ncell);
   const long long nt = max_tri > 0 ? max_tri : 1;
-  b.nodes = c.take<Node>(nt > 1 ? nt - 1 : 1);
-  if (wide) b.nodes4 = c.take<Node4>(nt > 1 ? nt - 1 : 1);
-  b.tris = c.take<Tri>(nt);
-  if (precise) {
-    b.vert_lo = c.take<float>(3 * max_mv);
-    b.tri_lo = c.take<float4>(3 * nt);
+  if (precise) b.vert_lo = c.take<float>(3 * max_mv);
+  if (!sweep) {
+    b.tris = c.take<Tri>(nt);
+    if (precise) b.tri_lo = c.take<float4>(3 * nt);
   }
+  b.cell_frame = c.take<double>(9 * ncell);
   if (learned) {
     b.raster_budget = max_mv + max_mv / 10 + 4096;
     b.rz_bits = c.take<unsigned>(b.raster_budget);
@@ -197,18 +202,38 @@ Buffers carve_domain(Carver& c, long long ncell, long long nvert, long long nhor
     b.rdesc = c.take<RasterDesc>(1);
     b.start_m = c.take<int16_t>(L * ncell);
   }
-  if (svf_part_len > 0) b.svf_part = c.take<double>(svf_part_len);
-  b.bvh.keys = c.take<uint32_t>(nt);
-  b.bvh.vals = c.take<int32_t>(nt);
-  b.bvh.keys_alt = c.take<uint32_t>(nt);
-  b.bvh.vals_alt = c.take<int32_t>(nt);
-  b.bvh.cxy = c.take<float2>(nt);
-  b.bvh.parent = c.take<int>(nt);
-  b.bvh.nsize = c.take<int>(nt);
-  b.bvh.counter = c.take<int>(nt);
-  b.bvh.cost = c.take<float>(nt);
-  b.bvh.bounds = c.take<unsigned>(16);
-  b.bvh.sort_scratch = c.take<char>(radix_scratch_u32(nt));
+  if (sweep) {
+    const long long cells = sweep_cells_cap(max_tri);
+    b.sweep.gv = c.take<float4>(max_mv);
+    b.sweep.bounds = c.take<unsigned>(16);
+    b.sweep.grid = c.take<GridDesc>(1);
+    b.sweep.count = c.take<uint32_t>(cells + 1);
+    b.sweep.partials = c.take<uint32_t>(scan_partials(cells + 1));
+    b.sweep.total = c.take<uint32_t>(4);
+    b.cell_f32 = c.take<float>(sweep_frame_floats() * ncell);
+    b.codes = c.take<int16_t>(L * ncell);
+    b.tan_m = c.take<float>(kTanTable);
+    if (learned) {
+      b.bvh.cxy = c.take<float2>(nt);
+      b.bvh.bounds = c.take<unsigned>(16);
+    }
+  } else {
+    b.cell_origin = c.take<float>(6 * ncell);
+    b.nodes = c.take<Node>(nt > 1 ? nt - 1 : 1);
+    if (wide) b.nodes4 = c.take<Node4>(nt > 1 ? nt - 1 : 1);
+    if (svf_part_len > 0) b.svf_part = c.take<double>(svf_part_len);
+    b.bvh.keys = c.take<uint32_t>(nt);
+    b.bvh.vals = c.take<int32_t>(nt);
+    b.bvh.keys_alt = c.take<uint32_t>(nt);
+    b.bvh.vals_alt = c.take<int32_t>(nt);
+    b.bvh.cxy = c.take<float2>(nt);
+    b.bvh.parent = c.take<int>(nt);
+    b.bvh.nsize = c.take<int>(nt);
+    b.bvh.counter = c.take<int>(nt);
+    b.bvh.cost = c.take<float>(nt);
+    b.bvh.bounds = c.take<unsigned>(16);
+    b.bvh.sort_scratch = c.take<char>(radix_scratch_u32(nt));
+  }
   b.order_scratch = c.take<char>(cell_order_scratch_bytes(ncell));
   b.cell_bounds = c.take<unsigned>(8);
   b.azim_cs = c.take<double2>(nhori * 50);  // L <= num_hori * max refine_factor
@@ -223,6 +248,9 @@ struct BatchBuffers {
   DomainDesc* doms;
   int32_t* order;                 // all work ids
   int* work;
+  int* list;                      // profile sweep: cells left to the repair
+  unsigned* listed;
+  SweepAll all;                   // its triangles, lists and pyramids, domain after domain
   unsigned long long* counters;   // rays, node visits, triangle tests
   unsigned long long* done;       // per domain: finished cells, completion time
   unsigned long long* t0;         // globaltimer at the start of the search
@@ -230,12 +258,39 @@ struct BatchBuffers {
   float* mlp;                     // learned warm start parameters (device copy)
 };
 
-BatchBuffers carve_batch(Carver& c, int n, long long total_cells) {
+// Sizes of the sweep's arrays over the domains of a call.
+struct SweepSizes {
+  long long tri = 0, cells = 0, refs = 0;
+};
+
+// Adds a domain's share and returns where it begins.
+SweepSizes add_domain(SweepSizes& all, long long nvert, int grid_type) {
+  const SweepSizes at = all;
+  const long long max_tri = (grid_type == 0 ? 4 : 6) * nvert;
+  all.tri += max_tri > 0 ? max_tri : 1;
+  all.cells += (sweep_cells_cap(max_tri) + 1 + 15) & ~15ll;  // 32-byte bricks in the pyramid
+  all.refs += sweep_refs_cap(max_tri);
+  return at;
+}
+
+BatchBuffers carve_batch(Carver& c, int n, long long total_cells, const SweepSizes* sweep = nullptr,
+                         bool precise = false) {
   BatchBuffers b;
+  std::memset(&b, 0, sizeof(b));
   b.mlp = c.take<float>(kMlpParams);
   b.doms = c.take<DomainDesc>(n);
   b.order = c.take<int32_t>(total_cells);
   b.work = c.take<int>(4);
+  if (sweep) {
+    b.list = c.take<int>(total_cells);
+    b.listed = c.take<unsigned>(total_cells / 32 + 1);
+    b.all.tris = c.take<Tri>(sweep->tri);
+    if (precise) b.all.tri_lo = c.take<float4>(3 * sweep->tri);
+    b.all.refs = c.take<uint2>(sweep->refs);
+    b.all.start = c.take<uint32_t>(sweep->cells);
+    b.all.top = c.take<uint16_t>(2 * sweep->cells);
+    b.all.low = c.take<uint16_t>(2 * sweep->cells);
+  }
   b.counters = c.take<unsigned long long>(kCounterWords);
   b.done = c.take<unsigned long long>(2 * (size_t)n);
   b.t0 = c.take<unsigned long long>(2);
@@ -452,6 +507,9 @@ __global__ void k_stamp(unsigned long long* t) {
 
 enum class Stop { kMesh, kEnu, kFull };
 
+// run_batch: the sweep's grid cannot hold a domain, nothing was written.
+constexpr int kRetryWithTree = -1;
+
 struct RunOut {
   std::vector<int> n_tri, n_mv;
   std::vector<double> latency_ms;
@@ -471,6 +529,8 @@ int resident_lanes(long long* lanes) {
 // Searches of more items than this many times the resident lanes queue the
 // border cells of each domain first (run_batch).
 constexpr long long kBorderFirstWaves = 4;
+// Sweep items per resident lane that a call aims at.
+constexpr long long kSweepWaves = 4;
 
 // Runs the pipeline for n domains whose arrays are device pointers in pr[].
 // With stop != kFull it ends after the mesh (or ENU) stage and leaves the
@@ -570,6 +630,8 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
     frames[d] = enu_frame_from_sum(sums[3 * d], sums[3 * d + 1], sums[3 * d + 2]);
     const double* so = sums + 3 * d;
     const double radius = sqrt(so[0] * so[0] + so[1] * so[1] + so[2] * so[2]);
+    // Cells spread over much of the sphere: not a domain for the sweep's grid.
+    if (b[d].codes && !(radius >= 0.9 * kEarthRadius * pr[d].ncell)) return kRetryWithTree;
     out->origin_lat[d] = rad2deg(asin(so[2] / radius));
     out->origin_lon[d] = rad2deg(atan2(so[1], so[0]));
   }
@@ -601,11 +663,20 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
   phase.next("hz: bvh");
   if (stop == Stop::kEnu) return HZ_OK;
 
-  // ---- BVH (cpp:395-432) ----
+  // ---- BVH (cpp:395-432), or the profile sweep's grid ----
+  const bool sweep = b[0].codes != nullptr;
   {
     Fork fk(E, s, n);
     HZ_CUDA(fk.begin());
     for (int d = 0; d < n; d++) {
+      if (sweep) {
+        HZ_CUDA(sweep_grid(b[d].vert32, b[d].vert_lo, b[d].vot, out->n_tri[d], out->n_mv[d],
+                           b[d].tri_base, (float)pr[d].dist_search, b[d].sweep, b[d].tris,
+                           b[d].tri_lo, bb.err, fk.on(d)));
+        if (b[d].rz)  // the learned start's raster is laid over these bounds
+          HZ_CUDA(bvh_tri_bounds(b[d].vert32, b[d].vot, out->n_tri[d], b[d].bvh, fk.on(d)));
+        continue;
+      }
       HZ_CUDA(bvh_build(b[d].vert32, b[d].vot, out->n_tri[d], b[d].nodes, b[d].tris, b[d].bvh,
                         fk.on(d), b[d].vert_lo, b[d].tri_lo, b[d].nodes4, opt.leaf_size,
                         opt.bvh_treelets != 0));
@@ -672,7 +743,13 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
     for (int d = 0; d < n; d++) items += (long long)pr[d].cell_count * pr[d].groups;
     const int rl = resident_lanes(&lanes);
     if (rl) return rl;
-    const bool border_first = items >= kBorderFirstWaves * lanes;
+    const bool border_first = !sweep && items >= kBorderFirstWaves * lanes;
+    // Sweep items: runs of consecutive azimuths per cell, enough of them to
+    // fill the lanes a few times over (the first azimuth of a run sweeps from
+    // the floor, 1.1 to 1.4 times the work of one that follows another).
+    long long cells_all = 0;
+    for (int d = 0; d < n; d++) cells_all += pr[d].cell_count;
+    const long long runs_wanted = (kSweepWaves * lanes + cells_all - 1) / std::max(1ll, cells_all);
     // Queue order of the domains: least work (cells x azimuths) first, so
     // that the small domains of a batch complete early (shortest job first:
     // the lowest mean completion time for the same total work).
@@ -689,7 +766,7 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
       const Problem& P = pr[d];
       const int L = P.nhori * P.refine;
       HZ_CUDA(trace_tables(b[d].azim_cs, b[d].elev_cs, b[d].svf_lattice, L, shift[d],
-                           hori_acc, P.svf_type, fk.on(d)));
+                           hori_acc, P.svf_type, fk.on(d), b[d].tan_m));
       if (learned) {
         HZ_CUDA(raster_build(b[d].vert32, b[d].vot, out->n_tri[d], b[d].bvh.bounds,
                              b[d].raster_budget, b[d].rdesc, b[d].rz_bits, b[d].rz, fk.on(d)));
@@ -751,6 +828,22 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
       D.item_begin = total_items;
       D.svf_part = b[d].svf_part;
       D.raw_j = n == 1 ? opt.raw_index : nullptr;
+      D.grid = b[d].sweep.grid;
+      D.top = b[d].sweep.top;
+      D.low = b[d].sweep.low;
+      D.gstart = b[d].sweep.start;
+      D.refs = b[d].sweep.refs;
+      D.cell_f32 = b[d].cell_f32;
+      D.codes = b[d].codes;
+      D.tan_m = b[d].tan_m;
+      D.cell_base = b[d].cell_base;
+      D.ref_base = b[d].ref_base;
+      if (sweep) {
+        // Lists name triangles by their number in the call's array.
+        D.tris = bb.all.tris;
+        D.tri_lo = bb.all.tri_lo;
+      }
+      D.runs = (int)std::max(1ll, std::min<long long>(L, runs_wanted));
       D.centre = frames[d].centre;
       D.pole = frames[d].pole;
       D.ray_org_elev = P.ray_org_elev;
@@ -769,7 +862,7 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
       D.tfar = (float)P.dist_search;
       desc[j] = D;  // in queue order: k_begin and item_begin increase with j
       total += P.cell_count;
-      total_items += (long long)P.cell_count * P.groups;
+      total_items += (long long)P.cell_count * (sweep ? D.runs : P.groups);
     }
     HZ_CUDA(fk.end());
     if (total_items > INT32_MAX - (1ll << 26))
@@ -785,6 +878,12 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
     note_launches(1);
     HZ_CUDA(cudaGetLastError());
     const TraceKnobs knobs{adv, leaf, opt.queue_chunk, variant};
+    if (sweep) {
+      // The lowest ray of a search: one step past the floor (cpp:538).
+      const int s_full = std::min(-1, (int)floor(opt.elev_floor_deg * 2.0) - 1);
+      HZ_CUDA(sweep_search(bb.doms, n, bb.order, (int)total, (int)total_items, s_full, bb.work,
+                           bb.list, bb.listed, bb.all, bb.counters, bb.err, b[0].tri_lo != nullptr, s));
+    } else
     HZ_CUDA(trace_flat(bb.doms, n, bb.order, (int)total, (int)total_items, bb.work,
                        bb.counters, bb.err, knobs, opt.count_work != 0,
                        b[0].tri_lo != nullptr, s));
@@ -816,6 +915,7 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
 #endif
   const int* errw = reinterpret_cast<const int*>(rb + 12);  // bit word, check code, index
   const int err1 = errw[0];
+  if (err1 & kErrGrid) return kRetryWithTree;
   if (err1 & kErrStack) return fail(HZ_ERR_INTERNAL, "BVH traversal stack overflow");
   if (err1 & kErrBounds)
     return fail(HZ_ERR_INTERNAL, "bounds check failed in the search: check %d, index %d",
@@ -991,6 +1091,32 @@ int azimuth_groups(const hz_domain* doms, int n, const hz_options& opt, int* gro
   return HZ_OK;
 }
 
+// Whether a call runs the profile sweep (hz_sweep.cu) rather than the tree
+// search: wherever both can run it is the faster one, from 500 cells (1.9
+// against 5.3 ms) to 3.1M (102 against 136 ms), at every spacing and azimuth
+// count measured, with the same results. The tree search keeps what belongs to it: its own kernels and knobs,
+// work counters (they count its visits), the bisected walk (a ray sequence of
+// its own); and searches whose floor lies below 88 deg or whose result codes (2
+// bytes per cell and azimuth) would not fit beside the outputs.
+constexpr long long kMaxCodeBytes = 16ll << 30;
+
+bool use_sweep(const hz_domain* doms, int n, const hz_options& opt) {
+  if (opt.kernel != HZ_KERNEL_PERSISTENT || opt.count_work ||
+      opt.elev_walk != HZ_WALK_REFERENCE || opt.advance_min || opt.leaf_min || opt.leaf_size ||
+      opt.queue_chunk || opt.bvh_treelets || !opt.occluder_cache)
+    return false;
+  if (!(opt.elev_floor_deg >= -88.0 && opt.elev_floor_deg <= 88.0)) return false;
+  long long bytes = 0;
+  SweepSizes all;
+  for (int d = 0; d < n; d++) {
+    bytes += 2ll * doms[d].num_cell * doms[d].num_hori * doms[d].refine_factor;
+    add_domain(all, doms[d].num_vertex, doms[d].grid_type);
+  }
+  // 32-bit indices into the call's arrays.
+  return bytes <= kMaxCodeBytes && all.tri < INT32_MAX && 2 * all.cells < INT32_MAX &&
+         all.refs < UINT32_MAX;
+}
+
 // Shared implementation of the host / device, single / batch entry points.
 int run_entry(hz_domain* doms, int n, bool on_device, cudaStream_t user_stream,
               const hz_options& opt, hz_stats* stats) {
@@ -1043,63 +1169,91 @@ int run_entry(hz_domain* doms, int n, bool on_device, cudaStream_t user_stream,
     return groups[d] > 1 && doms[d].refine_factor > 1
                ? (long long)groups[d] * doms[d].num_cell : 0ll;
   };
-  Carver dry(nullptr);
-  for (int d = 0; d < n; d++)
-    carve_domain(dry, doms[d].num_cell, doms[d].num_vertex, doms[d].num_hori,
-                 doms[d].grid_type, !on_device, precise, learned,
-                 (long long)doms[d].num_hori * doms[d].refine_factor, wide, svf_part_len(d));
-  carve_batch(dry, n, total_cells);
-  rc = E->reserve(dry.off, s);
-  if (rc) return rc;
-  Carver c(E->arena);
-  std::vector<Buffers> b(n);
-  for (int d = 0; d < n; d++)
-    b[d] = carve_domain(c, doms[d].num_cell, doms[d].num_vertex, doms[d].num_hori,
-                        doms[d].grid_type, !on_device, precise, learned,
-                        (long long)doms[d].num_hori * doms[d].refine_factor, wide,
-                        svf_part_len(d));
-  const BatchBuffers bb = carve_batch(c, n, total_cells);
-
-  std::vector<Problem> pr(n);
-  // Host <-> device phases are timed on the host: pageable buffers are
-  // copied partly by host threads.
-  const auto t_h2d = std::chrono::steady_clock::now();
-  for (int d = 0; d < n; d++) {
-    const hz_domain& h = doms[d];
-    if (!on_device) {
-      rc = stage_inputs(*E, h, b[d], s);
-      if (rc) return rc;
-    }
-    Problem& P = pr[d];
-    P.clon = on_device ? h.clon : b[d].clon;
-    P.clat = on_device ? h.clat : b[d].clat;
-    P.hsurf = on_device ? h.hsurf : b[d].hsurf;
-    P.vlon = on_device ? h.vlon : b[d].vlon;
-    P.vlat = on_device ? h.vlat : b[d].vlat;
-    P.cov = on_device ? h.cells_of_vertex : b[d].cov;
-    P.horizon = on_device ? h.horizon : b[d].horizon;
-    P.skyview = on_device ? h.skyview : b[d].skyview;
-    P.ncell = h.num_cell;
-    P.nvert = h.num_vertex;
-    P.nhori = h.num_hori;
-    P.grid_type = h.grid_type;
-    P.dist_search = h.dist_search;
-    P.ray_org_elev = h.ray_org_elev;
-    P.refine = h.refine_factor;
-    P.svf_type = h.svf_type;
-    rc = cell_range(opt, h.num_cell, &P.cell_begin, &P.cell_count);
-    if (rc) return rc;
-    P.groups = groups[d];
-  }
+  // The profile sweep where it can run; a domain its grid cannot hold (raised
+  // on the device before any output is written) runs the tree search instead.
+  bool sweep = use_sweep(doms, n, opt);
+  std::vector<Buffers> b;
+  std::vector<Problem> pr;
   double ms_h2d = 0.0;
-  if (!on_device) {
-    HZ_CUDA(cudaStreamSynchronize(s));
-    ms_h2d = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_h2d)
-                 .count();
-  }
-  if (stats) std::memset(stats, 0, sizeof(*stats));
   RunOut out;
-  rc = run_batch(*E, pr.data(), b.data(), n, bb, s, opt, stats, Stop::kFull, &out);
+  for (;;) {
+    Carver dry(nullptr);
+    for (int d = 0; d < n; d++)
+      carve_domain(dry, doms[d].num_cell, doms[d].num_vertex, doms[d].num_hori,
+                   doms[d].grid_type, !on_device, precise, learned,
+                   (long long)doms[d].num_hori * doms[d].refine_factor, wide, svf_part_len(d),
+                   sweep);
+    SweepSizes sizes;
+    if (sweep)
+      for (int d = 0; d < n; d++) add_domain(sizes, doms[d].num_vertex, doms[d].grid_type);
+    carve_batch(dry, n, total_cells, sweep ? &sizes : nullptr, precise);
+    rc = E->reserve(dry.off, s);
+    if (rc) return rc;
+    Carver c(E->arena);
+    b.assign(n, Buffers());
+    for (int d = 0; d < n; d++)
+      b[d] = carve_domain(c, doms[d].num_cell, doms[d].num_vertex, doms[d].num_hori,
+                          doms[d].grid_type, !on_device, precise, learned,
+                          (long long)doms[d].num_hori * doms[d].refine_factor, wide,
+                          svf_part_len(d), sweep);
+    const BatchBuffers bb = carve_batch(c, n, total_cells, sweep ? &sizes : nullptr, precise);
+    if (sweep) {
+      SweepSizes at;
+      for (int d = 0; d < n; d++) {
+        const SweepSizes o = add_domain(at, doms[d].num_vertex, doms[d].grid_type);
+        b[d].tri_base = (int)o.tri;
+        b[d].cell_base = (int)o.cells;
+        b[d].ref_base = (unsigned)o.refs;
+        b[d].tris = bb.all.tris + o.tri;
+        b[d].tri_lo = precise ? bb.all.tri_lo + 3 * o.tri : nullptr;
+        b[d].sweep.refs = bb.all.refs + o.refs;
+        b[d].sweep.start = bb.all.start + o.cells;
+        b[d].sweep.top = bb.all.top + 2 * o.cells;
+        b[d].sweep.low = bb.all.low + 2 * o.cells;
+      }
+    }
+
+    pr.assign(n, Problem());
+    // Host <-> device phases are timed on the host: pageable buffers are
+    // copied partly by host threads.
+    const auto t_h2d = std::chrono::steady_clock::now();
+    for (int d = 0; d < n; d++) {
+      const hz_domain& h = doms[d];
+      if (!on_device) {
+        rc = stage_inputs(*E, h, b[d], s);
+        if (rc) return rc;
+      }
+      Problem& P = pr[d];
+      P.clon = on_device ? h.clon : b[d].clon;
+      P.clat = on_device ? h.clat : b[d].clat;
+      P.hsurf = on_device ? h.hsurf : b[d].hsurf;
+      P.vlon = on_device ? h.vlon : b[d].vlon;
+      P.vlat = on_device ? h.vlat : b[d].vlat;
+      P.cov = on_device ? h.cells_of_vertex : b[d].cov;
+      P.horizon = on_device ? h.horizon : b[d].horizon;
+      P.skyview = on_device ? h.skyview : b[d].skyview;
+      P.ncell = h.num_cell;
+      P.nvert = h.num_vertex;
+      P.nhori = h.num_hori;
+      P.grid_type = h.grid_type;
+      P.dist_search = h.dist_search;
+      P.ray_org_elev = h.ray_org_elev;
+      P.refine = h.refine_factor;
+      P.svf_type = h.svf_type;
+      rc = cell_range(opt, h.num_cell, &P.cell_begin, &P.cell_count);
+      if (rc) return rc;
+      P.groups = groups[d];
+    }
+    if (!on_device) {
+      HZ_CUDA(cudaStreamSynchronize(s));
+      ms_h2d = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_h2d)
+                   .count();
+    }
+    if (stats) std::memset(stats, 0, sizeof(*stats));
+    rc = run_batch(*E, pr.data(), b.data(), n, bb, s, opt, stats, Stop::kFull, &out);
+    if (rc != kRetryWithTree) break;
+    sweep = false;
+  }
   if (rc) return rc;
   for (int d = 0; d < n; d++) doms[d].latency_ms = out.latency_ms[d];
   const auto t_d2h = std::chrono::steady_clock::now();

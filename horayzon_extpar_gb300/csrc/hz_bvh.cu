@@ -470,16 +470,25 @@ size_t bvh_scratch_bytes(long long n) {
   return b + 8 * 256;                     // alignment slack
 }
 
+cudaError_t bvh_tri_bounds(const float* vert32, const int* vot, int n, const BvhScratch& sc,
+                           cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  k_init_bounds<<<1, 1, 0, s>>>(sc.bounds);
+  k_tri_bounds<<<grid_for(n, 256), 256, 0, s>>>(vert32, vot, n, sc.cxy, sc.bounds);
+  note_launches(2);
+  return cudaGetLastError();
+}
+
 cudaError_t bvh_build(const float* vert32, const int* vot, int n, Node* nodes, Tri* tris,
                       const BvhScratch& sc, cudaStream_t s, const float* vert_lo,
                       float4* tri_lo, Node4* nodes4, int leaf_max, bool treelets) {
   if (leaf_max < 1 || leaf_max > 8) leaf_max = kLeafMax;
   if (n <= 0) return cudaSuccess;
-  k_init_bounds<<<1, 1, 0, s>>>(sc.bounds);
-  k_tri_bounds<<<grid_for(n, 256), 256, 0, s>>>(vert32, vot, n, sc.cxy, sc.bounds);
+  cudaError_t e = bvh_tri_bounds(vert32, vot, n, sc, s);
+  if (e != cudaSuccess) return e;
   k_morton<<<grid_for(n, 256), 256, 0, s>>>(sc.cxy, n, sc.bounds, sc.keys, sc.vals);
-  note_launches(3);
-  cudaError_t e = radix_sort_pairs(sc.keys, sc.vals, sc.keys_alt, sc.vals_alt, n, 32,
+  note_launches(1);
+  e = radix_sort_pairs(sc.keys, sc.vals, sc.keys_alt, sc.vals_alt, n, 32,
                                    sc.sort_scratch, s);
   if (e != cudaSuccess) return e;
   k_gather<<<grid_for(n, 256), 256, 0, s>>>(vert32, vot, sc.vals, n, tris, vert_lo,

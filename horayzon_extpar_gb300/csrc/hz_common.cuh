@@ -27,7 +27,8 @@ enum : int {
   kErrBadIndex = 1,     // cells_of_vertex entry outside [0, ncell) and != -2
   kErrStack = 2,        // traversal stack overflow
   kErrMeshCapacity = 4,  // mesh emission beyond the sized buffers
-  kErrBounds = 8         // checked builds (HZ_CHECKED): an index outside its array
+  kErrBounds = 8,        // checked builds (HZ_CHECKED): an index outside its array
+  kErrGrid = 16          // the sweep's grid cannot hold the domain (tree search instead)
 };
 
 // Leaf references are negative: ~(start << 3 | (count - 1)).

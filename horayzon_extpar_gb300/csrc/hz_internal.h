@@ -72,6 +72,10 @@ struct BvhScratch {
   void* sort_scratch;   // radix_scratch_u32(n)
 };
 size_t bvh_scratch_bytes(long long n_tri);
+// Bounds of the triangles' box centres and the largest coordinate, alone
+// (sc.cxy, sc.bounds; the first step of bvh_build).
+cudaError_t bvh_tri_bounds(const float* vert32, const int* vot, int n_tri, const BvhScratch& sc,
+                           cudaStream_t s);
 // Builds nodes[n_tri - 1] (or one node when n_tri <= leaf_max) and tris[n_tri];
 // leaves hold at most leaf_max triangles (1..8; other values: kLeafMax);
 // the root is node 0. n_tri == 0 leaves the tree empty.
@@ -113,11 +117,13 @@ struct TraceParams {
 constexpr int kElevMin = -256;
 constexpr int kElevTable = 1280;
 constexpr int kSvfTable = 2560;
+constexpr int kTanTable = 360;  // tan_m: tangents of (k - 180) * 0.5 deg (profile sweep)
 
 // Fills the lattice tables (device FP64 sin/cos); shift is the reference's
 // azimuth shift (cpp:662-668).
 cudaError_t trace_tables(double2* azim_cs, double2* elev_cs, double* svf_lattice, int L,
-                         double shift, double hori_acc, int svf_type, cudaStream_t s);
+                         double shift, double hori_acc, int svf_type, cudaStream_t s,
+                         float* tan_m = nullptr);
 // One thread per cell, nested loops as in the reference (simple; kept as the
 // second implementation the flattened kernel is tested against).
 // Any-hit flags (hit[i] = 1) of n_ray rays (org, dir: float3 on the device)
@@ -136,6 +142,21 @@ size_t cell_order_scratch_bytes(long long n);
 cudaError_t cell_order(const double* cell_enu, const int* cov, int nv, int ncell, int begin,
                        int count, int id_offset, int32_t* order, void* scratch,
                        unsigned* bounds, int* work, cudaStream_t s);
+
+// Regular grid of a domain in gnomonic coordinates (hz_sweep.cu).
+struct GridDesc {
+  float x0, y0, c, inv_c;     // origin, cell size
+  float pad;                  // margin by which triangles are grown
+  float hlo, iq, unit;        // heights as integers: (h - hlo) * iq, iq = 1 / unit
+  float hpad;                 // margin of a ray's height
+  float rlo, rhi;             // radii of the lowest and highest vertex
+  float tau_max;              // tangent of the search radius' angle at the centre
+  float cmin, cmax;           // bounds of the curvature term's factor
+  float dadd;                 // bound of a triangle's distance beyond the walk's
+  int W, H, L;                // cells; highest pyramid level
+  unsigned lmax;              // longest edge (float bits)
+  int ok;                     // 0: the grid cannot hold the domain (kErrGrid)
+};
 
 // One domain of the persistent search (device-resident array).
 struct DomainDesc {
@@ -173,6 +194,20 @@ struct DomainDesc {
   // 1: an upward step first tests the triangle that hid the step below
   // (k_trace_warp's occluder cache; same results, fewer traversals).
   int occ_cache;
+  // Profile sweep (hz_sweep.cu): grid, pyramid, list starts and lists; FP32
+  // cell frames [kFrameRows][ncell] by work position; result codes [L][ncell];
+  // items per cell (runs of consecutive azimuths).
+  const GridDesc* grid;
+  const uint16_t* top;
+  const uint16_t* low;
+  const uint32_t* gstart;
+  const uint2* refs;
+  float* cell_f32;
+  int16_t* codes;
+  int cell_base;              // of its cells in gstart (half of it: its pyramid) and of its
+  unsigned ref_base;          // list entries, in the call's arrays (SweepAll)
+  const float* tan_m;         // [kTanTable] tangents of (k - kTanTable / 2) * 0.5 deg
+  int runs;
   int16_t* raw_j;             // optional output: unclipped horizon j (h = j * 0.25 deg)
   double3 centre, pole;       // Earth centre / North Pole in ENU
   double ray_org_elev, hori_acc, elev_floor;
@@ -216,6 +251,45 @@ struct TraceKnobs {
 cudaError_t trace_flat(const DomainDesc* doms, int ndom, const int32_t* order, int total,
                        int total_items, int* work, unsigned long long* counters, int* err,
                        const TraceKnobs& k, bool count_work, bool precise, cudaStream_t s);
+
+// ---- hz_sweep.cu ------------------------------------------------------------
+// Capacities of a domain's grid cells and list entries, rows of the frame table.
+long long sweep_cells_cap(long long n_tri);
+long long sweep_refs_cap(long long n_tri);
+size_t sweep_frame_floats();
+struct SweepBuffers {
+  float4* gv;            // n_vert: gnomonic X, Y, height
+  unsigned* bounds;      // 8
+  GridDesc* grid;
+  uint32_t* count;       // cells cap + 1
+  uint32_t* start;       // cells cap + 1
+  uint32_t* partials;    // scan_partials(cells cap + 1)
+  uint32_t* total;
+  uint16_t* top;         // 2 x cells cap: pyramid of upper heights
+  uint16_t* low;         // and of lower ones
+  uint2* refs;           // refs cap
+};
+// Grid, lists and height pyramid of a domain, and its triangle records (mesh
+// order). Raises kErrGrid where the grid cannot hold the domain.
+cudaError_t sweep_grid(const float* vert32, const float* vert_lo, const int* vot, int n_tri,
+                       int n_vert, int tri_base, float tfar, const SweepBuffers& b, Tri* tris,
+                       float4* tri_lo, int* err, cudaStream_t s);
+// The arrays of all domains of a call.
+struct SweepAll {
+  Tri* tris;
+  float4* tri_lo;
+  uint2* refs;
+  uint32_t* start;
+  uint16_t* top;
+  uint16_t* low;
+};
+// Frames, sweep, repair and outputs of all domains (after cell_order and
+// trace_tables). s_full: the lowest lattice elevation a search can ask for.
+// work: 3 ints; list, listed: `total` work positions and bits.
+cudaError_t sweep_search(const DomainDesc* doms, int ndom, const int32_t* order, int total,
+                         int total_items, int s_full, int* work, int* list, unsigned* listed,
+                         const SweepAll& all, unsigned long long* counters, int* err,
+                         bool precise, cudaStream_t s);
 
 // ---- hz_static.cu -----------------------------------------------------------
 // Forgets the cached device address of the no-allocation entry point's

@@ -1,0 +1,1412 @@
+// hz_sweep.cu -- the horizon search as one profile sweep per (cell, azimuth).
+//
+// The reference tests the horizon of an azimuth with one ray per elevation
+// step (mo_lradtopo_horayzon.cpp:490-555). All rays of one (cell, azimuth)
+// lie in the plane through the ray origin, the azimuth's horizontal direction
+// and the cell's normal, and the normal points away from the Earth's centre:
+// the plane contains the centre. In the gnomonic projection from the centre
+// (X = R x / z, Y = R y / z in the domain's ENU axes, origin at the centre)
+// such a plane is one straight line, the same for every elevation. So the
+// rays of an azimuth share one track over a regular X/Y grid, and terrain
+// hides a ray exactly where its height above the sphere exceeds the ray's.
+//
+//   * grid build: the triangles of each grid cell (counting, scan, fill) with
+//     upper and lower bounds of their heights inside the cell, and a pyramid
+//     of the cells' bounds (every second level, 4 x 4 children);
+//   * k_sweep: walks the track front to back at the elevation of the lowest
+//     ray not yet known to be hidden, skipping every pyramid cell that lies
+//     below it. A triangle that hides the ray raises the elevation, and the
+//     walk goes on from there: what was skipped or passed lies below every
+//     higher ray of the plane, so nothing is walked twice. It ends with the
+//     lowest lattice elevation m that misses, every lattice ray from the
+//     sweep's start up to m - 1 known to hit, every one from m up known to
+//     miss: the hit pattern that the reference's bracketing search asks for,
+//     whatever elevation it starts from;
+//   * k_sweep_repair: azimuths whose hits are not one run of elevations (a
+//     cell that looks under the edge of the mesh, a ray that ends in mid-air
+//     at dist_search) are searched ray by ray as the reference does, a warp
+//     per cell and 32 elevations at a time;
+//   * k_sweep_finish: replays the reference's search of every cell on the hit
+//     patterns (its carried elevation, its accumulation of 0.5 deg steps, its
+//     ray count) and writes degrees and sky view factors.
+//
+// Exactness: hit decisions are those of the watertight FP32 test of the same
+// FP32 rays. The sweep's own classification of a triangle (below the ray,
+// beside the plane, hit) uses FP32 distances from the plane with error bounds
+// and decides only what lies outside them; anything nearer is put to the
+// watertight test itself (exact_hit), and a triangle that stays above an
+// unhidden ray hands the azimuth to k_sweep_repair.
+//
+// Against the tree search (GB300, whole call): one traversal of a bounding
+// volume tree per ray took 2.5 to 4 rays, 63 to 126 four-wide node visits and 38
+// to 76 triangle tests per evaluation; the sweep takes 53 to 90 two-byte steps and
+// 20 to 40 tests. 500 m, 3.1M cells 135.5 -> 102.3 ms; 100 m, 1.2M cells 107.9 ->
+// 77.4 ms; 2.5 km, 57k cells 8.0 -> 3.0 ms; 500 cells 5.3 -> 1.9 ms; 360 azimuths,
+// 21k cells 56.4 -> 13.9 ms. The small domains gain most: a sweep from the floor
+// needs no other azimuth's result, so a cell's azimuths run side by side.
+#include <algorithm>
+
+#include "hz_internal.h"
+#include "hz_ray.cuh"
+
+namespace hz {
+
+namespace {
+
+constexpr int kSweepBlock = 128;
+#ifndef HZ_SWEEP_MIN_BLOCKS
+#define HZ_SWEEP_MIN_BLOCKS 5
+#endif
+#ifndef HZ_WALK_STEPS
+#define HZ_WALK_STEPS 8  // pyramid steps per lane in one walk pass
+#endif
+#ifndef HZ_WALK_MIN
+#define HZ_WALK_MIN 12  // a walk pass ends when fewer lanes walk
+#endif
+#ifndef HZ_CELL_TRIS
+#define HZ_CELL_TRIS 1.0f  // cell area in mean triangle areas
+#endif
+#ifndef HZ_SWEEP_ADVANCE
+#define HZ_SWEEP_ADVANCE 8  // lanes that must wait before azimuths are set up
+#endif
+
+constexpr float kRf = 6371229.0f;         // kEarthRadius, exact in FP32
+constexpr float kEps = 9.5367431640625e-07f;  // 2^-20: relative error bound of a vertex's
+                                              // FP32 distances, 4 x the sum of its roundings
+constexpr float kMagic = 8388608.0f;      // 2^23: float(2^23 | n) = 2^23 + n
+constexpr float kBig = 1e30f;
+constexpr int kTanRange = 180;            // lattice elevations with a tangent: |m| < 180
+constexpr int kMaxM = 177;                // sweeps stop below 89 deg
+
+// Codes of a (cell, azimuth): the lowest missing lattice elevation, or
+constexpr int kCodeAllMiss = -20000;      // no lattice ray meets the terrain
+constexpr int kCodeGap = -20001;          // left to k_sweep_repair
+constexpr int kCodeStop = 10000;          // + ((m + 2000) << 1 | up): the search's stop itself
+
+__device__ __forceinline__ float height_magic(unsigned h16) {
+  return __uint_as_float(0x4B000000u | h16);
+}
+
+// ---------------------------------------------------------------------------
+// Grid build
+// ---------------------------------------------------------------------------
+
+// Gnomonic X, Y and height above the sphere of every mesh vertex, and their
+// bounds (ordered keys): min X, Y, H, z; max X, Y, H. The height is (r^2 -
+// R^2) / (r + R) with the numerator in FP64 (it cancels), good to 1e-3 m.
+__global__ void k_gnomonic(const float* __restrict__ vert, int n, float4* __restrict__ gv,
+                           unsigned* __restrict__ bounds) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = i < n;
+  float X = 0.f, Y = 0.f, H = 0.f, z = 0.f;
+  if (valid) {
+    const float x = vert[3LL * i], y = vert[3LL * i + 1], zz = vert[3LL * i + 2];
+    const double dx = x, dy = y, dz = zz;
+    const double r2 = dx * dx + dy * dy + dz * (dz + 2.0 * kEarthRadius);
+    z = (float)(dz + kEarthRadius);
+    const float f = __fdiv_rn(kRf, z);
+    X = x * f;
+    Y = y * f;
+    const float num = (float)r2;
+    H = __fdiv_rn(num, sqrtf((float)(kEarthRadius * kEarthRadius + r2)) + kRf);
+    gv[i] = make_float4(X, Y, H, 0.f);
+  }
+  const unsigned no = 0xFFFFFFFFu;
+  unsigned b[7] = {valid ? f2ord(X) : no, valid ? f2ord(Y) : no, valid ? f2ord(H) : no,
+                   valid ? f2ord(z) : no, valid ? f2ord(X) : 0u, valid ? f2ord(Y) : 0u,
+                   valid ? f2ord(H) : 0u};
+  block_bounds_atomic<4, 3>(b, bounds);
+}
+
+__global__ void k_grid_init(unsigned* b) {
+  for (int k = 0; k < 4; k++) b[k] = 0xFFFFFFFFu;
+  for (int k = 4; k < 8; k++) b[k] = 0u;
+}
+
+// Grid geometry: cells of HZ_CELL_TRIS times the mean triangle area.
+__global__ void k_grid_setup(const unsigned* __restrict__ b, int n_tri, long long cap0, float tfar,
+                             GridDesc* __restrict__ g, int* __restrict__ err) {
+  GridDesc q;
+  const float x0 = ord2f(b[0]), y0 = ord2f(b[1]), h0 = ord2f(b[2]), z0 = ord2f(b[3]);
+  const float x1 = ord2f(b[4]), y1 = ord2f(b[5]), h1 = ord2f(b[6]);
+  const float ex = fmaxf(x1 - x0, 1.f), ey = fmaxf(y1 - y0, 1.f);
+  const float big = fmaxf(fmaxf(fabsf(x0), fabsf(x1)), fmaxf(fabsf(y0), fabsf(y1)));
+  float c = sqrtf(ex * ey * HZ_CELL_TRIS / (float)(n_tri > 0 ? n_tri : 1));
+  c = fminf(fmaxf(c, fmaxf(ex, ey) * 6e-5f), 1e6f);  // at most ~16,000 cells a side
+  // Domains the projection cannot hold (a vertex 60 deg or more from the
+  // centre's axis) or inputs that are not finite.
+  bool ok = z0 > 0.5f * kRf && isfinite(ex) && isfinite(ey) && isfinite(h0) && isfinite(h1) &&
+            h1 - h0 < 2e5f && h0 > -1e5f && isfinite(c);
+  int W = 1, H = 1, L = 0;
+  float pad = 0.f;
+  for (int it = 0; ok; it++) {
+    pad = 3e-6f * big + 1e-6f * tfar + 2e-3f * c + 0.02f;
+    const int nx = (int)((ex + 3.f * pad) / c) + 2, ny = (int)((ey + 3.f * pad) / c) + 2;
+    L = 0;
+    while (L < 8 && (min(nx, ny) >> (L + 2)) >= 2) L += 2;
+    const int r = (4 << L) - 1;  // whole bricks at every level
+    W = (nx + r) & ~r;
+    H = (ny + r) & ~r;
+    if ((long long)W * H <= cap0) break;
+    c *= 1.1f;
+    if (it > 200) ok = false;
+  }
+  q.c = c;
+  q.inv_c = 1.f / c;
+  q.pad = pad;
+  q.x0 = x0 - 1.5f * pad;
+  q.y0 = y0 - 1.5f * pad;
+  q.hlo = h0;
+  q.iq = 65000.f / (h1 - h0 + 1.f);
+  q.unit = (h1 - h0 + 1.f) / 65000.f;
+  q.hpad = 0.05f + 2e-6f * tfar;
+  q.dadd = 2.f * c + 4.f * pad + (h1 - h0) + 1.f;
+  q.rlo = kRf + h0;
+  q.rhi = kRf + h1;
+  const float s = fminf(tfar / q.rlo, 0.5f);
+  q.tau_max = s / sqrtf(1.f - s * s) * 1.0001f;
+  q.cmin = (q.rlo / q.rhi) * (1.f - 0.25f * q.tau_max * q.tau_max) * 0.5f;
+  q.cmax = (q.rhi / q.rlo) * 0.5f;
+  q.W = W;
+  q.H = H;
+  q.L = L;
+  q.lmax = 0u;
+  q.ok = ok ? 1 : 0;
+  if (!ok) atomicOr(err, kErrGrid);
+  *g = q;
+}
+
+// Index of cell (a, b) of level l (even; a = i >> l of level 0's i): a level is
+// stored in bricks of 4 x 4 cells, the children of one cell of the level
+// above, so that a walk reads 16 neighbours with one 32-byte access; level l
+// begins at n2 - (n2 >> l / 2), n2 twice the cells of level 0.
+__device__ __forceinline__ int grid_index(int W, int n2, int a, int b, int l) {
+  return n2 - (n2 >> (l >> 1)) + ((((b >> 2) * (W >> (l + 2)) + (a >> 2)) << 4) | ((b & 3) << 2) |
+                                  (a & 3));
+}
+
+// Calls f(cell index, upper height, lower height) for every grid cell whose
+// square, grown by the grid's pad, meets triangle (a, b, c): bounding box,
+// then the three edge functions. The heights bound the triangle inside the
+// grown cell: its plane over the cell and the bounding box, at most the
+// highest vertex. Between its vertices a plane triangle lies lower than the
+// linear interpolation of their heights above the sphere, by at most
+// edge^2 / 8 R.
+template <class F>
+__device__ __forceinline__ void for_cells(const GridDesc& g, float4 a, float4 b, float4 c, F f) {
+  const float pad = g.pad;
+  // Coordinates relative to the first vertex.
+  const float bx = b.x - a.x, by = b.y - a.y, cx = c.x - a.x, cy = c.y - a.y;
+  const float lx = fminf(0.f, fminf(bx, cx)), hx = fmaxf(0.f, fmaxf(bx, cx));
+  const float ly = fminf(0.f, fminf(by, cy)), hy = fmaxf(0.f, fmaxf(by, cy));
+  const float hmx = fmaxf(a.z, fmaxf(b.z, c.z)), hmn = fminf(a.z, fminf(b.z, c.z));
+  const float gx0 = a.x - g.x0, gy0 = a.y - g.y0;
+  const int i0 = max(0, (int)floorf((gx0 + lx - pad) * g.inv_c));
+  const int i1 = min(g.W - 1, (int)floorf((gx0 + hx + pad) * g.inv_c));
+  const int j0 = max(0, (int)floorf((gy0 + ly - pad) * g.inv_c));
+  const int j1 = min(g.H - 1, (int)floorf((gy0 + hy + pad) * g.inv_c));
+  const float area = bx * cy - cx * by;
+  const float e2 = fmaxf(fmaxf(bx * bx + by * by, cx * cx + cy * cy),
+                         (cx - bx) * (cx - bx) + (cy - by) * (cy - by));
+  const float sag = e2 / (8.f * kRf) * 1.05f + 0.01f;
+  const bool flat = fabsf(area) > 1e-3f * e2;  // gradient usable
+  const float ia = 1.f / area;
+  const float px = ((b.z - a.z) * cy - (c.z - a.z) * by) * ia;
+  const float py = ((c.z - a.z) * bx - (b.z - a.z) * cx) * ia;
+  const float sgn = area >= 0.f ? 1.f : -1.f;
+  // Edge functions n . (P - vertex) >= 0 inside: edges a-b, b-c, c-a.
+  const float n0x = -by * sgn, n0y = bx * sgn;
+  const float n1x = (by - cy) * sgn, n1y = (cx - bx) * sgn;
+  const float n2x = cy * sgn, n2y = -cx * sgn;
+  const float hw = 0.5f * g.c + 1.05f * pad;
+  const float s0 = (fabsf(n0x) + fabsf(n0y)) * hw, s1 = (fabsf(n1x) + fabsf(n1y)) * hw,
+              s2 = (fabsf(n2x) + fabsf(n2y)) * hw;
+  const bool sat = fabsf(area) > 1e-6f * e2;  // else a sliver: its box
+  for (int j = j0; j <= j1; j++) {
+    const float y = ((float)j + 0.5f) * g.c - gy0;
+    for (int i = i0; i <= i1; i++) {
+      const float x = ((float)i + 0.5f) * g.c - gx0;
+      if (sat && (n0x * x + n0y * y + s0 < 0.f ||
+                  n1x * (x - bx) + n1y * (y - by) + s1 < 0.f ||
+                  n2x * x + n2y * y + s2 < 0.f))
+        continue;
+      float up = hmx, lo = hmn;
+      if (flat) {
+        const float xa = fmaxf(lx, x - hw), xb = fminf(hx, x + hw);
+        const float ya = fmaxf(ly, y - hw), yb = fminf(hy, y + hw);
+        const float u = a.z + px * (px > 0.f ? xb : xa) + py * (py > 0.f ? yb : ya);
+        const float v = a.z + px * (px > 0.f ? xa : xb) + py * (py > 0.f ? ya : yb);
+        up = fminf(up, u + 0.02f);
+        lo = fmaxf(lo, v - 0.02f);
+      }
+      f(grid_index(g.W, 2 * g.W * g.H, i, j, 0), up, lo - sag);
+    }
+  }
+}
+
+// Triangles per cell; also the triangle records (identity order; precise:
+// the FP32 residuals too) and the longest edge.
+__global__ void k_grid_count(const float* __restrict__ vert, const float* __restrict__ vert_lo,
+                             const int* __restrict__ vot, int n, const float4* __restrict__ gv,
+                             GridDesc* __restrict__ gd, uint32_t* __restrict__ count,
+                             Tri* __restrict__ tris, float4* __restrict__ tri_lo) {
+  __shared__ unsigned smax;
+  if (threadIdx.x == 0) smax = 0u;
+  __syncthreads();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n && gd->ok) {
+    const GridDesc& g = *gd;
+    const int v0 = vot[3LL * t], v1 = vot[3LL * t + 1], v2 = vot[3LL * t + 2];
+    const float* p0 = vert + 3LL * v0;
+    const float* p1 = vert + 3LL * v1;
+    const float* p2 = vert + 3LL * v2;
+    Tri r;
+    r.x = make_float4(p0[0], p1[0], p2[0], __int_as_float(t));
+    r.y = make_float4(p0[1], p1[1], p2[1], 0.f);
+    r.z = make_float4(p0[2], p1[2], p2[2], 0.f);
+    tris[t] = r;
+    if (tri_lo) {
+      const float* q0 = vert_lo + 3LL * v0;
+      const float* q1 = vert_lo + 3LL * v1;
+      const float* q2 = vert_lo + 3LL * v2;
+      for (int k = 0; k < 3; k++) tri_lo[3LL * t + k] = make_float4(q0[k], q1[k], q2[k], 0.f);
+    }
+    auto len2 = [](float x, float y, float z) { return x * x + y * y + z * z; };
+    const float e = fmaxf(len2(r.x.y - r.x.x, r.y.y - r.y.x, r.z.y - r.z.x),
+                          fmaxf(len2(r.x.z - r.x.x, r.y.z - r.y.x, r.z.z - r.z.x),
+                                len2(r.x.z - r.x.y, r.y.z - r.y.y, r.z.z - r.z.y)));
+    atomicMax(&smax, __float_as_uint(sqrtf(e)));
+    for_cells(g, gv[v0], gv[v1], gv[v2], [&](int cell, float, float) {
+      atomicAdd(&count[cell], 1u);
+    });
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && smax) atomicMax(&gd->lmax, smax);
+}
+
+// (triangle, upper | lower height << 16) into each cell's list (triangles are
+// numbered through the domains of a call); count runs down from the cell's number of entries.
+__global__ void k_grid_fill(const int* __restrict__ vot, int n, int tri_base,
+                            const float4* __restrict__ gv, const GridDesc* __restrict__ gd, uint32_t* __restrict__ count,
+                            const uint32_t* __restrict__ start, uint2* __restrict__ refs,
+                            long long cap_refs, int* __restrict__ err) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n || !gd->ok) return;
+  const GridDesc& g = *gd;
+  bool over = false;
+  for_cells(g, gv[vot[3LL * t]], gv[vot[3LL * t + 1]], gv[vot[3LL * t + 2]],
+            [&](int cell, float up, float lo) {
+              const long long pos = (long long)start[cell] + atomicSub(&count[cell], 1u) - 1;
+              if (pos >= cap_refs) {
+                over = true;
+                return;
+              }
+              const float u = ceilf((up - g.hlo) * g.iq) + 1.f;
+              const float l = floorf((lo - g.hlo) * g.iq);
+              const unsigned hu = (unsigned)fminf(fmaxf(u, 1.f), 65535.f);
+              const unsigned hl = (unsigned)fminf(fmaxf(l, 0.f), 65535.f);
+              refs[pos] = make_uint2((unsigned)(tri_base + t), hu | (hl << 16));
+            });
+  if (over) atomicOr(err, kErrGrid);
+}
+
+// Level 0 of the pyramid: bounds of each cell's list (empty: 0 and 65535).
+__global__ void k_grid_heights(const GridDesc* __restrict__ gd, const uint32_t* __restrict__ start,
+                               const uint2* __restrict__ refs, long long cap_refs,
+                               uint16_t* __restrict__ top, uint16_t* __restrict__ low) {
+  if (!gd->ok) return;
+  const long long n0 = (long long)gd->W * gd->H;
+  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n0) return;
+  unsigned hi = 0u, lo = 0xFFFFu;
+  const long long e = min((long long)start[k + 1], cap_refs);
+  for (long long q = start[k]; q < e; q++) {
+    const unsigned w = refs[q].y;
+    hi = max(hi, w & 0xFFFFu);
+    lo = min(lo, w >> 16);
+  }
+  top[k] = (uint16_t)hi;
+  low[k] = (uint16_t)lo;
+}
+
+// Level l of the pyramid from level l - 2: a cell's children are one brick.
+__global__ void k_grid_up(const GridDesc* __restrict__ gd, int l, uint16_t* __restrict__ top,
+                          uint16_t* __restrict__ low) {
+  if (!gd->ok || l > gd->L) return;
+  const int W = gd->W, n2 = 2 * W * gd->H;
+  const int w = W >> l, h = gd->H >> l;
+  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= (long long)w * h) return;
+  const int b = (int)(k / w), a = (int)(k - (long long)b * w);
+  const int from = grid_index(W, n2, 4 * a, 4 * b, l - 2), to = grid_index(W, n2, a, b, l);
+  unsigned hi = 0u, lo = 0xFFFFFFFFu;
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    const uint4 u = *reinterpret_cast<const uint4*>(top + from + 8 * r);
+    const uint4 v = *reinterpret_cast<const uint4*>(low + from + 8 * r);
+    hi = __vmaxu2(hi, __vmaxu2(__vmaxu2(u.x, u.y), __vmaxu2(u.z, u.w)));
+    lo = __vminu2(lo, __vminu2(__vminu2(v.x, v.y), __vminu2(v.z, v.w)));
+  }
+  top[to] = (uint16_t)max(hi & 0xFFFFu, hi >> 16);
+  low[to] = (uint16_t)min(lo & 0xFFFFu, lo >> 16);
+}
+
+// ---------------------------------------------------------------------------
+// Cell frames
+// ---------------------------------------------------------------------------
+
+// FP64 frame of a cell (mo_lradtopo_horayzon.cpp:694-720, the expressions of
+// the other searches).
+struct CellFrame {
+  V3 normal, north, east;
+  double ox, oy, oz;
+};
+__device__ __forceinline__ CellFrame cell_frame64(const DomainDesc& D, int cell) {
+  CellFrame f;
+  const V3 q{D.cell_enu[3LL * cell], D.cell_enu[3LL * cell + 1], D.cell_enu[3LL * cell + 2]};
+  f.normal = V3{q.x - D.centre.x, q.y - D.centre.y, q.z - D.centre.z};
+  unit3(f.normal);
+  const V3 v_n{D.pole.x - q.x, D.pole.y - q.y, D.pole.z - q.z};
+  const double dp = dot3(v_n, f.normal);
+  f.north = V3{v_n.x - dp * f.normal.x, v_n.y - dp * f.normal.y, v_n.z - dp * f.normal.z};
+  unit3(f.north);
+  f.east = cross3(f.north, f.normal);
+  f.ox = q.x + f.normal.x * D.ray_org_elev;
+  f.oy = q.y + f.normal.y * D.ray_org_elev;
+  f.oz = q.z + f.normal.z * D.ray_org_elev;
+  return f;
+}
+
+// Ray of azimuth a and lattice elevation m: the direction of search_step.
+template <bool kPrecise>
+__device__ __forceinline__ Ray lattice_ray(const DomainDesc& D, const CellFrame& f, int a, int m,
+                                           double2& ecs) {
+  const double2 cs = __ldg(&D.azim_cs[a]);
+  const double hx = cs.x * f.north.x + cs.y * f.east.x;
+  const double hy = cs.x * f.north.y + cs.y * f.east.y;
+  const double hz = cs.x * f.north.z + cs.y * f.east.z;
+  if (m >= kElevMin && m < kElevMin + kElevTable) {
+    ecs = __ldg(&D.elev_cs[m - kElevMin]);
+  } else {
+    const double e = (double)m * D.two_ha;
+    ecs = make_double2(cos(e), sin(e));
+  }
+  const float dx = (float)(ecs.x * hx + ecs.y * f.normal.x);
+  const float dy = (float)(ecs.x * hy + ecs.y * f.normal.y);
+  const float dz = (float)(ecs.x * hz + ecs.y * f.normal.z);
+  const float ox = (float)f.ox, oy = (float)f.oy, oz = (float)f.oz;
+  if (kPrecise)
+    return make_ray(ox, oy, oz, dx, dy, dz, D.tfar, (float)(f.ox - (double)ox),
+                    (float)(f.oy - (double)oy), (float)(f.oz - (double)oz));
+  return make_ray(ox, oy, oz, dx, dy, dz, D.tfar);
+}
+
+// The watertight test of one lattice ray and one triangle, for the few
+// triangles the sweep's own arithmetic leaves undecided (p: work position).
+// The FP64 frame comes from its table: recomputing it (two square roots and
+// six divisions) took more of the FP64 pipe than the whole rest of the sweep.
+template <bool kPrecise>
+__device__ __noinline__ bool exact_hit(const DomainDesc* D, int p, int a, int m, int tri) {
+  const long long nc = D->ncell;
+  const double* fr = D->cell_frame + p;
+  const float* o = D->cell_f32 + p;
+  const double2 cs = __ldg(&D->azim_cs[a]);
+  const double2 ecs = __ldg(&D->elev_cs[m - kElevMin]);
+  const float dx = (float)(ecs.x * (cs.x * fr[3 * nc] + cs.y * fr[6 * nc]) + ecs.y * fr[0]);
+  const float dy = (float)(ecs.x * (cs.x * fr[4 * nc] + cs.y * fr[7 * nc]) + ecs.y * fr[nc]);
+  const float dz = (float)(ecs.x * (cs.x * fr[5 * nc] + cs.y * fr[8 * nc]) + ecs.y * fr[2 * nc]);
+  const Ray r = kPrecise ? make_ray(o[0], o[nc], o[2 * nc], dx, dy, dz, D->tfar, o[15 * nc],
+                                    o[16 * nc], o[17 * nc])
+                         : make_ray(o[0], o[nc], o[2 * nc], dx, dy, dz, D->tfar);
+  return test_tri<kPrecise>(D->tris, D->tri_lo, r, tri);
+}
+
+// FP32 frame table by work position: origin, normal, north, east, gnomonic
+// X, Y and height of the origin, and (precise) the origin's FP32 residual.
+constexpr int kFrameRows = 18;
+
+template <bool kPrecise>
+__global__ void k_sweep_frames(const DomainDesc* __restrict__ doms, int ndom,
+                               const int* __restrict__ order, int total) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= total) return;
+  const long long gid = order[k];
+  const DomainDesc& D = doms[domain_of(doms, ndom, gid)];
+  const int cell = (int)(gid - D.cell_offset);
+  const long long p = k - D.k_begin, nc = D.ncell;
+  const CellFrame f = cell_frame64(D, cell);
+  double* fr = D.cell_frame + p;
+  fr[0] = f.normal.x; fr[nc] = f.normal.y; fr[2 * nc] = f.normal.z;
+  fr[3 * nc] = f.north.x; fr[4 * nc] = f.north.y; fr[5 * nc] = f.north.z;
+  fr[6 * nc] = f.east.x; fr[7 * nc] = f.east.y; fr[8 * nc] = f.east.z;
+  float* o = D.cell_f32 + p;
+  const float ox = (float)f.ox, oy = (float)f.oy, oz = (float)f.oz;
+  o[0] = ox; o[nc] = oy; o[2 * nc] = oz;
+  o[3 * nc] = (float)f.normal.x; o[4 * nc] = (float)f.normal.y; o[5 * nc] = (float)f.normal.z;
+  o[6 * nc] = (float)f.north.x; o[7 * nc] = (float)f.north.y; o[8 * nc] = (float)f.north.z;
+  o[9 * nc] = (float)f.east.x; o[10 * nc] = (float)f.east.y; o[11 * nc] = (float)f.east.z;
+  const double dz = oz;
+  const float fz = __fdiv_rn(kRf, (float)(dz + kEarthRadius));
+  o[12 * nc] = ox * fz;
+  o[13 * nc] = oy * fz;
+  const double r2 = (double)ox * ox + (double)oy * oy + dz * (dz + 2.0 * kEarthRadius);
+  o[14 * nc] = __fdiv_rn((float)r2, sqrtf((float)(kEarthRadius * kEarthRadius + r2)) + kRf);
+  if (kPrecise) {
+    o[15 * nc] = (float)(f.ox - (double)ox);
+    o[16 * nc] = (float)(f.oy - (double)oy);
+    o[17 * nc] = (float)(f.oz - (double)oz);
+  }
+}
+
+// Track of one (cell, azimuth) on the grid, in metres s along the gnomonic
+// line: cell coordinates o + s d, the factors that turn s into lower / upper
+// bounds of the distance from the origin's normal (r sin psi), and the end of
+// the walk. tan(psi) = s gh / (lambda + s gu) with gh, gu the components of
+// the line's direction along h and u.
+struct Track {
+  float ox, oy, dx, dy, ix, iy;
+  float xlo, xhi;   // metres of horizontal distance per metre of s, times 1
+  float smax;
+};
+__device__ __forceinline__ Track make_track(const GridDesc& g, float X0, float Y0, float hx,
+                                            float hy, float hz, float ux, float uy) {
+  Track t;
+  const float kx = X0 * (1.f / kRf), ky = Y0 * (1.f / kRf);
+  float gx = __fmaf_rn(-kx, hz, hx), gy = __fmaf_rn(-ky, hz, hy);
+  const float n = rsqrtf(__fmaf_rn(gx, gx, gy * gy));
+  gx *= n;
+  gy *= n;
+  const float gh = __fmaf_rn(gx, hx, gy * hy), gu = __fmaf_rn(gx, ux, gy * uy);
+  const float lambda = sqrtf(__fmaf_rn(X0, X0, __fmaf_rn(Y0, Y0, kRf * kRf)));
+  t.smax = __fdividef(g.tau_max * lambda, fmaxf(__fmaf_rn(-g.tau_max, gu, gh), 1e-3f)) * 1.0001f +
+           2.f * g.pad;
+  const float a0 = __fdividef(gh, lambda);
+  const float a1 = __fdividef(gh, __fmaf_rn(t.smax, gu, lambda));
+  t.xlo = fminf(a0, a1) * (1.f - 4e-6f) * g.rlo;
+  t.xhi = fmaxf(a0, a1) * (1.f + 4e-6f) * g.rhi;
+  t.ox = (X0 - g.x0) * g.inv_c;
+  t.oy = (Y0 - g.y0) * g.inv_c;
+  t.dx = gx * g.inv_c;
+  t.dy = gy * g.inv_c;
+  t.ix = fabsf(t.dx) > 1e-25f ? __fdividef(1.f, t.dx) : (t.dx < 0.f ? -kBig : kBig);
+  t.iy = fabsf(t.dy) > 1e-25f ? __fdividef(1.f, t.dy) : (t.dy < 0.f ? -kBig : kBig);
+  return t;
+}
+
+// ---------------------------------------------------------------------------
+// The sweep
+// ---------------------------------------------------------------------------
+enum : int { kLaneAdvance = 0, kLaneWalk = 1, kLaneList = 2 };
+// Lane flags; kFlagAbove and kFlagRedo also come back from the triangle pass.
+enum : int { kFlagAny = 1, kFlagAbove = 2, kFlagRedo = 4, kFlagGap = 8, kFlagTested = 16,
+             kFlagRetry = 32 };
+
+// What the triangle pass needs of a thread's azimuth and cell, in shared
+// memory: any lane of the warp tests triangles for any other. Quadruples, read
+// in one access each:
+//   kRowOrigin   ray origin; error bound of the distances of the cell's triangles
+//   kRowSide     lateral axis h x u; height below which list entries do not reach the ray
+//   kRowRay      u - tan(e) h; tan(e) at the current elevation
+//   kRowAlong    horizontal direction h of the azimuth; bound of the distance at the cell's exit
+//   kRowUp       cell normal u; search radius
+//   kRowRest     precise: FP32 residual of the origin
+enum : int { kRowOrigin, kRowSide, kRowRay, kRowAlong, kRowUp, kRowRest };
+constexpr int kWarps = kSweepBlock / 32;
+
+// Triangle records, list entries, list starts and pyramids of all domains of
+// the call, one after another (DomainDesc::cell_base and ref_base).
+struct SweepScene {
+  const Tri* tris;
+  const float4* tri_lo;
+  const uint2* refs;
+  const uint32_t* gstart;
+  const uint16_t* top;
+};
+
+template <bool kPrecise>
+struct SweepShared {
+  // Odd numbers of quadruples: threads' rows fall on different banks.
+  float4 v[kSweepBlock][kPrecise ? 7 : 5];
+  float4 grid[kSweepBlock];            // of the thread's domain: unit, 2 pad, error distance
+  // Domain, cell, work position, azimuth, end azimuth, previous result,
+  // elevation; elevation and flags from the triangle pass.
+  int dom[kSweepBlock], cell[kSweepBlock], pos[kSweepBlock], az[kSweepBlock], az_end[kSweepBlock],
+      prev[kSweepBlock], m[kSweepBlock], m_new[kSweepBlock], flags[kSweepBlock];
+  int2 entry[kSweepBlock];             // per list in order: thread, first entry - its number
+  int2 queue[kWarps][64];              // (thread, triangle) to be cut with the plane
+  float tan_m[kTanTable];
+  int wq[2][kWarps];                   // next and end of the warp's chunk of items
+};
+
+// A triangle's vertices relative to the ray origin of thread o.
+template <bool kPrecise>
+__device__ __forceinline__ void load_relative(const SweepShared<kPrecise>& sh, int o,
+                                              const float4 org, const SweepScene& sc, int tri,
+                                              float3& a, float3& b, float3& c) {
+  const float4* tp = reinterpret_cast<const float4*>(sc.tris + tri);
+  const float4 X = __ldg(tp), Y = __ldg(tp + 1), Z = __ldg(tp + 2);
+  if (kPrecise) {
+    const float4* lo = sc.tri_lo + 3LL * tri;
+    const float4 LX = __ldg(lo), LY = __ldg(lo + 1), LZ = __ldg(lo + 2);
+    const float4 q = sh.v[o][kPrecise ? kRowRest : 0];
+    a = make_float3(rel(X.x, LX.x, org.x, q.x), rel(Y.x, LY.x, org.y, q.y),
+                    rel(Z.x, LZ.x, org.z, q.z));
+    b = make_float3(rel(X.y, LX.y, org.x, q.x), rel(Y.y, LY.y, org.y, q.y),
+                    rel(Z.y, LZ.y, org.z, q.z));
+    c = make_float3(rel(X.z, LX.z, org.x, q.x), rel(Y.z, LY.z, org.y, q.y),
+                    rel(Z.z, LZ.z, org.z, q.z));
+  } else {
+    a = make_float3(X.x - org.x, Y.x - org.y, Z.x - org.z);
+    b = make_float3(X.y - org.x, Y.y - org.y, Z.y - org.z);
+    c = make_float3(X.z - org.x, Y.z - org.y, Z.z - org.z);
+  }
+}
+__device__ __forceinline__ float dot3f(const float3 a, const float4 b) {
+  return __fmaf_rn(a.x, b.x, __fmaf_rn(a.y, b.y, a.z * b.z));
+}
+
+// Whether triangle tri may hide the current ray of thread o or a higher one:
+// not when its vertices lie on one side of the plane of the rays, nor all
+// below the ray, nor when both edges that cross the plane (those at the vertex
+// alone on its side) cross it below the ray, each by more than the bound of
+// the errors. An edge from (q0, h0) to (q1, h1) crosses at the height (h0 |q1| +
+// h1 |q0|) / (|q0| + |q1|).
+template <bool kPrecise>
+__device__ __forceinline__ bool may_hide(const SweepShared<kPrecise>& sh, int o,
+                                         const float4 side, const SweepScene& sc, int tri) {
+  float3 a, b, c;
+  const float4 org = sh.v[o][kRowOrigin];
+  load_relative(sh, o, org, sc, tri, a, b, c);
+  const float q0 = dot3f(a, side), q1 = dot3f(b, side), q2 = dot3f(c, side);
+  const float mu = org.w;
+  if (fminf(q0, fminf(q1, q2)) > mu || fmaxf(q0, fmaxf(q1, q2)) < -mu) return false;
+  const float4 ray = sh.v[o][kRowRay];
+  const float h0 = dot3f(a, ray), h1 = dot3f(b, ray), h2 = dot3f(c, ray);
+  const float mh = -mu * (1.f + fabsf(ray.w));
+  if (fmaxf(h0, fmaxf(h1, h2)) < mh) return false;
+  const bool p0 = q0 > 0.f, p1 = q1 > 0.f, p2 = q2 > 0.f;
+  if (p0 == p1 && p1 == p2) return true;  // touches the plane
+  const bool odd0 = p1 == p2, odd2 = p0 == p1;
+  const float qo = fabsf(odd0 ? q0 : (odd2 ? q2 : q1)), ho = odd0 ? h0 : (odd2 ? h2 : h1);
+  const float qa = fabsf(odd0 ? q1 : q0), ha = odd0 ? h1 : h0;
+  const float qb = fabsf(odd2 ? q1 : q2), hb = odd2 ? h1 : h2;
+  return !(__fmaf_rn(ho, qa, ha * qo) < 4.f * mh * (qo + qa + fabsf(ho - ha)) &&
+           __fmaf_rn(ho, qb, hb * qo) < 4.f * mh * (qo + qb + fabsf(ho - hb)));
+}
+
+// Cuts triangle tri with the plane of thread o's rays and compares the segment
+// with its current ray: nothing to do (below, beside, behind, out of reach or
+// past the cell), kFlagAbove (it stays above the ray), or a raise: m_new, the
+// lowest elevation it is not known to hide, with kFlagRedo when it may hide
+// that one too. Distances in the plane: x along h, heights over the ray times
+// 1 / cos(e), each with a bound of its error.
+template <bool kPrecise>
+__device__ __forceinline__ int cut_triangle(const SweepShared<kPrecise>& sh, int o,
+                                            const SweepScene& sc, const DomainDesc* doms,
+                                            int tri, int& m_new) {
+  float3 a, b, c;
+  const float4 org = sh.v[o][kRowOrigin], side = sh.v[o][kRowSide], ray = sh.v[o][kRowRay],
+               along = sh.v[o][kRowAlong];
+  load_relative(sh, o, org, sc, tri, a, b, c);
+  const float q0 = dot3f(a, side), q1 = dot3f(b, side), q2 = dot3f(c, side);
+  const float h0 = dot3f(a, ray), h1 = dot3f(b, ray), h2 = dot3f(c, ray);
+  const float x0 = dot3f(a, along), x1 = dot3f(b, along), x2 = dot3f(c, along);
+  const float e0 = kEps * (fabsf(a.x) + fabsf(a.y) + fabsf(a.z)),
+              e1 = kEps * (fabsf(b.x) + fabsf(b.y) + fabsf(b.z)),
+              e2 = kEps * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z));
+  const float ta = ray.w, ts = 1.f + fabsf(ta), xexit = along.w, tfar = sh.v[o][kRowUp].w;
+  const int m = sh.m[o];
+  // Vertices in the plane within rounding: one of them is an end point of the
+  // segment whichever side it is taken to be on (the cell's own vertex, under
+  // the ray origin, always is); two leave the segment open.
+  const bool n0 = fabsf(q0) <= e0, n1 = fabsf(q1) <= e1, n2 = fabsf(q2) <= e2;
+  const bool near = (n0 && n1) || (n0 && n2) || (n1 && n2);
+  const bool p0 = q0 > 0.f, p1 = q1 > 0.f, p2 = q2 > 0.f;
+  if (p0 == p1 && p1 == p2) {
+    // Beside the plane, or touching it in one vertex.
+    const float hv = n0 ? h0 : (n1 ? h1 : h2), ev = n0 ? e0 : (n1 ? e1 : e2);
+    if (!(n0 || n1 || n2) || (!near && hv < -2.f * ts * ev)) return 0;
+    m_new = m + 1;
+    return exact_hit<kPrecise>(doms + sh.dom[o], sh.pos[o], sh.az[o], m, tri) ? kFlagRedo : kFlagAbove;
+  }
+  // End points on the two edges at the vertex that lies alone on its side.
+  const int odd = p0 == p1 ? 2 : (p1 == p2 ? 0 : 1);
+  const float qo = fabsf(odd == 0 ? q0 : (odd == 1 ? q1 : q2));
+  const float qa = fabsf(odd == 0 ? q1 : q0), qb = fabsf(odd == 2 ? q1 : q2);
+  const float ho = odd == 0 ? h0 : (odd == 1 ? h1 : h2);
+  const float ha = odd == 0 ? h1 : h0, hb = odd == 2 ? h1 : h2;
+  const float xo = odd == 0 ? x0 : (odd == 1 ? x1 : x2);
+  const float xa = odd == 0 ? x1 : x0, xb = odd == 2 ? x1 : x2;
+  const float eo = odd == 0 ? e0 : (odd == 1 ? e1 : e2);
+  const float va = odd == 0 ? e1 : e0, vb = odd == 2 ? e1 : e2;
+  const float ra = __fdividef(1.f, fmaxf(qo + qa, 1e-30f)),
+              rb = __fdividef(1.f, fmaxf(qo + qb, 1e-30f));
+  const float ah = __fmaf_rn(ho, qa, ha * qo) * ra, bh = __fmaf_rn(ho, qb, hb * qo) * rb;
+  const float ax = __fmaf_rn(xo, qa, xa * qo) * ra, bx = __fmaf_rn(xo, qb, xb * qo) * rb;
+  const float fa = __fmaf_rn(eo, qa, va * qo) * ra, fb = __fmaf_rn(eo, qb, vb * qo) * rb;
+  const float ga = 2.f * fa * __fmaf_rn(fabsf(ho - ha), ra, 1.f),
+              gb = 2.f * fb * __fmaf_rn(fabsf(ho - hb), rb, 1.f);
+  const float ea = ts * ga, eb = ts * gb;
+  const float xea = 2.f * fa * __fmaf_rn(fabsf(xo - xa), ra, 1.f),
+              xeb = 2.f * fb * __fmaf_rn(fabsf(xo - xb), rb, 1.f);
+  if (!near && ah < -ea && bh < -eb) return 0;  // below
+  const float xmin = fminf(ax, bx) - fmaxf(xea, xeb);
+  if (fmaxf(ax, bx) < -fmaxf(xea, xeb) || xmin > xexit) return 0;
+  const float cs = sqrtf(__fmaf_rn(ta, ta, 1.f));
+  if (xmin * (ta > 0.f ? cs : 1.f) > tfar * 1.00001f) return 0;
+  bool above = !near && ah > ea && bh > eb;
+  if (!near && ((ah > ea && bh < -eb) || (ah < -ea && bh > eb))) {
+    // It crosses the ray's line, in front of the origin or behind it.
+    const float fh = fabsf(ah), gh = fabsf(bh), r2 = __fdividef(1.f, fh + gh);
+    const float xc = __fmaf_rn(ax, gh, bx * fh) * r2;
+    const float xe = 2.f * r2 * (__fmaf_rn(xea, gh, xeb * fh) +
+                                 fabsf(ax - bx) * r2 * __fmaf_rn(ea, gh, eb * fh));
+    if (xc < -xe) {
+      if ((ax > bx ? ah : bh) < 0.f) return 0;
+      above = true;
+    } else if (xc > xe && xc * cs < tfar * 0.99999f - xe) {
+      // Hidden, and with it every ray up to the segment's higher end.
+      const bool top = ah > 0.f;
+      const float th = top ? ah : bh, tx = top ? ax : bx, tg = top ? ga : gb;
+      m_new = m + 1;
+      if (!(tx > 0.f)) return kFlagRedo;
+      const float sl = __fmaf_rn(th, __fdividef(1.f, tx), ta);
+      const float te = 2.f * tg * (1.f + fmaxf(fabsf(ta), fabsf(sl)));
+      if (!(tx * sqrtf(__fmaf_rn(sl, sl, 1.f)) < tfar * 0.9999f)) return kFlagRedo;
+      const int k = max(m, min((int)floorf(atanf(sl) * 114.591559f), kMaxM));
+      const float* tm = sh.tan_m + kTanRange;
+      if (k > m && !(__fmaf_rn(ta - tm[k], tx, th) > te)) {
+        m_new = max(m + 1, k - 1);
+        return __fmaf_rn(ta - tm[m_new - 1], tx, th) > te ? kFlagRedo : (m_new = m + 1, kFlagRedo);
+      }
+      m_new = k + 1;
+      return __fmaf_rn(ta - tm[k + 1], tx, th) < -te ? kFlagAny : kFlagRedo;
+    }
+  }
+  if (!above) {
+    // Undecided: the watertight test.
+    if (exact_hit<kPrecise>(doms + sh.dom[o], sh.pos[o], sh.az[o], m, tri)) {
+      m_new = m + 1;
+      return kFlagRedo;
+    }
+    // Not hidden by it: is it below the next ray at least?
+    const float d = sh.tan_m[m + 1 + kTanRange] - ta;
+    if (!near && __fmaf_rn(-d, ax, ah) < -ea && __fmaf_rn(-d, bx, bh) < -eb) return 0;
+  }
+  // Above the ray: unless it begins past this cell (by the angle at the
+  // Earth's centre), where the walk meets it again.
+  const GridDesc& g = *doms[sh.dom[o]].grid;
+  const bool first = ax < bx;
+  const float xm = first ? ax : bx, ym = __fmaf_rn(ta, xm, first ? ah : bh);
+  const float ro = dot3f(make_float3(org.x, org.y, org.z + kRf), sh.v[o][kRowUp]);
+  if (!near && __fdividef(xm, ro + ym) * g.rhi > __fmaf_rn(1e-5f, xexit, xexit))
+    return 0;
+  return kFlagAbove;
+}
+
+template <bool kPrecise>
+__global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
+    k_sweep(const DomainDesc* __restrict__ doms, int ndom, const int* __restrict__ order,
+            int total, int* __restrict__ work, int s_full, int* __restrict__ list,
+            int* __restrict__ list_n, unsigned* __restrict__ listed, const SweepScene sc,
+            int* __restrict__ err) {
+  __shared__ SweepShared<kPrecise> sh;
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr int kUnknown = -30000;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const unsigned below_me = (1u << lane) - 1u;
+  if (*err & kErrGrid) return;  // set by the grid build: the caller searches with the tree
+  for (int k = t; k < kTanTable; k += kSweepBlock) sh.tan_m[k] = __ldg(&doms[0].tan_m[k]);
+  if (lane == 0) {
+    sh.wq[0][wid] = 0;
+    sh.wq[1][wid] = 0;
+  }
+  sh.az[t] = 0;
+  sh.az_end[t] = 0;
+  sh.dom[t] = 0;
+  __syncthreads();
+
+  bool alive = true;
+  int st = kLaneAdvance, fl = 0;
+  int m = 0, mstop = 1 << 20;
+  int i = 0, j = 0, l = 0;
+  float s = 0.f, s1 = 0.f, smax = 0.f;      // walk position, exit of the current cell, end
+  float ox = 0.f, oy = 0.f, dx = 0.f, dy = 0.f, ix = 0.f, iy = 0.f;
+  float xlo = 0.f, xhi = 0.f, kc = 0.f, cq = 0.f, ta = 0.f;
+  int W = 0, H = 0, ltop = 0, cell0 = 0, at = 0;
+
+  // Slope and plane normal of the ray at lattice elevation m.
+  auto set_elevation = [&]() {
+    ta = sh.tan_m[m + kTanRange];
+    const float4 h = sh.v[t][kRowAlong], u = sh.v[t][kRowUp];
+    sh.v[t][kRowRay] = make_float4(__fmaf_rn(-ta, h.x, u.x), __fmaf_rn(-ta, h.y, u.y),
+                                   __fmaf_rn(-ta, h.z, u.z), ta);
+    sh.m[t] = m;
+  };
+  // Height (as encoded in the lists) below which terrain between sa and sb
+  // does not reach the ray: at distance x a ray of slope tan(e) is x (tan(e) +
+  // x / 2r) above its origin's sphere at least, lowest at the near end when
+  // that rises and at the far end when it falls.
+  auto threshold = [&](float sa, float sb) {
+    const float T = __fmaf_rn(sa, kc, ta);
+    return __fmaf_rn(T, T >= 0.f ? sa * xlo : sb * xhi, cq);
+  };
+
+  for (;;) {
+    const unsigned live = __ballot_sync(kFull, alive);
+    if (live == 0u) break;
+    const unsigned waiting = __ballot_sync(kFull, alive && st == kLaneAdvance);
+    if (waiting != 0u && (__popc(waiting) >= HZ_SWEEP_ADVANCE || waiting == live)) {
+      const bool mine = alive && st == kLaneAdvance;
+      bool again = false;
+      if (mine && sh.az[t] < sh.az_end[t]) {
+        // An azimuth has ended.
+        const DomainDesc& D = doms[sh.dom[t]];
+        const int a = sh.az[t];
+        int code;
+        if (fl & kFlagGap) {
+          code = kCodeGap;
+        } else if (fl & kFlagAny) {
+          code = m;
+        } else if (m > s_full) {
+          // Nothing met the start's ray or any above it: start lower.
+          again = true;
+          mstop = m;
+          m = (fl & kFlagRetry) ? s_full : max(s_full, m - 4);
+          fl = kFlagRetry;
+        } else {
+          code = kCodeAllMiss;
+        }
+        if (!again) {
+          D.codes[(long long)a * D.ncell + sh.cell[t]] = (int16_t)code;
+          if (code == kCodeGap) {
+            const long long q = D.k_begin + sh.pos[t];
+            const unsigned bit = 1u << (q & 31);
+            if (!(atomicOr(&listed[q >> 5], bit) & bit)) list[atomicAdd(list_n, 1)] = (int)q;
+          }
+          sh.prev[t] = code > kCodeAllMiss ? code : kUnknown;
+          sh.az[t] = a + 1;
+          if (a + 1 == sh.az_end[t] && D.done) {
+            const unsigned long long fin = atomicAdd(&D.done[0], 1ull) + 1ull;
+            if (fin == (unsigned long long)D.ncell_traced * (unsigned long long)D.runs) {
+              unsigned long long now;
+              asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+              D.done[1] = now;
+            }
+          }
+        }
+      }
+      // New items for the lanes whose azimuths are done.
+      const unsigned starting = __ballot_sync(kFull, mine && sh.az[t] >= sh.az_end[t]);
+      if (starting != 0u) {
+        const int nreq = __popc(starting);
+        int first = 0, take = 0, nb = 0;
+        if (lane == 0) {
+          take = min(sh.wq[1][wid] - sh.wq[0][wid], nreq);
+          first = sh.wq[0][wid];
+          sh.wq[0][wid] += take;
+          if (take < nreq) {
+            // Near the end of the queue a warp takes only what it needs.
+            const int left = total - *(volatile int*)work;
+            const bool tail = left < (int)min(2147483647ll, (long long)gridDim.x * kWarps * 32);
+            const int grab = tail ? nreq - take : max(32, nreq - take);
+            nb = atomicAdd(work, grab);
+            sh.wq[0][wid] = nb + (nreq - take);
+            sh.wq[1][wid] = nb + grab;
+          }
+        }
+        first = __shfl_sync(kFull, first, 0);
+        take = __shfl_sync(kFull, take, 0);
+        nb = __shfl_sync(kFull, nb, 0);
+        if (starting >> lane & 1u) {
+          const int rank = __popc(starting & below_me);
+          const int item = rank < take ? first + rank : nb + (rank - take);
+          if (item >= total) {
+            alive = false;
+          } else {
+            const int dom = domain_of_item(doms, ndom, item);
+            const DomainDesc& D = doms[dom];
+            const unsigned local = (unsigned)(item - D.item_begin);
+            const unsigned run = local / (unsigned)D.ncell_traced;
+            const int p = (int)(local - run * (unsigned)D.ncell_traced);
+            const long long nc = D.ncell;
+            const float* fr = D.cell_f32 + p;
+            sh.v[t][kRowOrigin] = make_float4(fr[0], fr[nc], fr[2 * nc], 0.f);
+            sh.v[t][kRowUp] = make_float4(fr[3 * nc], fr[4 * nc], fr[5 * nc], D.tfar);
+            if (kPrecise)
+              sh.v[t][kPrecise ? kRowRest : 0] =
+                  make_float4(fr[15 * nc], fr[16 * nc], fr[17 * nc], 0.f);
+            const GridDesc& g = *D.grid;
+            cq = __fmaf_rn(fr[14 * nc] - g.hpad - g.hlo, g.iq, kMagic);
+            cell0 = D.cell_base;
+            sh.grid[t] = make_float4(g.unit, 2.f * g.pad, g.dadd + 2.f * __uint_as_float(g.lmax),
+                                     __uint_as_float(D.ref_base));
+            W = g.W;
+            H = g.H;
+            ltop = g.L;
+            sh.dom[t] = dom;
+            sh.cell[t] = (int)(order[D.k_begin + p] - D.cell_offset);
+            sh.pos[t] = p;
+            sh.az[t] = (int)(run * (unsigned)D.L / (unsigned)D.runs);
+            sh.az_end[t] = (int)((run + 1) * (unsigned)D.L / (unsigned)D.runs);
+            sh.prev[t] = kUnknown;
+          }
+        }
+      }
+      if (mine && alive) {
+        const DomainDesc& D = doms[sh.dom[t]];
+        const GridDesc& g = *D.grid;
+        if (!again) {
+          const int a = sh.az[t];
+          const int prev = sh.prev[t];
+          mstop = 1 << 20;
+          fl = 0;
+          // Two steps below the previous azimuth's result, or from the floor.
+          m = prev == kUnknown ? s_full : max(s_full, prev - 2);
+          if (D.start_m && (D.start_all || a % (D.L / D.groups) == 0)) {
+            const int m0 = clamp_start(D.start_m[(long long)a * D.ncell + sh.cell[t]]);
+            m = max(min(m, m0 - 1), 1 - kTanRange);
+            if (m0 > kMaxM) fl = kFlagGap;  // a start at the zenith: ray by ray
+          }
+          const double2 cs64 = __ldg(&D.azim_cs[a]);
+          const float c = (float)cs64.x, n = (float)cs64.y;
+          const long long nc = D.ncell;
+          const float* fr = D.cell_f32 + sh.pos[t];
+          const float hx = __fmaf_rn(c, fr[6 * nc], n * fr[9 * nc]);
+          const float hy = __fmaf_rn(c, fr[7 * nc], n * fr[10 * nc]);
+          const float hz = __fmaf_rn(c, fr[8 * nc], n * fr[11 * nc]);
+          const float4 u = sh.v[t][kRowUp];
+          const float ux = u.x, uy = u.y, uz = u.z;
+          sh.v[t][kRowAlong] = make_float4(hx, hy, hz, 0.f);
+          sh.v[t][kRowSide] = make_float4(__fmaf_rn(hy, uz, -hz * uy), __fmaf_rn(hz, ux, -hx * uz),
+                                          __fmaf_rn(hx, uy, -hy * ux), 0.f);
+          const Track tr = make_track(g, fr[12 * nc], fr[13 * nc], hx, hy, hz, ux, uy);
+          ox = tr.ox; oy = tr.oy; dx = tr.dx; dy = tr.dy; ix = tr.ix; iy = tr.iy;
+          smax = tr.smax;
+          xlo = tr.xlo * g.iq;
+          xhi = tr.xhi * g.iq;
+          kc = tr.xlo * g.cmin / g.rlo;
+        }
+        i = min(max((int)floorf(ox), 0), W - 1);
+        j = min(max((int)floorf(oy), 0), H - 1);
+        l = 0;
+        s = 0.f;
+        st = (fl & kFlagGap) ? kLaneAdvance : kLaneWalk;
+        set_elevation();
+      }
+    }
+
+    // Walk pass: pyramid steps while enough lanes walk. A step looks at the
+    // cell of level l at the walk's position: visible, it goes down (to the
+    // cell's list from level 0), else on to the next cell, and up a level where
+    // that one begins a cell of it.
+#pragma unroll 1
+    for (int q = 0; q < HZ_WALK_STEPS; q++) {
+      if (st == kLaneWalk) {
+        const int a = i >> l, b = j >> l;
+        at = grid_index(W, 2 * W * H, a, b, l);
+        const unsigned w = __ldg(sc.top + (2 * cell0 + at));
+        const int nx = (int)(__float_as_uint(dx) >> 31), ny = (int)(__float_as_uint(dy) >> 31);
+        const int bx = (a + 1 - nx) << l, by = (b + 1 - ny) << l;
+        const float tx = ((float)bx - ox) * ix, ty = ((float)by - oy) * iy;
+        s1 = fmaxf(s, fminf(fminf(tx, ty), smax));
+        const float thr = threshold(s, s1);
+        if (w != 0u && height_magic(w) >= thr && !(fl & kFlagTested)) {
+          if (l == 0) st = kLaneList;
+          l = max(l - 2, 0);
+        } else {
+          fl &= ~kFlagTested;
+          s = s1;
+          const bool xx = tx < ty;
+          const int top = (1 << l) - 1;
+          const int fi = min(max((int)floorf(__fmaf_rn(s, dx, ox)), a << l), (a << l) + top);
+          const int fj = min(max((int)floorf(__fmaf_rn(s, dy, oy)), b << l), (b << l) + top);
+          i = xx ? bx - nx : fi;
+          j = xx ? fj : by - ny;
+          if (((xx ? bx : by) & (3 << l)) == 0 && l < ltop) l += 2;
+          if (s >= smax || (unsigned)i >= (unsigned)W || (unsigned)j >= (unsigned)H)
+            st = kLaneAdvance;
+        }
+      }
+      if (__popc(__ballot_sync(kFull, st == kLaneWalk)) < HZ_WALK_MIN) break;
+    }
+
+    // Triangle pass: the lists of all lanes that reached a cell, their
+    // entries spread over the warp.
+    const unsigned lists = __ballot_sync(kFull, st == kLaneList);
+    if (lists == 0u) continue;
+    int n = 0;
+    unsigned k0 = 0;
+    if (st == kLaneList) {
+      const uint32_t k = __ldg(sc.gstart + (cell0 + at));
+      n = (int)(__ldg(sc.gstart + (cell0 + at + 1)) - k);
+      const float4 g = sh.grid[t];
+      const float xexit = s1 * xhi * g.x;
+      k0 = __float_as_uint(g.w) + k;
+      sh.v[t][kRowOrigin].w = kEps * __fmaf_rn(1.1f, xexit, g.z);
+      sh.v[t][kRowSide].w = threshold(s, s1);
+      sh.v[t][kRowAlong].w = xexit + g.y;
+      sh.m_new[t] = m;
+      sh.flags[t] = 0;
+    }
+    int off = n;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(kFull, off, d);
+      if (lane >= d) off += v;
+    }
+    const int entries = __shfl_sync(kFull, off, 31);
+    off -= n;
+    const unsigned filled = __ballot_sync(kFull, n > 0);
+    if (n > 0) sh.entry[wid * 32 + __popc(filled & below_me)] = make_int2(t, (int)k0 - off);
+    __syncwarp();
+    int queued = 0;
+    auto cut = [&](int count) {
+      if (lane < count) {
+        const int2 e = sh.queue[wid][lane];
+        int m_new = 0;
+        const int r = cut_triangle<kPrecise>(sh, e.x, sc, doms, e.y, m_new);
+        if (r == kFlagAbove) atomicOr(&sh.flags[e.x], kFlagAbove);
+        else if (r != 0) {
+          atomicMax(&sh.m_new[e.x], m_new);
+          if (r == kFlagRedo) atomicOr(&sh.flags[e.x], kFlagRedo);
+        }
+      }
+      __syncwarp();
+    };
+    for (int base = 0; base < entries; base += 32) {
+      // Lists that begin in this stretch mark their first entry; the rank of
+      // a list among all gives its owner.
+      const int rel0 = off - base;
+      const unsigned marks = __reduce_or_sync(
+          kFull, n > 0 && rel0 >= 0 && rel0 < 32 ? 1u << rel0 : 0u);
+      const int before = __popc(__ballot_sync(kFull, n > 0 && off < base));
+      const int x = base + lane;
+      bool want = false;
+      int o = 0, tri = 0;
+      if (x < entries) {
+        const int2 e = sh.entry[wid * 32 + before + __popc(marks & ((2u << lane) - 1u)) - 1];
+        o = e.x;
+        const uint2 rf = __ldg(sc.refs + (unsigned)(e.y + x));
+        const float4 side = sh.v[o][kRowSide];
+        if (height_magic(rf.y & 0xFFFFu) >= side.w) {
+          tri = (int)rf.x;
+          want = may_hide<kPrecise>(sh, o, side, sc, tri);
+        }
+      }
+      const unsigned wants = __ballot_sync(kFull, want);
+      if (want) sh.queue[wid][queued + __popc(wants & below_me)] = make_int2(o, tri);
+      queued += __popc(wants);
+      __syncwarp();
+      if (queued >= 32) {
+        cut(32);
+        queued -= 32;
+        const int2 e = sh.queue[wid][32 + lane];
+        __syncwarp();
+        if (lane < queued) sh.queue[wid][lane] = e;
+        __syncwarp();
+      }
+    }
+    if (queued > 0) cut(queued);
+    if (st == kLaneList) {
+      const int f = sh.flags[t], mn = sh.m_new[t];
+      if (mn > m) {
+        fl |= kFlagAny;
+        if (mn >= mstop) {
+          m = mstop;  // known to miss from the sweep above
+          st = kLaneAdvance;
+        } else if (mn > kMaxM) {
+          fl |= kFlagGap;
+          st = kLaneAdvance;
+        } else {
+          m = mn;
+          set_elevation();
+          // Triangles that were above the ray, or may hide the new one too:
+          // the list again.
+          if (!(f & (kFlagAbove | kFlagRedo))) {
+            fl |= kFlagTested;
+            st = kLaneWalk;
+          }
+        }
+      } else if (f & kFlagAbove) {
+        // A triangle stays above with nothing hiding the ray: the hits of this
+        // azimuth are not one run of elevations.
+        fl |= kFlagGap;
+        st = kLaneAdvance;
+      } else {
+        fl |= kFlagTested;
+        st = kLaneWalk;
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Ray by ray
+// ---------------------------------------------------------------------------
+
+// Any-hit query of one lattice ray on the grid.
+template <bool kPrecise>
+__device__ bool grid_ray(const DomainDesc& D, const GridDesc& g, const Ray& r, const Track& tr,
+                         float ho, float slope) {
+  const int W = g.W, H = g.H, n2 = 2 * W * H;
+  const float kl = tr.xlo * g.cmin / g.rlo, kh = tr.xhi * g.cmax / g.rlo;
+  const float cl = __fmaf_rn(ho - g.hpad - g.hlo, g.iq, kMagic);
+  const float ch = __fmaf_rn(ho + g.hpad - g.hlo, g.iq, kMagic + 2.f);
+  const float xlo = tr.xlo * g.iq, xhi = tr.xhi * g.iq;
+  int i = min(max((int)floorf(tr.ox), 0), W - 1);
+  int j = min(max((int)floorf(tr.oy), 0), H - 1);
+  int l = 0;
+  float s = 0.f;
+  bool tested = false;
+  for (;;) {
+    const int a = i >> l, b = j >> l;
+    const int at = grid_index(W, n2, a, b, l);
+    const unsigned hi = __ldg(D.top + at), lo = __ldg(D.low + at);
+    const bool sx = tr.dx > 0.f, sy = tr.dy > 0.f;
+    const float tx = ((float)((sx ? a + 1 : a) << l) - tr.ox) * tr.ix;
+    const float ty = ((float)((sy ? b + 1 : b) << l) - tr.oy) * tr.iy;
+    const float s1 = fmaxf(s, fminf(fminf(tx, ty), tr.smax));
+    // Lowest and highest height of the ray over [s, s1].
+    const float T0 = __fmaf_rn(s, kl, slope), T1 = __fmaf_rn(s1, kh, slope);
+    const float tlo = __fmaf_rn(T0, T0 >= 0.f ? s * xlo : s1 * xhi, cl);
+    const float thi = __fmaf_rn(T1, T1 >= 0.f ? s1 * xhi : s * xlo, ch);
+    const bool vis = hi != 0u && height_magic(hi) >= tlo && height_magic(lo) <= thi && !tested;
+    if (vis && l > 0) {
+      l -= 2;
+      continue;
+    }
+    if (vis) {
+      const unsigned e = D.gstart[at + 1];
+      for (unsigned k = D.gstart[at]; k < e; k++) {
+        const uint2 rf = __ldg(D.refs + k);
+        if (height_magic(rf.y & 0xFFFFu) < tlo || height_magic(rf.y >> 16) > thi) continue;
+        if (test_tri<kPrecise>(D.tris, D.tri_lo, r, (int)rf.x)) return true;
+      }
+      tested = true;
+      continue;
+    }
+    tested = false;
+    s = s1;
+    const bool xx = tx < ty;
+    int cross;
+    if (xx) {
+      cross = sx ? a + 1 : a;
+      i = sx ? cross << l : (cross << l) - 1;
+      j = min(max((int)floorf(__fmaf_rn(s, tr.dy, tr.oy)), b << l), ((b + 1) << l) - 1);
+    } else {
+      cross = sy ? b + 1 : b;
+      j = sy ? cross << l : (cross << l) - 1;
+      i = min(max((int)floorf(__fmaf_rn(s, tr.dx, tr.ox)), a << l), ((a + 1) << l) - 1);
+    }
+    if ((cross & 3) == 0 && l < g.L) l += 2;
+    if (s >= tr.smax || (unsigned)i >= (unsigned)W || (unsigned)j >= (unsigned)H) return false;
+  }
+}
+
+// The reference's search of one azimuth from (m, elev), given a lattice hit
+// pattern that ends at the lowest miss M (kCodeAllMiss: no hits) or, for a
+// code of k_sweep_repair, its stop. Returns true when it went up; n counts
+// the steps (one ray each after the first).
+__device__ __forceinline__ bool replay(int code, const DomainDesc& D, int& m, double& elev,
+                                       int& n) {
+  n = 0;
+  if (code >= kCodeStop) {
+    const int v = code - kCodeStop, stop = (v >> 1) - 2000;
+    if (v & 1) {
+      for (; m < stop; n++) {
+        m++;
+        elev += D.two_ha;
+      }
+      return true;
+    }
+    for (; m > stop; n++) {
+      m--;
+      elev -= D.two_ha;
+    }
+    return false;
+  }
+  if (m < code) {
+    for (; m < code; n++) {
+      m++;
+      elev += D.two_ha;
+    }
+    return true;
+  }
+  while (m >= code && elev > D.elev_floor) {
+    m--;
+    elev -= D.two_ha;
+    n++;
+  }
+  return false;
+}
+
+// First elevation of azimuth a: carried, or given (DomainDesc::start_m; 0 for
+// the first azimuth, cpp:511).
+__device__ __forceinline__ void chain_start(const DomainDesc& D, int cell, int a, int& m,
+                                            double& elev) {
+  if (a == 0) {
+    m = 0;
+    elev = 0.0;
+  }
+  if (D.start_m && (D.start_all || a % (D.L / D.groups) == 0)) {
+    m = clamp_start(D.start_m[(long long)a * D.ncell + cell]);
+    elev = (double)m * D.two_ha;
+  }
+}
+
+// A warp per listed cell: replays the cell's azimuths and searches the ones
+// left open by rays, 32 elevations at a time.
+template <bool kPrecise>
+__global__ void __launch_bounds__(128)
+    k_sweep_repair(const DomainDesc* __restrict__ doms, int ndom, const int* __restrict__ order,
+                   const int* __restrict__ list, const int* __restrict__ list_n,
+                   int* __restrict__ next, const int* __restrict__ err) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  if (*err & kErrGrid) return;
+  const int n = *list_n;
+  for (;;) {
+    int w = 0;
+    if (lane == 0) w = atomicAdd(next, 1);
+    w = __shfl_sync(kFull, w, 0);
+    if (w >= n) return;
+    const long long gid = order[list[w]];
+    const DomainDesc& D = doms[domain_of(doms, ndom, gid)];
+    const GridDesc& g = *D.grid;
+    const int cell = (int)(gid - D.cell_offset);
+    const CellFrame f = cell_frame64(D, cell);
+    const float ox = (float)f.ox, oy = (float)f.oy;
+    const double dz = (float)f.oz;
+    const float fz = __fdiv_rn(kRf, (float)(dz + kEarthRadius));
+    const double r2 = (double)ox * ox + (double)oy * oy + dz * (dz + 2.0 * kEarthRadius);
+    const float ho = __fdiv_rn((float)r2, sqrtf((float)(kEarthRadius * kEarthRadius + r2)) + kRf);
+    const float ux = (float)f.normal.x, uy = (float)f.normal.y;
+    int m = 0;
+    double elev = 0.0;
+    for (int a = 0; a < D.L; a++) {
+      chain_start(D, cell, a, m, elev);
+      int16_t* slot = D.codes + (long long)a * D.ncell + cell;
+      const int code = *slot;
+      int steps;
+      if (code != kCodeGap) {
+        replay(code, D, m, elev, steps);
+        continue;
+      }
+      const double2 cs = __ldg(&D.azim_cs[a]);
+      const float hx = (float)(cs.x * f.north.x + cs.y * f.east.x);
+      const float hy = (float)(cs.x * f.north.y + cs.y * f.east.y);
+      const float hz = (float)(cs.x * f.north.z + cs.y * f.east.z);
+      auto ray_hits = [&](int mm) {
+        double2 ecs;
+        const Ray r = lattice_ray<kPrecise>(D, f, a, mm, ecs);
+        // Beyond the zenith the ray runs along the opposite azimuth.
+        const float sg = ecs.x < 0.0 ? -1.f : 1.f;
+        const Track tr = make_track(g, ox * fz, oy * fz, sg * hx, sg * hy, sg * hz, ux, uy);
+        const float c = fmaxf(fabsf((float)ecs.x), 1e-7f);
+        return grid_ray<kPrecise>(D, g, r, tr, ho, __fdiv_rn((float)ecs.y, c));
+      };
+      // Lanes 0-15: m .. m + 15; lanes 16-31: m - 1 .. m - 16.
+      unsigned hits = __ballot_sync(kFull, ray_hits(lane < 16 ? m + lane : m - (lane - 15)));
+      bool up = hits & 1u;
+      if (up) {
+        int base = m, have = 16, left = kMaxUpSteps;
+        for (;;) {
+          const unsigned miss = ~hits & (have == 32 ? kFull : 0xFFFFu);
+          const int reach = miss ? __ffs(miss) - 1 : have;  // first miss at base + reach
+          const int to = min(base + reach, m + left);       // up to there
+          for (; m < to; left--) {
+            m++;
+            elev += D.two_ha;
+          }
+          if (miss || left == 0) break;
+          base += have;
+          have = 32;
+          hits = __ballot_sync(kFull, ray_hits(base + lane));
+        }
+      } else {
+        int base = m - 1, have = 16;
+        unsigned below = hits >> 16;
+        for (;;) {
+          bool hit = false;
+          int q = 0;
+          for (; q < have && elev > D.elev_floor && !hit; q++) {
+            m--;
+            elev -= D.two_ha;
+            hit = below >> q & 1u;
+          }
+          if (hit || !(elev > D.elev_floor)) break;
+          base -= have;
+          have = 32;
+          below = __ballot_sync(kFull, ray_hits(base - lane));
+        }
+      }
+      if (lane == 0) *slot = (int16_t)(kCodeStop + (((m + 2000) << 1) | (up ? 1 : 0)));
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Outputs
+// ---------------------------------------------------------------------------
+
+// The reference's search of every traced cell on its hit patterns: carried
+// elevations, clip, sector means, SVF sums, ray count (cpp:490-555, 736-754).
+template <bool kRefine1>
+__device__ __forceinline__ unsigned finish_sweep(const DomainDesc& D, int cell) {
+  const long long nc = D.ncell;
+  const float inv_ha = (float)(1.0 / D.hori_acc);
+  const double ha = D.hori_acc, refine = (double)D.refine;
+  const int span = D.L / D.groups;
+  int m = 0;
+  double elev = 0.0, sector = 0.0, svf = 0.0, part = 0.0;
+  unsigned rays = 0;
+  constexpr int kAhead = 8;
+  int in_sector = 0, row = 0, in_group = 0;
+  for (int a0 = 0; a0 < D.L; a0 += kAhead) {
+    int code[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; u++)
+      code[u] = a0 + u < D.L ? D.codes[(long long)(a0 + u) * nc + cell] : 0;
+#pragma unroll
+    for (int u = 0; u < kAhead; u++) {
+      const int a = a0 + u;
+      if (a >= D.L) break;
+      chain_start(D, cell, a, m, elev);
+      int steps;
+      const bool up = replay(code[u], D, m, elev, steps);
+      rays += 1u + (unsigned)steps;
+      double h = up ? elev - ha : elev + ha;
+      const int j = up ? 2 * m - 1 : 2 * m + 1;
+      if (D.raw_j) D.raw_j[(long long)a * nc + cell] = (int16_t)j;
+      if (h < 0.0) h = 0.0;
+      if (kRefine1) {
+        svf = svf + finish_svf_term(D, h, inv_ha);
+        D.horizon[(long long)a * nc + cell] = __dmul_rn(div_pi_rn(h), 180.0);
+      } else {
+        part = part + lattice_svf_term(D, h, j);
+        sector = sector + h;
+        if (++in_sector == D.refine) {
+          D.horizon[(long long)row * nc + cell] = __dmul_rn(div_pi_rn(sector), 180.0) / refine;
+          sector = 0.0;
+          in_sector = 0;
+          row++;
+        }
+        if (++in_group == span) {
+          svf = a + 1 == span ? part : svf + part;
+          part = 0.0;
+          in_group = 0;
+        }
+      }
+    }
+  }
+  D.skyview[cell] = svf / (double)D.L;
+  return rays;
+}
+
+__global__ void k_sweep_finish(const DomainDesc* __restrict__ doms, int ndom, int total,
+                               unsigned long long* __restrict__ counters,
+                               const int* __restrict__ err) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned long long rays = 0;
+  if (k < total && !(*err & kErrGrid)) {
+    int lo = 0, hi = ndom - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (doms[mid].k_begin <= k) lo = mid;
+      else hi = mid - 1;
+    }
+    const DomainDesc& D = doms[lo];
+    const int cell = D.cell_begin + (int)(k - D.k_begin);
+    rays = D.refine == 1 ? finish_sweep<true>(D, cell) : finish_sweep<false>(D, cell);
+  }
+  rays = warp_sum_u64(rays);
+  if ((threadIdx.x & 31) == 0 && rays) atomicAdd(&counters[0], rays);
+}
+
+}  // namespace
+
+long long sweep_cells_cap(long long n_tri) { return std::max(4096ll, 5 * n_tri / 2); }
+long long sweep_refs_cap(long long n_tri) { return 12 * n_tri + 4096; }
+size_t sweep_frame_floats() { return kFrameRows; }
+
+cudaError_t sweep_grid(const float* vert32, const float* vert_lo, const int* vot, int n_tri,
+                       int n_vert, int tri_base, float tfar, const SweepBuffers& b, Tri* tris,
+                       float4* tri_lo, int* err, cudaStream_t s) {
+  const long long cap0 = sweep_cells_cap(n_tri);
+  cudaError_t e = cudaMemsetAsync(b.count, 0, sizeof(uint32_t) * (size_t)(cap0 + 1), s);
+  if (e != cudaSuccess) return e;
+  k_grid_init<<<1, 1, 0, s>>>(b.bounds);
+  k_gnomonic<<<grid_for(n_vert, 256), 256, 0, s>>>(vert32, n_vert, b.gv, b.bounds);
+  k_grid_setup<<<1, 1, 0, s>>>(b.bounds, n_tri, cap0, tfar, b.grid, err);
+  note_launches(3);
+  if (n_tri > 0) {
+    k_grid_count<<<grid_for(n_tri, 256), 256, 0, s>>>(vert32, vert_lo, vot, n_tri, b.gv, b.grid,
+                                                      b.count, tris, vert_lo ? tri_lo : nullptr);
+    note_launches(1);
+  }
+  e = scan_exclusive_u32(b.count, b.start, cap0 + 1, b.total, b.partials, s);
+  if (e != cudaSuccess) return e;
+  if (n_tri > 0) {
+    k_grid_fill<<<grid_for(n_tri, 256), 256, 0, s>>>(vot, n_tri, tri_base, b.gv, b.grid, b.count, b.start,
+                                                     b.refs, sweep_refs_cap(n_tri), err);
+    note_launches(1);
+  }
+  k_grid_heights<<<grid_for(cap0, 256), 256, 0, s>>>(b.grid, b.start, b.refs,
+                                                     sweep_refs_cap(n_tri), b.top, b.low);
+  note_launches(1);
+  for (int l = 2; l <= 8; l += 2) {
+    k_grid_up<<<grid_for(cap0 >> (2 * l), 128), 128, 0, s>>>(b.grid, l, b.top, b.low);
+    note_launches(1);
+  }
+  return cudaGetLastError();
+}
+
+// Resident blocks of the sweep over the device, at most one per kSweepBlock items.
+template <typename... P, typename... A>
+static cudaError_t launch_resident(void (*kernel)(P...), int block, long long most,
+                                   cudaStream_t s, A... args) {
+  int dev = 0, sms = 0, per_sm = 0;
+  prefer_l1(kernel, HZ_SWEEP_MIN_BLOCKS);
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0);
+  long long blocks = (long long)sms * (per_sm > 0 ? per_sm : 1);
+  blocks = std::max(1ll, std::min(blocks, most));
+  kernel<<<(unsigned)blocks, block, 0, s>>>(args...);
+  note_launches(1);
+  return cudaGetLastError();
+}
+
+cudaError_t sweep_search(const DomainDesc* doms, int ndom, const int32_t* order, int total,
+                         int total_items, int s_full, int* work, int* list, unsigned* listed,
+                         const SweepAll& all, unsigned long long* counters, int* err,
+                         bool precise, cudaStream_t s) {
+  if (total <= 0 || ndom <= 0) return cudaSuccess;
+  // work[0] is reset by cell_order; work[1]: listed cells, work[2]: taken by the repair.
+  cudaError_t e = cudaMemsetAsync(work + 1, 0, 2 * sizeof(int), s);
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(listed, 0, sizeof(unsigned) * ((size_t)total / 32 + 1), s);
+  if (e != cudaSuccess) return e;
+  if (precise) k_sweep_frames<true><<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, order, total);
+  else k_sweep_frames<false><<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, order, total);
+  note_launches(1);
+  const SweepScene sc{all.tris, all.tri_lo, all.refs, all.start, all.top};
+  const long long most = ((long long)total_items + kSweepBlock - 1) / kSweepBlock;
+  e = precise ? launch_resident(k_sweep<true>, kSweepBlock, most, s, doms, ndom, order,
+                                total_items, work, s_full, list, work + 1, listed, sc, err)
+              : launch_resident(k_sweep<false>, kSweepBlock, most, s, doms, ndom, order,
+                                total_items, work, s_full, list, work + 1, listed, sc, err);
+  if (e != cudaSuccess) return e;
+  const long long warps = ((long long)total + 3) / 4;
+  e = precise ? launch_resident(k_sweep_repair<true>, 128, warps, s, doms, ndom, order, list,
+                                work + 1, work + 2, err)
+              : launch_resident(k_sweep_repair<false>, 128, warps, s, doms, ndom, order, list,
+                                work + 1, work + 2, err);
+  if (e != cudaSuccess) return e;
+  k_sweep_finish<<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, total, counters, err);
+  note_launches(1);
+  return cudaGetLastError();
+}
+
+}  // namespace hz

@@ -51,7 +51,13 @@ typedef struct hz_options {
     int32_t cell_begin;      /* trace only cells [cell_begin, cell_begin + cell_count); */
     int32_t cell_count;      /* cell_count <= 0: all cells. Other entries of horizon /
                                 skyview are left untouched (multi-GPU cell shards). */
-    int32_t kernel;          /* HZ_KERNEL_PERSISTENT (default) or HZ_KERNEL_PER_CELL */
+    int32_t kernel;          /* HZ_KERNEL_PERSISTENT (default) or HZ_KERNEL_PER_CELL. The
+                                default runs the profile sweep (one walk per cell and
+                                azimuth), and the tree search with the same results where
+                                an option of the tree is set (count_work, advance_min,
+                                leaf_min, leaf_size, queue_chunk, bvh_treelets, elev_walk,
+                                occluder_cache 0) or the domain is too wide for the
+                                sweep's projection */
     int32_t advance_min;     /* persistent kernel: lanes of a warp that must wait before
                                 the search state advances (1..32; 0 = library default) */
     int32_t precision;       /* HZ_PRECISION_REFERENCE (default) or HZ_PRECISION_LOCAL */

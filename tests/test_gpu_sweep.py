@@ -1,0 +1,121 @@
+"""The profile sweep against the tree search: the same lattice rays decide, so
+horizons, sky view factors and ray counts are the same bits. Cases at the edges
+of its ranges: one triangle fan, no triangle, cells under and beside the mesh,
+coarse grids whose search radius spans much of the domain, azimuth counts that
+do not divide into the sweep's runs, floors, cell ranges, given starts, and
+domains its grid cannot hold."""
+import numpy as np
+import pytest
+
+from horayzon_extpar_gb300 import horizon_svf_comp_py, synthetic
+from horayzon_extpar_gb300.horizon_svf import horizon_svf_comp_batch
+
+pytestmark = pytest.mark.gpu
+
+
+def _same(inputs, args, **kw):
+    # An explicit tree option selects the tree search.
+    h0, s0, st0 = horizon_svf_comp_py(*inputs, *args, return_stats=True, leaf_size=2, **kw)
+    h1, s1, st1 = horizon_svf_comp_py(*inputs, *args, return_stats=True, **kw)
+    assert np.array_equal(h0, h1, equal_nan=True)
+    assert np.array_equal(s0, s1, equal_nan=True)
+    assert st0["num_rays"] == st1["num_rays"]
+    assert st0["n_tri"] == st1["n_tri"]
+    return st0, st1
+
+
+@pytest.mark.parametrize("dkw,args,kw", [
+    # nearly every cell lies on the border and looks under the mesh's edge
+    (dict(edge_km=1.0, box_km=4.0, seed=1), (24, 1, 40000.0, 0.2, 1, 2), {}),
+    (dict(edge_km=1.0, box_km=6.0, seed=2), (7, 0, 1000.0, 0.1, 3, 0), {}),
+    # steep, fine terrain; azimuths that do not divide into runs
+    (dict(edge_km=0.1, box_km=8.0, seed=3, kind="eroded", hmin=0.0, hmax=3000.0),
+     (37, 1, 8000.0, 0.2, 1, 1), {}),
+    (dict(edge_km=0.1, box_km=5.0, seed=4, kind="eroded", hmin=0.0, hmax=2500.0),
+     (24, 0, 15000.0, 2.0, 2, 2), {"precision": 1}),
+    # coarse cells, a search radius of a quarter of the domain, high latitude
+    (dict(edge_km=40.0, box_km=2000.0, seed=5, hmax=6000.0, lat0_deg=70.0),
+     (24, 1, 500000.0, 0.2, 1, 2), {}),
+    (dict(edge_km=10.0, box_km=900.0, seed=6, lat0_deg=-33.0, lon0_deg=151.0,
+          face_rotation_deg=41.0), (48, 1, 100000.0, 0.2, 1, 0), {"precision": 1}),
+    # flat terrain: horizons decided by the smallest differences
+    (dict(edge_km=2.0, box_km=60.0, seed=7, hmin=100.0, hmax=100.0, n_features=0),
+     (24, 1, 40000.0, 0.1, 1, 2), {}),
+    # floors of the downward walk
+    (dict(edge_km=2.5, box_km=80.0, seed=8), (24, 1, 40000.0, 0.2, 1, 2),
+     {"elev_floor_deg": -0.25}),
+    (dict(edge_km=2.5, box_km=80.0, seed=8), (24, 1, 40000.0, 0.2, 1, 2),
+     {"elev_floor_deg": 7.3}),
+    # a range of cells
+    (dict(edge_km=1.0, box_km=40.0, seed=9), (24, 1, 20000.0, 0.2, 5, 1),
+     {"cells": (1001, 1778)}),
+])
+def test_gpu_sweep_is_the_tree_search(dkw, args, kw):
+    d = synthetic.make_domain(**dkw)
+    _same(d.inputs(), args, **kw)
+
+
+def test_gpu_sweep_without_triangles_and_with_one_fan():
+    d = synthetic.make_domain(edge_km=1.0, box_km=6.0, seed=11)
+    cov = np.full_like(d.cells_of_vertex, -2)
+    _same((*d.inputs()[:5], cov), (24, 1, 40000.0, 0.2, 1, 2))
+    full = np.nonzero((d.cells_of_vertex != -2).all(axis=0))[0][0]
+    cov[:, full] = d.cells_of_vertex[:, full]
+    for gt in (0, 1):
+        _same((*d.inputs()[:5], cov), (24, gt, 40000.0, 0.2, 1, 2))
+
+
+def test_gpu_sweep_with_holes_and_spikes():
+    """Patches of the mesh missing (rays pass under and through the edges) and
+    single cells a kilometre above their neighbours."""
+    d = synthetic.make_domain(edge_km=0.5, box_km=30.0, seed=12)
+    rng = np.random.default_rng(12)
+    clon, clat, h, vlon, vlat, cov = (np.array(a) for a in d.inputs())
+    cov[:, rng.random(cov.shape[1]) < 0.1] = -2
+    h[rng.random(h.size) < 0.01] += 1000.0
+    for gt in (0, 1):
+        _same((clon, clat, h, vlon, vlat, cov), (24, gt, 20000.0, 0.2, 1, 2))
+
+
+def test_gpu_sweep_falls_back_on_wide_domains():
+    """Cells around half the globe: the grid cannot hold them, the tree search
+    runs in its place."""
+    d = synthetic.make_domain(edge_km=2.0, box_km=30.0, seed=13)
+    clon, clat, h, vlon, vlat, cov = (np.array(a) for a in d.inputs())
+    n = clon.size // 2
+    clon[n:] += 2.0  # the second half of the cells 115 degrees further east
+    _same((clon, clat, h, vlon, vlat, cov), (12, 1, 20000.0, 0.2, 1, 2))
+    clon[n:] -= 0.7  # 75 degrees: the mean direction does not show it
+    _same((clon, clat, h, vlon, vlat, cov), (12, 1, 20000.0, 0.2, 1, 2))
+
+
+def test_gpu_sweep_batch_of_unlike_domains():
+    doms = [(synthetic.make_domain(edge_km=e, box_km=b, seed=s).inputs(),
+             (nh, gt, dist, 0.2, rf, sv))
+            for e, b, s, nh, gt, dist, rf, sv in
+            [(2.5, 20.0, 21, 24, 1, 40000.0, 1, 2), (0.2, 12.0, 22, 5, 0, 3000.0, 1, 0),
+             (1.0, 50.0, 23, 36, 1, 25000.0, 2, 1), (5.0, 300.0, 24, 16, 1, 90000.0, 1, 2)]]
+    tree = horizon_svf_comp_batch(doms, leaf_size=2)
+    for (h0, s0), (h1, s1) in zip(tree, horizon_svf_comp_batch(doms)):
+        assert np.array_equal(h0, h1) and np.array_equal(s0, s1)
+
+
+@pytest.mark.parametrize("groups,every", [(0, False), (4, False), (0, True)])
+def test_gpu_sweep_given_starts(groups, every):
+    torch = pytest.importorskip("torch")
+    from horayzon_extpar_gb300 import horizon_svf_comp_device
+    d = synthetic.make_domain(edge_km=0.2, box_km=12.0, seed=31, kind="eroded", hmax=2500.0)
+    t = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in d.inputs()]
+    args = (24, 1, 8000.0, 0.2, 2, 2)
+    g = torch.Generator().manual_seed(5)
+    start = torch.randint(-200, 200, (48, d.ncell), generator=g).to(torch.int16)
+    start[:, ::3] = torch.randint(-4, 12, start[:, ::3].shape, generator=g).to(torch.int16)
+    start = start.cuda()
+    out = []
+    for kw in ({"leaf_size": 2}, {}):
+        raw = torch.empty((48, d.ncell), dtype=torch.int16, device="cuda")
+        h, s, st = horizon_svf_comp_device(*t, *args, start_index=start, raw_index=raw,
+                                           mlp_azimuth_groups=groups, mlp_every_azimuth=every, **kw)
+        out.append((h, s, raw, st["num_rays"]))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    assert torch.equal(out[0][2], out[1][2]) and out[0][3] == out[1][3]
