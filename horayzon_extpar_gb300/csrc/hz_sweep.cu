@@ -77,6 +77,7 @@ constexpr float kMagic = 8388608.0f;      // 2^23: float(2^23 | n) = 2^23 + n
 constexpr float kBig = 1e30f;
 constexpr int kTanRange = 180;            // lattice elevations with a tangent: |m| < 180
 constexpr int kMaxM = 177;                // sweeps stop below 89 deg
+constexpr int kRunStart = -14;            // start of a run's first azimuth (-7 deg)
 
 // Codes of a (cell, azimuth): the lowest missing lattice elevation, or
 constexpr int kCodeAllMiss = -20000;      // no lattice ray meets the terrain
@@ -622,12 +623,29 @@ __device__ __forceinline__ int cut_triangle(const SweepShared<kPrecise>& sh, int
   const bool n0 = fabsf(q0) <= e0, n1 = fabsf(q1) <= e1, n2 = fabsf(q2) <= e2;
   const bool near = (n0 && n1) || (n0 && n2) || (n1 && n2);
   const bool p0 = q0 > 0.f, p1 = q1 > 0.f, p2 = q2 > 0.f;
-  if (p0 == p1 && p1 == p2) {
-    // Beside the plane, or touching it in one vertex.
-    const float hv = n0 ? h0 : (n1 ? h1 : h2), ev = n0 ? e0 : (n1 ? e1 : e2);
-    if (!(n0 || n1 || n2) || (!near && hv < -2.f * ts * ev)) return 0;
-    m_new = m + 1;
-    return exact_hit<kPrecise>(doms + sh.dom[o], sh.pos[o], sh.az[o], m, tri) ? kFlagRedo : kFlagAbove;
+  const bool beside = p0 == p1 && p1 == p2;
+  if (beside && !(n0 || n1 || n2)) return 0;
+  if (near || beside) {
+    // It meets the plane in an edge or in one vertex, if at all: nowhere but
+    // at the vertices in the plane and between them. Which of the triangles at
+    // such an edge a ray hits is the watertight test's to say.
+    const auto all = [&](auto f) {
+      return (!n0 || f(h0, x0, e0)) && (!n1 || f(h1, x1, e1)) && (!n2 || f(h2, x2, e2));
+    };
+    if (all([&](float h, float, float e) { return h < -2.f * ts * e; }) ||
+        all([&](float, float x, float e) { return x < -2.f * e; }) ||
+        all([&](float, float x, float e) { return x - 2.f * e > xexit; }))
+      return 0;
+    int k = m;
+    while (k <= kMaxM && exact_hit<kPrecise>(doms + sh.dom[o], sh.pos[o], sh.az[o], k, tri)) k++;
+    if (k > m) {
+      m_new = k;
+      return kFlagRedo;
+    }
+    const float tn = sh.tan_m[m + 1 + kTanRange];
+    return all([&](float h, float x, float e) {
+      return __fmaf_rn(ta - tn, x, h) < -2.f * (1.f + fabsf(tn)) * e;
+    }) ? 0 : kFlagAbove;
   }
   // End points on the two edges at the vertex that lies alone on its side.
   const int odd = p0 == p1 ? 2 : (p1 == p2 ? 0 : 1);
@@ -649,13 +667,13 @@ __device__ __forceinline__ int cut_triangle(const SweepShared<kPrecise>& sh, int
   const float ea = ts * ga, eb = ts * gb;
   const float xea = 2.f * fa * __fmaf_rn(fabsf(xo - xa), ra, 1.f),
               xeb = 2.f * fb * __fmaf_rn(fabsf(xo - xb), rb, 1.f);
-  if (!near && ah < -ea && bh < -eb) return 0;  // below
+  if (ah < -ea && bh < -eb) return 0;  // below
   const float xmin = fminf(ax, bx) - fmaxf(xea, xeb);
   if (fmaxf(ax, bx) < -fmaxf(xea, xeb) || xmin > xexit) return 0;
   const float cs = sqrtf(__fmaf_rn(ta, ta, 1.f));
   if (xmin * (ta > 0.f ? cs : 1.f) > tfar * 1.00001f) return 0;
-  bool above = !near && ah > ea && bh > eb;
-  if (!near && ((ah > ea && bh < -eb) || (ah < -ea && bh > eb))) {
+  bool above = ah > ea && bh > eb;
+  if ((ah > ea && bh < -eb) || (ah < -ea && bh > eb)) {
     // It crosses the ray's line, in front of the origin or behind it.
     const float fh = fabsf(ah), gh = fabsf(bh), r2 = __fdividef(1.f, fh + gh);
     const float xc = __fmaf_rn(ax, gh, bx * fh) * r2;
@@ -691,7 +709,7 @@ __device__ __forceinline__ int cut_triangle(const SweepShared<kPrecise>& sh, int
     }
     // Not hidden by it: is it below the next ray at least?
     const float d = sh.tan_m[m + 1 + kTanRange] - ta;
-    if (!near && __fmaf_rn(-d, ax, ah) < -ea && __fmaf_rn(-d, bx, bh) < -eb) return 0;
+    if (__fmaf_rn(-d, ax, ah) < -ea && __fmaf_rn(-d, bx, bh) < -eb) return 0;
   }
   // Above the ray: unless it begins past this cell (by the angle at the
   // Earth's centre), where the walk meets it again.
@@ -699,7 +717,7 @@ __device__ __forceinline__ int cut_triangle(const SweepShared<kPrecise>& sh, int
   const bool first = ax < bx;
   const float xm = first ? ax : bx, ym = __fmaf_rn(ta, xm, first ? ah : bh);
   const float ro = dot3f(make_float3(org.x, org.y, org.z + kRf), sh.v[o][kRowUp]);
-  if (!near && __fdividef(xm, ro + ym) * g.rhi > __fmaf_rn(1e-5f, xexit, xexit))
+  if (__fdividef(xm, ro + ym) * g.rhi > __fmaf_rn(1e-5f, xexit, xexit))
     return 0;
   return kFlagAbove;
 }
@@ -712,7 +730,7 @@ __global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
             int* __restrict__ err) {
   __shared__ SweepShared<kPrecise> sh;
   constexpr unsigned kFull = 0xffffffffu;
-  constexpr int kUnknown = -30000;
+  constexpr int kUnknown = -30000, kFirst = -30001;
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
   const unsigned below_me = (1u << lane) - 1u;
   if (*err & kErrGrid) return;  // set by the grid build: the caller searches with the tree
@@ -849,7 +867,7 @@ __global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
             sh.pos[t] = p;
             sh.az[t] = (int)(run * (unsigned)D.L / (unsigned)D.runs);
             sh.az_end[t] = (int)((run + 1) * (unsigned)D.L / (unsigned)D.runs);
-            sh.prev[t] = kUnknown;
+            sh.prev[t] = sh.az[t] == 0 ? 2 : kFirst;  // the search starts at 0 (cpp:511)
           }
         }
       }
@@ -861,8 +879,10 @@ __global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
           const int prev = sh.prev[t];
           mstop = 1 << 20;
           fl = 0;
-          // Two steps below the previous azimuth's result, or from the floor.
-          m = prev == kUnknown ? s_full : max(s_full, prev - 2);
+          // Two steps below the previous azimuth's result; a run's first azimuth
+          // well below any horizon of its neighbourhood (k_sweep_runs checks
+          // that the search came from no lower); else from the floor.
+          m = prev == kUnknown ? s_full : max(s_full, (prev == kFirst ? kRunStart + 2 : prev) - 2);
           if (D.start_m && (D.start_all || a % (D.L / D.groups) == 0)) {
             const int m0 = clamp_start(D.start_m[(long long)a * D.ncell + sh.cell[t]]);
             m = max(min(m, m0 - 1), 1 - kTanRange);
@@ -1104,6 +1124,30 @@ __device__ bool grid_ray(const DomainDesc& D, const GridDesc& g, const Ray& r, c
   }
 }
 
+// The first azimuth of every run but a cell's first was swept from kRunStart:
+// where the search can come to it from below that (the azimuth before has no
+// hits from there up, or is open), the cell goes to the repair.
+__global__ void k_sweep_runs(const DomainDesc* __restrict__ doms, int ndom, int total,
+                             int* __restrict__ list, int* __restrict__ list_n,
+                             unsigned* __restrict__ listed, const int* __restrict__ order,
+                             const int* __restrict__ err) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= total || (*err & kErrGrid)) return;
+  const long long gid = order[k];
+  const DomainDesc& D = doms[domain_of(doms, ndom, gid)];
+  const int cell = (int)(gid - D.cell_offset);
+  bool open = false;
+  for (int r = 1; r < D.runs; r++) {
+    const int a = (int)((unsigned)r * (unsigned)D.L / (unsigned)D.runs);
+    const int16_t* c = D.codes + (long long)a * D.ncell + cell;
+    open |= *c > kCodeAllMiss && c[-(long long)D.ncell] <= kRunStart + 1;
+  }
+  if (open) {
+    const unsigned bit = 1u << (k & 31);
+    if (!(atomicOr(&listed[k >> 5], bit) & bit)) list[atomicAdd(list_n, 1)] = k;
+  }
+}
+
 // The reference's search of one azimuth from (m, elev), given a lattice hit
 // pattern that ends at the lowest miss M (kCodeAllMiss: no hits) or, for a
 // code of k_sweep_repair, its stop. Returns true when it went up; n counts
@@ -1161,7 +1205,7 @@ template <bool kPrecise>
 __global__ void __launch_bounds__(128)
     k_sweep_repair(const DomainDesc* __restrict__ doms, int ndom, const int* __restrict__ order,
                    const int* __restrict__ list, const int* __restrict__ list_n,
-                   int* __restrict__ next, const int* __restrict__ err) {
+                   int* __restrict__ next, int s_full, const int* __restrict__ err) {
   constexpr unsigned kFull = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   if (*err & kErrGrid) return;
@@ -1182,14 +1226,23 @@ __global__ void __launch_bounds__(128)
     const double r2 = (double)ox * ox + (double)oy * oy + dz * (dz + 2.0 * kEarthRadius);
     const float ho = __fdiv_rn((float)r2, sqrtf((float)(kEarthRadius * kEarthRadius + r2)) + kRf);
     const float ux = (float)f.normal.x, uy = (float)f.normal.y;
-    int m = 0;
+    int m = 0, run = 0, before = 0;
     double elev = 0.0;
     for (int a = 0; a < D.L; a++) {
       chain_start(D, cell, a, m, elev);
       int16_t* slot = D.codes + (long long)a * D.ncell + cell;
       const int code = *slot;
       int steps;
-      if (code != kCodeGap) {
+      // Where this azimuth's sweep began: the hits below that are not known.
+      int from = s_full;
+      if ((int)((unsigned)run * (unsigned)D.L / (unsigned)D.runs) == a) {
+        from = a == 0 ? 0 : max(s_full, kRunStart);
+        run++;
+      } else if (before > kCodeAllMiss) {
+        from = max(s_full, before - 2);
+      }
+      before = code;
+      if (code != kCodeGap && (m >= from || code == kCodeAllMiss)) {
         replay(code, D, m, elev, steps);
         continue;
       }
@@ -1398,11 +1451,16 @@ cudaError_t sweep_search(const DomainDesc* doms, int ndom, const int32_t* order,
               : launch_resident(k_sweep<false>, kSweepBlock, most, s, doms, ndom, order,
                                 total_items, work, s_full, list, work + 1, listed, sc, err);
   if (e != cudaSuccess) return e;
+  if (total_items > total) {
+    k_sweep_runs<<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, total, list, work + 1, listed,
+                                                      order, err);
+    note_launches(1);
+  }
   const long long warps = ((long long)total + 3) / 4;
   e = precise ? launch_resident(k_sweep_repair<true>, 128, warps, s, doms, ndom, order, list,
-                                work + 1, work + 2, err)
+                                work + 1, work + 2, s_full, err)
               : launch_resident(k_sweep_repair<false>, 128, warps, s, doms, ndom, order, list,
-                                work + 1, work + 2, err);
+                                work + 1, work + 2, s_full, err);
   if (e != cudaSuccess) return e;
   k_sweep_finish<<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, total, counters, err);
   note_launches(1);
