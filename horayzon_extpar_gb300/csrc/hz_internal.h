@@ -149,7 +149,7 @@ struct GridDesc {
   float pad;                  // margin by which triangles are grown
   float hlo, iq, unit;        // heights as integers: (h - hlo) * iq, iq = 1 / unit
   float hpad;                 // margin of a ray's height
-  float rlo, rhi;             // radii of the lowest and highest vertex
+  float rlo, rhi, irlo;       // radii of the lowest and highest vertex, 1 / rlo
   float tau_max;              // tangent of the search radius' angle at the centre
   float cmin, cmax;           // bounds of the curvature term's factor
   float dadd;                 // bound of a triangle's distance beyond the walk's

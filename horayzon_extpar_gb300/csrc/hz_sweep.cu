@@ -40,9 +40,9 @@
 // Against the tree search (GB300, whole call): one traversal of a bounding
 // volume tree per ray took 2.5 to 4 rays, 63 to 126 four-wide node visits and 38
 // to 76 triangle tests per evaluation; the sweep takes 53 to 90 two-byte steps and
-// 20 to 40 tests. 500 m, 3.1M cells 135.5 -> 102.3 ms; 100 m, 1.2M cells 107.9 ->
-// 77.4 ms; 2.5 km, 57k cells 8.0 -> 3.0 ms; 500 cells 5.3 -> 1.9 ms; 360 azimuths,
-// 21k cells 56.4 -> 13.9 ms. The small domains gain most: a sweep from the floor
+// 20 to 40 tests. 500 m, 3.1M cells 130.7 -> 91.0 ms; 100 m, 1.2M cells 117.5 ->
+// 68.5 ms; 2.5 km, 57k cells 8.3 -> 2.2 ms; 500 cells 5.3 -> 1.0 ms; 360 azimuths,
+// 21k cells 57.6 -> 13.4 ms. The small domains gain most: a sweep from the floor
 // needs no other azimuth's result, so a cell's azimuths run side by side.
 #include <algorithm>
 
@@ -54,8 +54,14 @@ namespace hz {
 namespace {
 
 constexpr int kSweepBlock = 128;
+// Resident blocks per SM: 6 of 80 registers (1.2M cells at 100 m: 70.6 ms with 5, 67.4
+// with 6, spills from 7 on: 31 ms against 26 of a 300 km domain); 5 of 96 where
+// the watertight test recomputes rays in FP64 (10.0 ms, 11.6 with 6).
 #ifndef HZ_SWEEP_MIN_BLOCKS
-#define HZ_SWEEP_MIN_BLOCKS 5
+#define HZ_SWEEP_MIN_BLOCKS 6
+#endif
+#ifndef HZ_SWEEP_MIN_BLOCKS_EXACT
+#define HZ_SWEEP_MIN_BLOCKS_EXACT 5
 #endif
 #ifndef HZ_WALK_STEPS
 #define HZ_WALK_STEPS 8  // pyramid steps per lane in one walk pass
@@ -71,10 +77,12 @@ constexpr int kSweepBlock = 128;
 #endif
 
 constexpr float kRf = 6371229.0f;         // kEarthRadius, exact in FP32
-constexpr float kEps = 9.5367431640625e-07f;  // 2^-20: relative error bound of a vertex's
-                                              // FP32 distances, 4 x the sum of its roundings
+// Bound of the error of a vertex's FP32 distances from the plane and over the
+// ray, over its distance (1-norm) from the origin: with u = 2^-24, 12 u of the
+// sweep's own (axes 5 u a component, coordinates u, sums 3 u) and 7 u of the
+// watertight test (sheared coordinates 6 u, direction 1 u).
+constexpr float kEps = 1.28e-6f;
 constexpr float kMagic = 8388608.0f;      // 2^23: float(2^23 | n) = 2^23 + n
-constexpr float kBig = 1e30f;
 constexpr int kTanRange = 180;            // lattice elevations with a tangent: |m| < 180
 constexpr int kMaxM = 177;                // sweeps stop below 89 deg
 constexpr int kRunStart = -14;            // start of a run's first azimuth (-7 deg)
@@ -164,6 +172,7 @@ __global__ void k_grid_setup(const unsigned* __restrict__ b, int n_tri, long lon
   q.dadd = 2.f * c + 4.f * pad + (h1 - h0) + 1.f;
   q.rlo = kRf + h0;
   q.rhi = kRf + h1;
+  q.irlo = 1.f / q.rlo;
   const float s = fminf(tfar / q.rlo, 0.5f);
   q.tau_max = s / sqrtf(1.f - s * s) * 1.0001f;
   q.cmin = (q.rlo / q.rhi) * (1.f - 0.25f * q.tau_max * q.tau_max) * 0.5f;
@@ -465,12 +474,12 @@ __global__ void k_sweep_frames(const DomainDesc* __restrict__ doms, int ndom,
 // the walk. tan(psi) = s gh / (lambda + s gu) with gh, gu the components of
 // the line's direction along h and u.
 struct Track {
-  float ox, oy, dx, dy, ix, iy;
+  float ox, oy, dx, dy;
   float xlo, xhi;   // metres of horizontal distance per metre of s, times 1
   float smax;
 };
 __device__ __forceinline__ Track make_track(const GridDesc& g, float X0, float Y0, float hx,
-                                            float hy, float hz, float ux, float uy) {
+                                            float hy, float hz, float ux, float uy, float uz) {
   Track t;
   const float kx = X0 * (1.f / kRf), ky = Y0 * (1.f / kRf);
   float gx = __fmaf_rn(-kx, hz, hx), gy = __fmaf_rn(-ky, hz, hy);
@@ -478,7 +487,7 @@ __device__ __forceinline__ Track make_track(const GridDesc& g, float X0, float Y
   gx *= n;
   gy *= n;
   const float gh = __fmaf_rn(gx, hx, gy * hy), gu = __fmaf_rn(gx, ux, gy * uy);
-  const float lambda = sqrtf(__fmaf_rn(X0, X0, __fmaf_rn(Y0, Y0, kRf * kRf)));
+  const float lambda = __fdividef(kRf, uz);  // |(X0, Y0, R)|, along u
   t.smax = __fdividef(g.tau_max * lambda, fmaxf(__fmaf_rn(-g.tau_max, gu, gh), 1e-3f)) * 1.0001f +
            2.f * g.pad;
   const float a0 = __fdividef(gh, lambda);
@@ -489,8 +498,9 @@ __device__ __forceinline__ Track make_track(const GridDesc& g, float X0, float Y
   t.oy = (Y0 - g.y0) * g.inv_c;
   t.dx = gx * g.inv_c;
   t.dy = gy * g.inv_c;
-  t.ix = fabsf(t.dx) > 1e-25f ? __fdividef(1.f, t.dx) : (t.dx < 0.f ? -kBig : kBig);
-  t.iy = fabsf(t.dy) > 1e-25f ? __fdividef(1.f, t.dy) : (t.dy < 0.f ? -kBig : kBig);
+  // Never 0: the distance to the next column or row stays finite.
+  if (fabsf(t.dx) < 1e-12f) t.dx = t.dx < 0.f ? -1e-12f : 1e-12f;
+  if (fabsf(t.dy) < 1e-12f) t.dy = t.dy < 0.f ? -1e-12f : 1e-12f;
   return t;
 }
 
@@ -510,8 +520,12 @@ enum : int { kFlagAny = 1, kFlagAbove = 2, kFlagRedo = 4, kFlagGap = 8, kFlagTes
 //   kRowRay      u - tan(e) h; tan(e) at the current elevation
 //   kRowAlong    horizontal direction h of the azimuth; bound of the distance at the cell's exit
 //   kRowUp       cell normal u; search radius
+//   kRowTrack    track: origin and direction in grid cells
+//   kRowHeight   a ray's height at s: T s (y if T >= 0 else z) + w, T = s x + tan(e)
 //   kRowRest     precise: FP32 residual of the origin
-enum : int { kRowOrigin, kRowSide, kRowRay, kRowAlong, kRowUp, kRowRest };
+// The walk reads its own thread's track anew in each pass: kept in registers
+// through the triangle pass they cost a quarter of the resident warps.
+enum : int { kRowOrigin, kRowSide, kRowRay, kRowAlong, kRowUp, kRowTrack, kRowHeight, kRowRest };
 constexpr int kWarps = kSweepBlock / 32;
 
 // Triangle records, list entries, list starts and pyramids of all domains of
@@ -527,12 +541,16 @@ struct SweepScene {
 template <bool kPrecise>
 struct SweepShared {
   // Odd numbers of quadruples: threads' rows fall on different banks.
-  float4 v[kSweepBlock][kPrecise ? 7 : 5];
+  float4 v[kSweepBlock][kPrecise ? 9 : 7];
   float4 grid[kSweepBlock];            // of the thread's domain: unit, 2 pad, error distance
+  int4 size[kSweepBlock];              // its columns, rows, highest level, first cell
+  float smax[kSweepBlock];             // end of the walk
+  int mstop[kSweepBlock];              // elevation known to miss
   // Domain, cell, work position, azimuth, end azimuth, previous result,
   // elevation; elevation and flags from the triangle pass.
   int dom[kSweepBlock], cell[kSweepBlock], pos[kSweepBlock], az[kSweepBlock], az_end[kSweepBlock],
       prev[kSweepBlock], m[kSweepBlock], m_new[kSweepBlock], flags[kSweepBlock];
+  float reach[kSweepBlock];            // the search radius times cos(e)
   int2 entry[kSweepBlock];             // per list in order: thread, first entry - its number
   int2 queue[kWarps][64];              // (thread, triangle) to be cut with the plane
   float tan_m[kTanTable];
@@ -591,8 +609,8 @@ __device__ __forceinline__ bool may_hide(const SweepShared<kPrecise>& sh, int o,
   const float qo = fabsf(odd0 ? q0 : (odd2 ? q2 : q1)), ho = odd0 ? h0 : (odd2 ? h2 : h1);
   const float qa = fabsf(odd0 ? q1 : q0), ha = odd0 ? h1 : h0;
   const float qb = fabsf(odd2 ? q1 : q2), hb = odd2 ? h1 : h2;
-  return !(__fmaf_rn(ho, qa, ha * qo) < 4.f * mh * (qo + qa + fabsf(ho - ha)) &&
-           __fmaf_rn(ho, qb, hb * qo) < 4.f * mh * (qo + qb + fabsf(ho - hb)));
+  return !(__fmaf_rn(ho, qa, ha * qo) < 2.f * mh * (qo + qa + fabsf(ho - ha)) &&
+           __fmaf_rn(ho, qb, hb * qo) < 2.f * mh * (qo + qb + fabsf(ho - hb)));
 }
 
 // Cuts triangle tri with the plane of thread o's rays and compares the segment
@@ -615,101 +633,118 @@ __device__ __forceinline__ int cut_triangle(const SweepShared<kPrecise>& sh, int
   const float e0 = kEps * (fabsf(a.x) + fabsf(a.y) + fabsf(a.z)),
               e1 = kEps * (fabsf(b.x) + fabsf(b.y) + fabsf(b.z)),
               e2 = kEps * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z));
-  const float ta = ray.w, ts = 1.f + fabsf(ta), xexit = along.w, tfar = sh.v[o][kRowUp].w;
+  const float ta = ray.w, ts = 1.f + fabsf(ta), xexit = along.w, reach = sh.reach[o];
+  const float* tm = sh.tan_m + kTanRange;
   const int m = sh.m[o];
   // Vertices in the plane within rounding: one of them is an end point of the
   // segment whichever side it is taken to be on (the cell's own vertex, under
   // the ray origin, always is); two leave the segment open.
   const bool n0 = fabsf(q0) <= e0, n1 = fabsf(q1) <= e1, n2 = fabsf(q2) <= e2;
-  const bool near = (n0 && n1) || (n0 && n2) || (n1 && n2);
   const bool p0 = q0 > 0.f, p1 = q1 > 0.f, p2 = q2 > 0.f;
   const bool beside = p0 == p1 && p1 == p2;
-  if (beside && !(n0 || n1 || n2)) return 0;
-  if (near || beside) {
+  const bool edge = beside || (n0 && n1) || (n0 && n2) || (n1 && n2);
+  float ah = 0.f, bh = 0.f, ax = 0.f, bx = 0.f, ea = 0.f, eb = 0.f;
+  bool decided = false;  // above for certain; else the watertight test is asked
+  const auto all = [&](auto f) {
+    return (!n0 || f(h0, x0, e0)) && (!n1 || f(h1, x1, e1)) && (!n2 || f(h2, x2, e2));
+  };
+  if (edge) {
     // It meets the plane in an edge or in one vertex, if at all: nowhere but
     // at the vertices in the plane and between them. Which of the triangles at
     // such an edge a ray hits is the watertight test's to say.
-    const auto all = [&](auto f) {
-      return (!n0 || f(h0, x0, e0)) && (!n1 || f(h1, x1, e1)) && (!n2 || f(h2, x2, e2));
-    };
-    if (all([&](float h, float, float e) { return h < -2.f * ts * e; }) ||
-        all([&](float, float x, float e) { return x < -2.f * e; }) ||
-        all([&](float, float x, float e) { return x - 2.f * e > xexit; }))
+    if ((beside && !(n0 || n1 || n2)) ||
+        all([&](float h, float, float e) { return h < -ts * e; }) ||
+        all([&](float, float x, float e) { return x < -e; }) ||
+        all([&](float, float x, float e) { return x - e > xexit; }))
       return 0;
+  } else {
+    // End points on the two edges at the vertex that lies alone on its side.
+    const bool odd0 = p1 == p2, odd2 = p0 == p1;
+    const float qo = fabsf(odd0 ? q0 : (odd2 ? q2 : q1));
+    const float qa = fabsf(odd0 ? q1 : q0), qb = fabsf(odd2 ? q1 : q2);
+    const float ho = odd0 ? h0 : (odd2 ? h2 : h1);
+    const float ha = odd0 ? h1 : h0, hb = odd2 ? h1 : h2;
+    const float xo = odd0 ? x0 : (odd2 ? x2 : x1);
+    const float xa = odd0 ? x1 : x0, xb = odd2 ? x1 : x2;
+    const float eo = odd0 ? e0 : (odd2 ? e2 : e1);
+    const float va = odd0 ? e1 : e0, vb = odd2 ? e1 : e2;
+    const float ra = __fdividef(1.f, qo + qa), rb = __fdividef(1.f, qo + qb);
+    ah = __fmaf_rn(ho, qa, ha * qo) * ra;
+    bh = __fmaf_rn(ho, qb, hb * qo) * rb;
+    ax = __fmaf_rn(xo, qa, xa * qo) * ra;
+    bx = __fmaf_rn(xo, qb, xb * qo) * rb;
+    const float fa = ra * __fmaf_rn(eo, qa, va * qo), fb = rb * __fmaf_rn(eo, qb, vb * qo);
+    const float ga = __fmaf_rn(fa * ra, fabsf(ho - ha), fa),
+                gb = __fmaf_rn(fb * rb, fabsf(ho - hb), fb);
+    ea = ts * ga;
+    eb = ts * gb;
+    const float xea = __fmaf_rn(fa * ra, fabsf(xo - xa), fa),
+                xeb = __fmaf_rn(fb * rb, fabsf(xo - xb), fb);
+    const float xem = fmaxf(xea, xeb), xmin = fminf(ax, bx) - xem;
+    // Below, behind, past the cell (its own cell follows), out of reach. (The
+    // reach along x is that of the ray for rising ones, whose higher
+    // neighbours reach less far, and the radius itself for falling ones.)
+    if ((ah < -ea && bh < -eb) || fmaxf(ax, bx) < -xem || xmin > xexit ||
+        xmin > 1.00001f * (ta > 0.f ? reach : sh.v[o][kRowUp].w))
+      return 0;
+    decided = ah > ea && bh > eb;
+    if ((ah > ea && bh < -eb) || (ah < -ea && bh > eb)) {
+      // It crosses the ray's line, in front of the origin or behind it.
+      const float fh = fabsf(ah), gh = fabsf(bh), r2 = __fdividef(1.f, fh + gh);
+      const float xc = __fmaf_rn(ax, gh, bx * fh) * r2;
+      const float xe = 2.f * r2 * (__fmaf_rn(xea, gh, xeb * fh) +
+                                   fabsf(ax - bx) * r2 * __fmaf_rn(ea, gh, eb * fh));
+      if (xc < -xe) {
+        if ((ax > bx ? ah : bh) < 0.f) return 0;
+        decided = true;
+      } else if (xc > xe && xc < reach * 0.99999f - xe) {
+        // Hidden, and with it every ray up to the segment's higher end.
+        const bool top = ah > 0.f;
+        const float th = top ? ah : bh, tx = top ? ax : bx, tg = top ? ga : gb;
+        m_new = m + 1;
+        if (!(tx > 0.f)) return kFlagRedo;
+        // Ray k is hidden where it passes the higher end below it by more than
+        // the error te and within the radius (so do all between m and k then):
+        // it meets the segment between ray m's crossing and that end.
+        const float far2 = 0.999f * sh.v[o][kRowUp].w * sh.v[o][kRowUp].w;
+        const float tx2 = fmaxf(tx, xc) * fmaxf(tx, xc);
+        float v = 0.f, te = 0.f;
+        const auto hides = [&](int k) {
+          const float tk = tm[k];
+          v = __fmaf_rn(ta - tk, tx, th);
+          te = tg * (1.f + fabsf(ta) + fabsf(tk));
+          return v > te && __fmaf_rn(tx2 * tk, tk, tx2) < far2;
+        };
+        int k = m;
+        if (__fmaf_rn(ta - tm[min(m + 4, kMaxM)], tx, th) > 0.f) {  // far up: near the end at once
+          k = max(m, min((int)floorf(atanf(__fmaf_rn(th, __fdividef(1.f, tx), ta)) * 114.591559f),
+                         kMaxM) - 1);
+          if (k > m && !hides(k)) return kFlagRedo;
+        }
+        while (hides(k + 1) && k < kMaxM) k++;
+        m_new = k + 1;
+        return v < -te ? kFlagAny : kFlagRedo;
+      }
+    }
+  }
+  if (!decided) {
+    // Undecided: the watertight test (along an edge, as many rays as it hides);
+    // and, where it does not hide this one, whether it is below the next.
     int k = m;
-    while (k <= kMaxM && exact_hit<kPrecise>(doms + sh.dom[o], sh.pos[o], sh.az[o], k, tri)) k++;
+    while (k <= kMaxM && (edge || k == m) &&
+           exact_hit<kPrecise>(doms + sh.dom[o], sh.pos[o], sh.az[o], k, tri))
+      k++;
     if (k > m) {
       m_new = k;
       return kFlagRedo;
     }
-    const float tn = sh.tan_m[m + 1 + kTanRange];
-    return all([&](float h, float x, float e) {
-      return __fmaf_rn(ta - tn, x, h) < -2.f * (1.f + fabsf(tn)) * e;
-    }) ? 0 : kFlagAbove;
-  }
-  // End points on the two edges at the vertex that lies alone on its side.
-  const int odd = p0 == p1 ? 2 : (p1 == p2 ? 0 : 1);
-  const float qo = fabsf(odd == 0 ? q0 : (odd == 1 ? q1 : q2));
-  const float qa = fabsf(odd == 0 ? q1 : q0), qb = fabsf(odd == 2 ? q1 : q2);
-  const float ho = odd == 0 ? h0 : (odd == 1 ? h1 : h2);
-  const float ha = odd == 0 ? h1 : h0, hb = odd == 2 ? h1 : h2;
-  const float xo = odd == 0 ? x0 : (odd == 1 ? x1 : x2);
-  const float xa = odd == 0 ? x1 : x0, xb = odd == 2 ? x1 : x2;
-  const float eo = odd == 0 ? e0 : (odd == 1 ? e1 : e2);
-  const float va = odd == 0 ? e1 : e0, vb = odd == 2 ? e1 : e2;
-  const float ra = __fdividef(1.f, fmaxf(qo + qa, 1e-30f)),
-              rb = __fdividef(1.f, fmaxf(qo + qb, 1e-30f));
-  const float ah = __fmaf_rn(ho, qa, ha * qo) * ra, bh = __fmaf_rn(ho, qb, hb * qo) * rb;
-  const float ax = __fmaf_rn(xo, qa, xa * qo) * ra, bx = __fmaf_rn(xo, qb, xb * qo) * rb;
-  const float fa = __fmaf_rn(eo, qa, va * qo) * ra, fb = __fmaf_rn(eo, qb, vb * qo) * rb;
-  const float ga = 2.f * fa * __fmaf_rn(fabsf(ho - ha), ra, 1.f),
-              gb = 2.f * fb * __fmaf_rn(fabsf(ho - hb), rb, 1.f);
-  const float ea = ts * ga, eb = ts * gb;
-  const float xea = 2.f * fa * __fmaf_rn(fabsf(xo - xa), ra, 1.f),
-              xeb = 2.f * fb * __fmaf_rn(fabsf(xo - xb), rb, 1.f);
-  if (ah < -ea && bh < -eb) return 0;  // below
-  const float xmin = fminf(ax, bx) - fmaxf(xea, xeb);
-  if (fmaxf(ax, bx) < -fmaxf(xea, xeb) || xmin > xexit) return 0;
-  const float cs = sqrtf(__fmaf_rn(ta, ta, 1.f));
-  if (xmin * (ta > 0.f ? cs : 1.f) > tfar * 1.00001f) return 0;
-  bool above = ah > ea && bh > eb;
-  if ((ah > ea && bh < -eb) || (ah < -ea && bh > eb)) {
-    // It crosses the ray's line, in front of the origin or behind it.
-    const float fh = fabsf(ah), gh = fabsf(bh), r2 = __fdividef(1.f, fh + gh);
-    const float xc = __fmaf_rn(ax, gh, bx * fh) * r2;
-    const float xe = 2.f * r2 * (__fmaf_rn(xea, gh, xeb * fh) +
-                                 fabsf(ax - bx) * r2 * __fmaf_rn(ea, gh, eb * fh));
-    if (xc < -xe) {
-      if ((ax > bx ? ah : bh) < 0.f) return 0;
-      above = true;
-    } else if (xc > xe && xc * cs < tfar * 0.99999f - xe) {
-      // Hidden, and with it every ray up to the segment's higher end.
-      const bool top = ah > 0.f;
-      const float th = top ? ah : bh, tx = top ? ax : bx, tg = top ? ga : gb;
-      m_new = m + 1;
-      if (!(tx > 0.f)) return kFlagRedo;
-      const float sl = __fmaf_rn(th, __fdividef(1.f, tx), ta);
-      const float te = 2.f * tg * (1.f + fmaxf(fabsf(ta), fabsf(sl)));
-      if (!(tx * sqrtf(__fmaf_rn(sl, sl, 1.f)) < tfar * 0.9999f)) return kFlagRedo;
-      const int k = max(m, min((int)floorf(atanf(sl) * 114.591559f), kMaxM));
-      const float* tm = sh.tan_m + kTanRange;
-      if (k > m && !(__fmaf_rn(ta - tm[k], tx, th) > te)) {
-        m_new = max(m + 1, k - 1);
-        return __fmaf_rn(ta - tm[m_new - 1], tx, th) > te ? kFlagRedo : (m_new = m + 1, kFlagRedo);
-      }
-      m_new = k + 1;
-      return __fmaf_rn(ta - tm[k + 1], tx, th) < -te ? kFlagAny : kFlagRedo;
-    }
-  }
-  if (!above) {
-    // Undecided: the watertight test.
-    if (exact_hit<kPrecise>(doms + sh.dom[o], sh.pos[o], sh.az[o], m, tri)) {
-      m_new = m + 1;
-      return kFlagRedo;
-    }
-    // Not hidden by it: is it below the next ray at least?
-    const float d = sh.tan_m[m + 1 + kTanRange] - ta;
-    if (__fmaf_rn(-d, ax, ah) < -ea && __fmaf_rn(-d, bx, bh) < -eb) return 0;
+    const float tn = tm[m + 1], d = ta - tn;
+    if (edge ? all([&](float h, float x, float e) {
+          return __fmaf_rn(d, x, h) < -(1.f + fabsf(tn)) * e;
+        })
+             : __fmaf_rn(d, ax, ah) < -ea && __fmaf_rn(d, bx, bh) < -eb)
+      return 0;
+    if (edge) return kFlagAbove;
   }
   // Above the ray: unless it begins past this cell (by the angle at the
   // Earth's centre), where the walk meets it again.
@@ -717,13 +752,12 @@ __device__ __forceinline__ int cut_triangle(const SweepShared<kPrecise>& sh, int
   const bool first = ax < bx;
   const float xm = first ? ax : bx, ym = __fmaf_rn(ta, xm, first ? ah : bh);
   const float ro = dot3f(make_float3(org.x, org.y, org.z + kRf), sh.v[o][kRowUp]);
-  if (__fdividef(xm, ro + ym) * g.rhi > __fmaf_rn(1e-5f, xexit, xexit))
-    return 0;
-  return kFlagAbove;
+  return __fdividef(xm, ro + ym) * g.rhi > __fmaf_rn(1e-5f, xexit, xexit) ? 0 : kFlagAbove;
 }
 
 template <bool kPrecise>
-__global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
+__global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EXACT
+                                                      : HZ_SWEEP_MIN_BLOCKS)
     k_sweep(const DomainDesc* __restrict__ doms, int ndom, const int* __restrict__ order,
             int total, int* __restrict__ work, int s_full, int* __restrict__ list,
             int* __restrict__ list_n, unsigned* __restrict__ listed, const SweepScene sc,
@@ -746,12 +780,10 @@ __global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
 
   bool alive = true;
   int st = kLaneAdvance, fl = 0;
-  int m = 0, mstop = 1 << 20;
+  int m = 0;
   int i = 0, j = 0, l = 0;
-  float s = 0.f, s1 = 0.f, smax = 0.f;      // walk position, exit of the current cell, end
-  float ox = 0.f, oy = 0.f, dx = 0.f, dy = 0.f, ix = 0.f, iy = 0.f;
-  float xlo = 0.f, xhi = 0.f, kc = 0.f, cq = 0.f, ta = 0.f;
-  int W = 0, H = 0, ltop = 0, cell0 = 0, at = 0;
+  float s = 0.f, s1 = 0.f, ta = 0.f;        // walk position, exit of the current cell, tan(e)
+  int at = 0;
 
   // Slope and plane normal of the ray at lattice elevation m.
   auto set_elevation = [&]() {
@@ -760,14 +792,15 @@ __global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
     sh.v[t][kRowRay] = make_float4(__fmaf_rn(-ta, h.x, u.x), __fmaf_rn(-ta, h.y, u.y),
                                    __fmaf_rn(-ta, h.z, u.z), ta);
     sh.m[t] = m;
+    sh.reach[t] = u.w * rsqrtf(__fmaf_rn(ta, ta, 1.f));
   };
   // Height (as encoded in the lists) below which terrain between sa and sb
   // does not reach the ray: at distance x a ray of slope tan(e) is x (tan(e) +
   // x / 2r) above its origin's sphere at least, lowest at the near end when
   // that rises and at the far end when it falls.
-  auto threshold = [&](float sa, float sb) {
-    const float T = __fmaf_rn(sa, kc, ta);
-    return __fmaf_rn(T, T >= 0.f ? sa * xlo : sb * xhi, cq);
+  auto threshold = [&](const float4 hc, float sa, float sb) {
+    const float T = __fmaf_rn(sa, hc.x, ta);
+    return __fmaf_rn(T, T >= 0.f ? sa * hc.y : sb * hc.z, hc.w);
   };
 
   for (;;) {
@@ -789,7 +822,7 @@ __global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
         } else if (m > s_full) {
           // Nothing met the start's ray or any above it: start lower.
           again = true;
-          mstop = m;
+          sh.mstop[t] = m;
           m = (fl & kFlagRetry) ? s_full : max(s_full, m - 4);
           fl = kFlagRetry;
         } else {
@@ -855,13 +888,10 @@ __global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
               sh.v[t][kPrecise ? kRowRest : 0] =
                   make_float4(fr[15 * nc], fr[16 * nc], fr[17 * nc], 0.f);
             const GridDesc& g = *D.grid;
-            cq = __fmaf_rn(fr[14 * nc] - g.hpad - g.hlo, g.iq, kMagic);
-            cell0 = D.cell_base;
+            sh.v[t][kRowHeight].w = __fmaf_rn(fr[14 * nc] - g.hpad - g.hlo, g.iq, kMagic);
             sh.grid[t] = make_float4(g.unit, 2.f * g.pad, g.dadd + 2.f * __uint_as_float(g.lmax),
                                      __uint_as_float(D.ref_base));
-            W = g.W;
-            H = g.H;
-            ltop = g.L;
+            sh.size[t] = make_int4(g.W, g.H, g.L, D.cell_base);
             sh.dom[t] = dom;
             sh.cell[t] = (int)(order[D.k_begin + p] - D.cell_offset);
             sh.pos[t] = p;
@@ -877,7 +907,7 @@ __global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
         if (!again) {
           const int a = sh.az[t];
           const int prev = sh.prev[t];
-          mstop = 1 << 20;
+          sh.mstop[t] = 1 << 20;
           fl = 0;
           // Two steps below the previous azimuth's result; a run's first azimuth
           // well below any horizon of its neighbourhood (k_sweep_runs checks
@@ -900,15 +930,15 @@ __global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
           sh.v[t][kRowAlong] = make_float4(hx, hy, hz, 0.f);
           sh.v[t][kRowSide] = make_float4(__fmaf_rn(hy, uz, -hz * uy), __fmaf_rn(hz, ux, -hx * uz),
                                           __fmaf_rn(hx, uy, -hy * ux), 0.f);
-          const Track tr = make_track(g, fr[12 * nc], fr[13 * nc], hx, hy, hz, ux, uy);
-          ox = tr.ox; oy = tr.oy; dx = tr.dx; dy = tr.dy; ix = tr.ix; iy = tr.iy;
-          smax = tr.smax;
-          xlo = tr.xlo * g.iq;
-          xhi = tr.xhi * g.iq;
-          kc = tr.xlo * g.cmin / g.rlo;
+          const Track tr = make_track(g, fr[12 * nc], fr[13 * nc], hx, hy, hz, ux, uy, uz);
+          sh.v[t][kRowTrack] = make_float4(tr.ox, tr.oy, tr.dx, tr.dy);
+          sh.v[t][kRowHeight].x = tr.xlo * g.cmin * g.irlo;
+          sh.v[t][kRowHeight].y = tr.xlo * g.iq;
+          sh.v[t][kRowHeight].z = tr.xhi * g.iq;
+          sh.smax[t] = tr.smax;
         }
-        i = min(max((int)floorf(ox), 0), W - 1);
-        j = min(max((int)floorf(oy), 0), H - 1);
+        i = min(max((int)floorf(sh.v[t][kRowTrack].x), 0), sh.size[t].x - 1);
+        j = min(max((int)floorf(sh.v[t][kRowTrack].y), 0), sh.size[t].y - 1);
         l = 0;
         s = 0.f;
         st = (fl & kFlagGap) ? kLaneAdvance : kLaneWalk;
@@ -920,17 +950,24 @@ __global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
     // cell of level l at the walk's position: visible, it goes down (to the
     // cell's list from level 0), else on to the next cell, and up a level where
     // that one begins a cell of it.
+    {
+    const float4 tr = sh.v[t][kRowTrack], hc = sh.v[t][kRowHeight];
+    const int4 size = sh.size[t];
+    const float smax = sh.smax[t];
+    const int W = size.x, n2 = 2 * size.x * size.y;
+    const uint16_t* top = sc.top + 2 * (long long)size.w;
+    const int nx = (int)(__float_as_uint(tr.z) >> 31), ny = (int)(__float_as_uint(tr.w) >> 31);
+    const float ix = __fdividef(1.f, tr.z), iy = __fdividef(1.f, tr.w);
 #pragma unroll 1
     for (int q = 0; q < HZ_WALK_STEPS; q++) {
       if (st == kLaneWalk) {
         const int a = i >> l, b = j >> l;
-        at = grid_index(W, 2 * W * H, a, b, l);
-        const unsigned w = __ldg(sc.top + (2 * cell0 + at));
-        const int nx = (int)(__float_as_uint(dx) >> 31), ny = (int)(__float_as_uint(dy) >> 31);
+        at = grid_index(W, n2, a, b, l);
+        const unsigned w = __ldg(top + at);
         const int bx = (a + 1 - nx) << l, by = (b + 1 - ny) << l;
-        const float tx = ((float)bx - ox) * ix, ty = ((float)by - oy) * iy;
+        const float tx = ((float)bx - tr.x) * ix, ty = ((float)by - tr.y) * iy;
         s1 = fmaxf(s, fminf(fminf(tx, ty), smax));
-        const float thr = threshold(s, s1);
+        const float thr = threshold(hc, s, s1);
         if (w != 0u && height_magic(w) >= thr && !(fl & kFlagTested)) {
           if (l == 0) st = kLaneList;
           l = max(l - 2, 0);
@@ -938,17 +975,18 @@ __global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
           fl &= ~kFlagTested;
           s = s1;
           const bool xx = tx < ty;
-          const int top = (1 << l) - 1;
-          const int fi = min(max((int)floorf(__fmaf_rn(s, dx, ox)), a << l), (a << l) + top);
-          const int fj = min(max((int)floorf(__fmaf_rn(s, dy, oy)), b << l), (b << l) + top);
+          const int last = (1 << l) - 1;
+          const int fi = min(max((int)floorf(__fmaf_rn(s, tr.z, tr.x)), a << l), (a << l) + last);
+          const int fj = min(max((int)floorf(__fmaf_rn(s, tr.w, tr.y)), b << l), (b << l) + last);
           i = xx ? bx - nx : fi;
           j = xx ? fj : by - ny;
-          if (((xx ? bx : by) & (3 << l)) == 0 && l < ltop) l += 2;
-          if (s >= smax || (unsigned)i >= (unsigned)W || (unsigned)j >= (unsigned)H)
+          if (((xx ? bx : by) & (3 << l)) == 0 && l < size.z) l += 2;
+          if (s >= smax || (unsigned)i >= (unsigned)W || (unsigned)j >= (unsigned)size.y)
             st = kLaneAdvance;
         }
       }
       if (__popc(__ballot_sync(kFull, st == kLaneWalk)) < HZ_WALK_MIN) break;
+    }
     }
 
     // Triangle pass: the lists of all lanes that reached a cell, their
@@ -958,13 +996,15 @@ __global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
     int n = 0;
     unsigned k0 = 0;
     if (st == kLaneList) {
-      const uint32_t k = __ldg(sc.gstart + (cell0 + at));
-      n = (int)(__ldg(sc.gstart + (cell0 + at + 1)) - k);
+      const uint32_t* gs = sc.gstart + (sh.size[t].w + at);
+      const uint32_t k = __ldg(gs);
+      n = (int)(__ldg(gs + 1) - k);
       const float4 g = sh.grid[t];
-      const float xexit = s1 * xhi * g.x;
+      const float4 hc = sh.v[t][kRowHeight];
+      const float xexit = s1 * hc.z * g.x;
       k0 = __float_as_uint(g.w) + k;
       sh.v[t][kRowOrigin].w = kEps * __fmaf_rn(1.1f, xexit, g.z);
-      sh.v[t][kRowSide].w = threshold(s, s1);
+      sh.v[t][kRowSide].w = threshold(hc, s, s1);
       sh.v[t][kRowAlong].w = xexit + g.y;
       sh.m_new[t] = m;
       sh.flags[t] = 0;
@@ -1032,8 +1072,8 @@ __global__ void __launch_bounds__(kSweepBlock, HZ_SWEEP_MIN_BLOCKS)
       const int f = sh.flags[t], mn = sh.m_new[t];
       if (mn > m) {
         fl |= kFlagAny;
-        if (mn >= mstop) {
-          m = mstop;  // known to miss from the sweep above
+        if (mn >= sh.mstop[t]) {
+          m = sh.mstop[t];  // known to miss from the sweep above
           st = kLaneAdvance;
         } else if (mn > kMaxM) {
           fl |= kFlagGap;
@@ -1084,8 +1124,8 @@ __device__ bool grid_ray(const DomainDesc& D, const GridDesc& g, const Ray& r, c
     const int at = grid_index(W, n2, a, b, l);
     const unsigned hi = __ldg(D.top + at), lo = __ldg(D.low + at);
     const bool sx = tr.dx > 0.f, sy = tr.dy > 0.f;
-    const float tx = ((float)((sx ? a + 1 : a) << l) - tr.ox) * tr.ix;
-    const float ty = ((float)((sy ? b + 1 : b) << l) - tr.oy) * tr.iy;
+    const float tx = __fdividef((float)((sx ? a + 1 : a) << l) - tr.ox, tr.dx);
+    const float ty = __fdividef((float)((sy ? b + 1 : b) << l) - tr.oy, tr.dy);
     const float s1 = fmaxf(s, fminf(fminf(tx, ty), tr.smax));
     // Lowest and highest height of the ray over [s, s1].
     const float T0 = __fmaf_rn(s, kl, slope), T1 = __fmaf_rn(s1, kh, slope);
@@ -1225,7 +1265,7 @@ __global__ void __launch_bounds__(128)
     const float fz = __fdiv_rn(kRf, (float)(dz + kEarthRadius));
     const double r2 = (double)ox * ox + (double)oy * oy + dz * (dz + 2.0 * kEarthRadius);
     const float ho = __fdiv_rn((float)r2, sqrtf((float)(kEarthRadius * kEarthRadius + r2)) + kRf);
-    const float ux = (float)f.normal.x, uy = (float)f.normal.y;
+    const float ux = (float)f.normal.x, uy = (float)f.normal.y, uz = (float)f.normal.z;
     int m = 0, run = 0, before = 0;
     double elev = 0.0;
     for (int a = 0; a < D.L; a++) {
@@ -1255,7 +1295,7 @@ __global__ void __launch_bounds__(128)
         const Ray r = lattice_ray<kPrecise>(D, f, a, mm, ecs);
         // Beyond the zenith the ray runs along the opposite azimuth.
         const float sg = ecs.x < 0.0 ? -1.f : 1.f;
-        const Track tr = make_track(g, ox * fz, oy * fz, sg * hx, sg * hy, sg * hz, ux, uy);
+        const Track tr = make_track(g, ox * fz, oy * fz, sg * hx, sg * hy, sg * hz, ux, uy, uz);
         const float c = fmaxf(fabsf((float)ecs.x), 1e-7f);
         return grid_ray<kPrecise>(D, g, r, tr, ho, __fdiv_rn((float)ecs.y, c));
       };

@@ -49,6 +49,11 @@ def _same(inputs, args, **kw):
     # a range of cells
     (dict(edge_km=1.0, box_km=40.0, seed=9), (24, 1, 20000.0, 0.2, 5, 1),
      {"cells": (1001, 1778)}),
+    # a triangle cut by many rays at the search radius, beyond it at the higher
+    (dict(edge_km=0.24629858041449693, box_km=17.611548057004665, kind="eroded",
+          hmin=268.98230903271724, hmax=9000, hurst=0.9368420793831944, n_features=6, seed=319,
+          lat0_deg=18.69738742425085, lon0_deg=-85.1331917032566, face_rotation_deg=0.0),
+     (24, 1, 5000.0, 0.2, 1, 2), {}),
 ])
 def test_gpu_sweep_is_the_tree_search(dkw, args, kw):
     d = synthetic.make_domain(**dkw)
