@@ -290,6 +290,7 @@ BatchBuffers carve_batch(Carver& c, int n, long long total_cells, const SweepSiz
     b.all.start = c.take<uint32_t>(sweep->cells);
     b.all.top = c.take<uint16_t>(2 * sweep->cells);
     b.all.low = c.take<uint16_t>(2 * sweep->cells);
+    b.all.planes = c.take<uint2>(2 * sweep->cells);
   }
   b.counters = c.take<unsigned long long>(kCounterWords);
   b.done = c.take<unsigned long long>(2 * (size_t)n);
@@ -829,7 +830,7 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
       D.svf_part = b[d].svf_part;
       D.raw_j = n == 1 ? opt.raw_index : nullptr;
       D.grid = b[d].sweep.grid;
-      D.top = b[d].sweep.top;
+      D.planes = b[d].sweep.planes;
       D.low = b[d].sweep.low;
       D.gstart = b[d].sweep.start;
       D.refs = b[d].sweep.refs;
@@ -1210,6 +1211,7 @@ int run_entry(hz_domain* doms, int n, bool on_device, cudaStream_t user_stream,
         b[d].sweep.start = bb.all.start + o.cells;
         b[d].sweep.top = bb.all.top + 2 * o.cells;
         b[d].sweep.low = bb.all.low + 2 * o.cells;
+        b[d].sweep.planes = bb.all.planes + 2 * o.cells;
       }
     }
 

@@ -198,7 +198,7 @@ struct DomainDesc {
   // cell frames [kFrameRows][ncell] by work position; result codes [L][ncell];
   // items per cell (runs of consecutive azimuths).
   const GridDesc* grid;
-  const uint16_t* top;
+  const uint2* planes;
   const uint16_t* low;
   const uint32_t* gstart;
   const uint2* refs;
@@ -267,6 +267,7 @@ struct SweepBuffers {
   uint32_t* total;
   uint16_t* top;         // 2 x cells cap: pyramid of upper heights
   uint16_t* low;         // and of lower ones
+  uint2* planes;         // and of the upper bounds as planes
   uint2* refs;           // refs cap
 };
 // Grid, lists and height pyramid of a domain, and its triangle records (mesh
@@ -282,6 +283,7 @@ struct SweepAll {
   uint32_t* start;
   uint16_t* top;
   uint16_t* low;
+  uint2* planes;
 };
 // Frames, sweep, repair and outputs of all domains (after cell_order and
 // trace_tables). s_full: the lowest lattice elevation a search can ask for.
