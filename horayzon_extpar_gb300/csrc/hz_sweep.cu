@@ -88,6 +88,13 @@ constexpr float kEps = 1.28e-6f;
 constexpr float kMagic = 8388608.0f;      // 2^23: float(2^23 | n) = 2^23 + n
 constexpr int kTanRange = 180;            // lattice elevations with a tangent: |m| < 180
 constexpr int kMaxM = 177;                // sweeps stop below 89 deg
+// A sweep that nothing met starts over kLower steps lower, then twice that, then
+// from the floor; a run's first azimuth, whose start is well below any horizon
+// of its neighbourhood, from the floor at once: it looks over the mesh's edge.
+// Against the floor after one lower start (there every elevation up to the
+// horizon is a raise): 1.2M cells at 100 m 49.4 -> 45.0 ms, 500 cells 0.98 -> 0.70;
+// with the two lower starts for first azimuths too 0.76. Third lower starts: no gain.
+constexpr int kLower = 4, kLowerTries = 2;
 constexpr int kRunStart = -14;            // start of a run's first azimuth (-7 deg)
 
 // Codes of a (cell, azimuth): the lowest missing lattice elevation, or
@@ -615,7 +622,7 @@ __device__ __forceinline__ Track make_track(const GridDesc& g, float X0, float Y
 enum : int { kLaneAdvance = 0, kLaneWalk = 1, kLaneList = 2 };
 // Lane flags; kFlagAbove and kFlagRedo also come back from the triangle pass.
 enum : int { kFlagAny = 1, kFlagAbove = 2, kFlagRedo = 4, kFlagGap = 8, kFlagTested = 16,
-             kFlagRetry = 32 };
+             kFlagRetry = 32 };  // and up: lower starts so far
 
 // What the triangle pass needs of a thread's azimuth and cell, in shared
 // memory: any lane of the warp tests triangles for any other. Quadruples, read
@@ -933,8 +940,9 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
           // Nothing met the start's ray or any above it: start lower.
           again = true;
           sh.mstop[t] = m;
-          m = (fl & kFlagRetry) ? s_full : max(s_full, m - 4);
-          fl = kFlagRetry;
+          const int tries = fl / kFlagRetry;
+          m = tries < kLowerTries ? max(s_full, m - (kLower << tries)) : s_full;
+          fl = (tries + 1) * kFlagRetry;
         } else {
           code = kCodeAllMiss;
         }
@@ -1018,7 +1026,7 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
           const int a = sh.az[t];
           const int prev = sh.prev[t];
           sh.mstop[t] = 1 << 20;
-          fl = 0;
+          fl = prev == kFirst ? kLowerTries * kFlagRetry : 0;
           // Two steps below the previous azimuth's result; a run's first azimuth
           // well below any horizon of its neighbourhood (k_sweep_runs checks
           // that the search came from no lower); else from the floor.
