@@ -528,18 +528,23 @@ __device__ __forceinline__ Ray lattice_ray(const DomainDesc& D, const CellFrame&
 // The FP64 frame comes from its table: recomputing it (two square roots and
 // six divisions) took more of the FP64 pipe than the whole rest of the sweep.
 template <bool kPrecise>
-__device__ __noinline__ bool exact_hit(const DomainDesc* D, int p, int a, int m, int tri) {
-  const long long nc = D->ncell;
-  const double* fr = D->cell_frame + p;
-  const float* o = D->cell_f32 + p;
-  const double2 cs = __ldg(&D->azim_cs[a]);
-  const double2 ecs = __ldg(&D->elev_cs[m - kElevMin]);
+__device__ __forceinline__ Ray table_ray(const DomainDesc& D, int p, int a, int m, double2& ecs) {
+  const long long nc = D.ncell;
+  const double* fr = D.cell_frame + p;
+  const float* o = D.cell_f32 + p;
+  const double2 cs = __ldg(&D.azim_cs[a]);
+  ecs = __ldg(&D.elev_cs[m - kElevMin]);
   const float dx = (float)(ecs.x * (cs.x * fr[3 * nc] + cs.y * fr[6 * nc]) + ecs.y * fr[0]);
   const float dy = (float)(ecs.x * (cs.x * fr[4 * nc] + cs.y * fr[7 * nc]) + ecs.y * fr[nc]);
   const float dz = (float)(ecs.x * (cs.x * fr[5 * nc] + cs.y * fr[8 * nc]) + ecs.y * fr[2 * nc]);
-  const Ray r = kPrecise ? make_ray(o[0], o[nc], o[2 * nc], dx, dy, dz, D->tfar, o[15 * nc],
-                                    o[16 * nc], o[17 * nc])
-                         : make_ray(o[0], o[nc], o[2 * nc], dx, dy, dz, D->tfar);
+  return kPrecise ? make_ray(o[0], o[nc], o[2 * nc], dx, dy, dz, D.tfar, o[15 * nc], o[16 * nc],
+                             o[17 * nc])
+                  : make_ray(o[0], o[nc], o[2 * nc], dx, dy, dz, D.tfar);
+}
+template <bool kPrecise>
+__device__ __noinline__ bool exact_hit(const DomainDesc* D, int p, int a, int m, int tri) {
+  double2 ecs;
+  const Ray r = table_ray<kPrecise>(*D, p, a, m, ecs);
   return test_tri<kPrecise>(D->tris, D->tri_lo, r, tri);
 }
 
@@ -1331,41 +1336,73 @@ __global__ void k_sweep_runs(const DomainDesc* __restrict__ doms, int ndom, int 
   }
 }
 
+// n additions of c (+-two_ha) to elev, each rounded, as the reference carries
+// its elevation. While the sum stays in one binade an addition moves it by the
+// same number of its last places, c rounded to them (unless c lies half way
+// between two): one integer addition for all steps, where each FP64 addition
+// holds the SM's pipe for 16 cycles. The step that leaves a binade is an FP64
+// addition; so is one that would reach its lower end, below which the places
+// are finer.
+__device__ __forceinline__ void add_steps(double& elev, double c, int n) {
+  const long long cb = __double_as_longlong(c);
+  const unsigned long long mant = (1ull << 52) - 1;
+  const unsigned long long mc = ((unsigned long long)cb & mant) | (mant + 1);
+  const int ec = (int)((unsigned long long)cb >> 52) & 0x7ff;
+#pragma unroll 1
+  while (n > 0) {
+    const unsigned long long x = (unsigned long long)__double_as_longlong(elev);
+    const int sh = ((int)(x >> 52) & 0x7ff) - ec;
+    if (sh > 0 && sh < 20) {
+      const unsigned long long half = 1ull << (sh - 1), rest = mc & (2 * half - 1);
+      const unsigned long long k = (mc >> sh) + (rest > half ? 1ull : 0ull);
+      const bool grows = (long long)x >= 0 == (cb >= 0);
+      // Steps to the binade's end, rounded down.
+      const unsigned long long room = grows ? mant - (x & mant) : x & mant;
+      const int t = min(n, (int)(__fdividef((float)(unsigned)(room >> 20),
+                                            (float)(unsigned)(k >> 20)) * 0.9999f));
+      const unsigned long long y = grows ? x + (unsigned)t * k : x - (unsigned)t * k;
+      if (rest != half && (y >> 52) == (x >> 52) && (grows || (y & mant) != 0ull)) {
+        elev = __longlong_as_double((long long)y);
+        n -= t;
+      }
+    }
+    if (n > 0) {
+      elev += c;
+      n--;
+    }
+  }
+}
+
+// Lattice elevations from here up are more than the rounding of any carried
+// elevation above the floor of the downward search.
+__device__ __forceinline__ int above_floor(const DomainDesc& D) {
+  return (int)floorf((float)D.elev_floor / (float)D.two_ha) + 2;
+}
+
 // The reference's search of one azimuth from (m, elev), given a lattice hit
 // pattern that ends at the lowest miss M (kCodeAllMiss: no hits) or, for a
 // code of k_sweep_repair, its stop. Returns true when it went up; n counts
 // the steps (one ray each after the first).
-__device__ __forceinline__ bool replay(int code, const DomainDesc& D, int& m, double& elev,
-                                       int& n) {
-  n = 0;
+__device__ __forceinline__ bool replay(int code, const DomainDesc& D, int safe, int& m,
+                                       double& elev, int& n) {
+  const int from = m;
+  bool up = m < code;
+  int stop = up ? code : min(m, max(code, safe) - 1);
   if (code >= kCodeStop) {
-    const int v = code - kCodeStop, stop = (v >> 1) - 2000;
-    if (v & 1) {
-      for (; m < stop; n++) {
-        m++;
-        elev += D.two_ha;
-      }
-      return true;
-    }
-    for (; m > stop; n++) {
+    stop = ((code - kCodeStop) >> 1) - 2000;
+    up = (code - kCodeStop) & 1;
+    if (up ? stop < m : stop > m) stop = m;
+  }
+  add_steps(elev, up ? D.two_ha : -D.two_ha, abs(stop - m));
+  m = stop;
+  if (code < kCodeStop && !up) {
+    while (m >= code && elev > D.elev_floor) {
       m--;
       elev -= D.two_ha;
     }
-    return false;
   }
-  if (m < code) {
-    for (; m < code; n++) {
-      m++;
-      elev += D.two_ha;
-    }
-    return true;
-  }
-  while (m >= code && elev > D.elev_floor) {
-    m--;
-    elev -= D.two_ha;
-    n++;
-  }
-  return false;
+  n = abs(m - from);
+  return up;
 }
 
 // First elevation of azimuth a: carried, or given (DomainDesc::start_m; 0 for
@@ -1402,19 +1439,20 @@ __global__ void __launch_bounds__(128)
     const DomainDesc& D = doms[domain_of(doms, ndom, gid)];
     const GridDesc& g = *D.grid;
     const int cell = (int)(gid - D.cell_offset);
-    const CellFrame f = cell_frame64(D, cell);
-    const float ox = (float)f.ox, oy = (float)f.oy;
-    const double dz = (float)f.oz;
-    const float fz = __fdiv_rn(kRf, (float)(dz + kEarthRadius));
-    const double r2 = (double)ox * ox + (double)oy * oy + dz * (dz + 2.0 * kEarthRadius);
-    const float ho = __fdiv_rn((float)r2, sqrtf((float)(kEarthRadius * kEarthRadius + r2)) + kRf);
-    const float ux = (float)f.normal.x, uy = (float)f.normal.y, uz = (float)f.normal.z;
+    const int p = list[w] - (int)D.k_begin;
+    const long long nc = D.ncell;
+    const float* fr = D.cell_f32 + p;
+    const float ux = fr[3 * nc], uy = fr[4 * nc], uz = fr[5 * nc], X0 = fr[12 * nc],
+                Y0 = fr[13 * nc], ho = fr[14 * nc];
+    const int safe = above_floor(D);
+    int codes = 0;
     int m = 0, run = 0, before = 0;
     double elev = 0.0;
     for (int a = 0; a < D.L; a++) {
       chain_start(D, cell, a, m, elev);
       int16_t* slot = D.codes + (long long)a * D.ncell + cell;
-      const int code = *slot;
+      if ((a & 31) == 0 && a + lane < D.L) codes = slot[(long long)lane * nc];
+      const int code = __shfl_sync(kFull, codes, a & 31);
       int steps;
       // Where this azimuth's sweep began: the hits below that are not known.
       int from = s_full;
@@ -1426,19 +1464,20 @@ __global__ void __launch_bounds__(128)
       }
       before = code;
       if (code != kCodeGap && (m >= from || code == kCodeAllMiss)) {
-        replay(code, D, m, elev, steps);
+        replay(code, D, safe, m, elev, steps);
         continue;
       }
       const double2 cs = __ldg(&D.azim_cs[a]);
-      const float hx = (float)(cs.x * f.north.x + cs.y * f.east.x);
-      const float hy = (float)(cs.x * f.north.y + cs.y * f.east.y);
-      const float hz = (float)(cs.x * f.north.z + cs.y * f.east.z);
+      const float c = (float)cs.x, e = (float)cs.y;
+      const float hx = __fmaf_rn(c, fr[6 * nc], e * fr[9 * nc]);
+      const float hy = __fmaf_rn(c, fr[7 * nc], e * fr[10 * nc]);
+      const float hz = __fmaf_rn(c, fr[8 * nc], e * fr[11 * nc]);
       auto ray_hits = [&](int mm) {
         double2 ecs;
-        const Ray r = lattice_ray<kPrecise>(D, f, a, mm, ecs);
+        const Ray r = table_ray<kPrecise>(D, p, a, mm, ecs);
         // Beyond the zenith the ray runs along the opposite azimuth.
         const float sg = ecs.x < 0.0 ? -1.f : 1.f;
-        const Track tr = make_track(g, ox * fz, oy * fz, sg * hx, sg * hy, sg * hz, ux, uy, uz);
+        const Track tr = make_track(g, X0, Y0, sg * hx, sg * hy, sg * hz, ux, uy, uz);
         const float c = fmaxf(fabsf((float)ecs.x), 1e-7f);
         return grid_ray<kPrecise>(D, g, r, tr, ho, __fdiv_rn((float)ecs.y, c));
       };
@@ -1451,10 +1490,9 @@ __global__ void __launch_bounds__(128)
           const unsigned miss = ~hits & (have == 32 ? kFull : 0xFFFFu);
           const int reach = miss ? __ffs(miss) - 1 : have;  // first miss at base + reach
           const int to = min(base + reach, m + left);       // up to there
-          for (; m < to; left--) {
-            m++;
-            elev += D.two_ha;
-          }
+          add_steps(elev, D.two_ha, to - m);
+          left -= to - m;
+          m = to;
           if (miss || left == 0) break;
           base += have;
           have = 32;
@@ -1464,8 +1502,12 @@ __global__ void __launch_bounds__(128)
         int base = m - 1, have = 16;
         unsigned below = hits >> 16;
         for (;;) {
-          bool hit = false;
-          int q = 0;
+          // Down to the first hit, the last of the rays at hand, or near the floor.
+          const int hit_at = below ? __ffs(below) - 1 : 64;
+          int q = max(0, min(min(have, hit_at + 1), m - safe + 1));
+          add_steps(elev, -D.two_ha, q);
+          m -= q;
+          bool hit = q == hit_at + 1;
           for (; q < have && elev > D.elev_floor && !hit; q++) {
             m--;
             elev -= D.two_ha;
@@ -1488,29 +1530,35 @@ __global__ void __launch_bounds__(128)
 
 // The reference's search of every traced cell on its hit patterns: carried
 // elevations, clip, sector means, SVF sums, ray count (cpp:490-555, 736-754).
+// Bound by the FP64 pipe (60 % busy) and by what the lanes of a warp do not
+// share of the walk up and down: with an FP64 addition per elevation step 1.2M cells
+// took 2.05 ms and 500 cells 0.157 (border cells step down to the floor), with
+// add_steps 0.76 and 0.051. Codes come four azimuths at a time, packed, and the
+// loop over them is not unrolled: eight times over it ran out of the
+// instruction cache.
 template <bool kRefine1>
 __device__ __forceinline__ unsigned finish_sweep(const DomainDesc& D, int cell) {
   const long long nc = D.ncell;
   const float inv_ha = (float)(1.0 / D.hori_acc);
   const double ha = D.hori_acc, refine = (double)D.refine;
-  const int span = D.L / D.groups;
+  const int span = D.L / D.groups, safe = above_floor(D);
   int m = 0;
   double elev = 0.0, sector = 0.0, svf = 0.0, part = 0.0;
   unsigned rays = 0;
-  constexpr int kAhead = 8;
   int in_sector = 0, row = 0, in_group = 0;
-  for (int a0 = 0; a0 < D.L; a0 += kAhead) {
-    int code[kAhead];
+#pragma unroll 1
+  for (int a0 = 0; a0 < D.L; a0 += 4) {
+    unsigned long long codes = 0;
 #pragma unroll
-    for (int u = 0; u < kAhead; u++)
-      code[u] = a0 + u < D.L ? D.codes[(long long)(a0 + u) * nc + cell] : 0;
-#pragma unroll
-    for (int u = 0; u < kAhead; u++) {
-      const int a = a0 + u;
-      if (a >= D.L) break;
+    for (int u = 0; u < 4; u++)
+      if (a0 + u < D.L)
+        codes |= (unsigned long long)(uint16_t)D.codes[(long long)(a0 + u) * nc + cell] << (16 * u);
+    const int end = min(a0 + 4, D.L);
+#pragma unroll 1
+    for (int a = a0; a < end; a++, codes >>= 16) {
       chain_start(D, cell, a, m, elev);
       int steps;
-      const bool up = replay(code[u], D, m, elev, steps);
+      const bool up = replay((int16_t)codes, D, safe, m, elev, steps);
       rays += 1u + (unsigned)steps;
       double h = up ? elev - ha : elev + ha;
       const int j = up ? 2 * m - 1 : 2 * m + 1;
