@@ -210,7 +210,7 @@ Buffers carve_domain(Carver& c, long long ncell, long long nvert, long long nhor
     b.sweep.count = c.take<uint32_t>(cells + 1);
     b.sweep.partials = c.take<uint32_t>(scan_partials(cells + 1));
     b.sweep.total = c.take<uint32_t>(4);
-    b.cell_f32 = c.take<float>(sweep_frame_floats() * ncell);
+    b.cell_f32 = c.take<float>(sweep_frame_floats(precise) * ncell);
     b.codes = c.take<int16_t>(L * ncell);
     b.tan_m = c.take<float>(kTanTable);
     if (learned) {
@@ -845,6 +845,8 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
         D.tri_lo = bb.all.tri_lo;
       }
       D.runs = (int)std::max(1ll, std::min<long long>(L, runs_wanted));
+      D.run_len = L / D.runs;
+      D.run_extra = L % D.runs;
       D.centre = frames[d].centre;
       D.pole = frames[d].pole;
       D.ray_org_elev = P.ray_org_elev;

@@ -195,8 +195,8 @@ struct DomainDesc {
   // (k_trace_warp's occluder cache; same results, fewer traversals).
   int occ_cache;
   // Profile sweep (hz_sweep.cu): grid, pyramid, list starts and lists; FP32
-  // cell frames [kFrameRows][ncell] by work position; result codes [L][ncell];
-  // items per cell (runs of consecutive azimuths).
+  // cell frames by work position; result codes [L][ncell]; items per cell (runs of
+  // consecutive azimuths: run_len each, the first run_extra one more).
   const GridDesc* grid;
   const uint2* planes;
   const uint16_t* low;
@@ -207,7 +207,7 @@ struct DomainDesc {
   int cell_base;              // of its cells in gstart (half of it: its pyramid) and of its
   unsigned ref_base;          // list entries, in the call's arrays (SweepAll)
   const float* tan_m;         // [kTanTable] tangents of (k - kTanTable / 2) * 0.5 deg
-  int runs;
+  int runs, run_len, run_extra;
   int16_t* raw_j;             // optional output: unclipped horizon j (h = j * 0.25 deg)
   double3 centre, pole;       // Earth centre / North Pole in ENU
   double ray_org_elev, hori_acc, elev_floor;
@@ -256,7 +256,7 @@ cudaError_t trace_flat(const DomainDesc* doms, int ndom, const int32_t* order, i
 // Capacities of a domain's grid cells and list entries, rows of the frame table.
 long long sweep_cells_cap(long long n_tri);
 long long sweep_refs_cap(long long n_tri);
-size_t sweep_frame_floats();
+size_t sweep_frame_floats(bool precise);
 struct SweepBuffers {
   float4* gv;            // n_vert: gnomonic X, Y, height
   unsigned* bounds;      // 8

@@ -58,8 +58,8 @@ namespace {
 
 constexpr int kSweepBlock = 128;
 // Resident blocks per SM: 6 of 80 registers (1.2M cells at 100 m: 70.6 ms with 5, 67.4
-// with 6, spills from 7 on: 31 ms against 26 of a 300 km domain); 5 of 96 where
-// the watertight test recomputes rays in FP64 (10.0 ms, 11.6 with 6).
+// with 6, spills from 7 on: 31 ms against 26 of a 300 km domain); 5 of 96 for the
+// FP64 ray mode (10.0 ms, 11.6 with 6).
 #ifndef HZ_SWEEP_MIN_BLOCKS
 #define HZ_SWEEP_MIN_BLOCKS 6
 #endif
@@ -523,23 +523,33 @@ __device__ __forceinline__ Ray lattice_ray(const DomainDesc& D, const CellFrame&
   return make_ray(ox, oy, oz, dx, dy, dz, D.tfar);
 }
 
+// FP32 frame table by work position, quadruples of one cell together: origin
+// and its height, normal, north and the origin's gnomonic X, east and Y, and
+// (precise) the origin's FP32 residual. Lanes set up azimuths of scattered
+// cells: four accesses, where one row after another over all cells took 14 (FP64 ray
+// mode, 194k cells: 7.15 -> 6.93 ms).
+enum : int { kFrameOrigin, kFrameNormal, kFrameNorth, kFrameEast, kFrameRest };
+template <bool kPrecise>
+__device__ __forceinline__ float4* cell_rows(const DomainDesc& D, long long p) {
+  return reinterpret_cast<float4*>(D.cell_f32) + p * (kPrecise ? 5 : 4);
+}
+
 // The watertight test of one lattice ray and one triangle, for the few
 // triangles the sweep's own arithmetic leaves undecided (p: work position).
 // The FP64 frame comes from its table: recomputing it (two square roots and
 // six divisions) took more of the FP64 pipe than the whole rest of the sweep.
 template <bool kPrecise>
 __device__ __forceinline__ Ray table_ray(const DomainDesc& D, int p, int a, int m, double2& ecs) {
-  const long long nc = D.ncell;
-  const double* fr = D.cell_frame + p;
-  const float* o = D.cell_f32 + p;
+  const double* fr = D.cell_frame + 9ll * p;
+  const float4* f32 = cell_rows<kPrecise>(D, p);
+  const float4 o = __ldg(f32), q = kPrecise ? __ldg(f32 + kFrameRest) : o;
   const double2 cs = __ldg(&D.azim_cs[a]);
   ecs = __ldg(&D.elev_cs[m - kElevMin]);
-  const float dx = (float)(ecs.x * (cs.x * fr[3 * nc] + cs.y * fr[6 * nc]) + ecs.y * fr[0]);
-  const float dy = (float)(ecs.x * (cs.x * fr[4 * nc] + cs.y * fr[7 * nc]) + ecs.y * fr[nc]);
-  const float dz = (float)(ecs.x * (cs.x * fr[5 * nc] + cs.y * fr[8 * nc]) + ecs.y * fr[2 * nc]);
-  return kPrecise ? make_ray(o[0], o[nc], o[2 * nc], dx, dy, dz, D.tfar, o[15 * nc], o[16 * nc],
-                             o[17 * nc])
-                  : make_ray(o[0], o[nc], o[2 * nc], dx, dy, dz, D.tfar);
+  const float dx = (float)(ecs.x * (cs.x * fr[3] + cs.y * fr[6]) + ecs.y * fr[0]);
+  const float dy = (float)(ecs.x * (cs.x * fr[4] + cs.y * fr[7]) + ecs.y * fr[1]);
+  const float dz = (float)(ecs.x * (cs.x * fr[5] + cs.y * fr[8]) + ecs.y * fr[2]);
+  return kPrecise ? make_ray(o.x, o.y, o.z, dx, dy, dz, D.tfar, q.x, q.y, q.z)
+                  : make_ray(o.x, o.y, o.z, dx, dy, dz, D.tfar);
 }
 template <bool kPrecise>
 __device__ __noinline__ bool exact_hit(const DomainDesc* D, int p, int a, int m, int tri) {
@@ -547,10 +557,6 @@ __device__ __noinline__ bool exact_hit(const DomainDesc* D, int p, int a, int m,
   const Ray r = table_ray<kPrecise>(*D, p, a, m, ecs);
   return test_tri<kPrecise>(D->tris, D->tri_lo, r, tri);
 }
-
-// FP32 frame table by work position: origin, normal, north, east, gnomonic
-// X, Y and height of the origin, and (precise) the origin's FP32 residual.
-constexpr int kFrameRows = 18;
 
 template <bool kPrecise>
 __global__ void k_sweep_frames(const DomainDesc* __restrict__ doms, int ndom,
@@ -560,29 +566,27 @@ __global__ void k_sweep_frames(const DomainDesc* __restrict__ doms, int ndom,
   const long long gid = order[k];
   const DomainDesc& D = doms[domain_of(doms, ndom, gid)];
   const int cell = (int)(gid - D.cell_offset);
-  const long long p = k - D.k_begin, nc = D.ncell;
+  const long long p = k - D.k_begin;
   const CellFrame f = cell_frame64(D, cell);
-  double* fr = D.cell_frame + p;
-  fr[0] = f.normal.x; fr[nc] = f.normal.y; fr[2 * nc] = f.normal.z;
-  fr[3 * nc] = f.north.x; fr[4 * nc] = f.north.y; fr[5 * nc] = f.north.z;
-  fr[6 * nc] = f.east.x; fr[7 * nc] = f.east.y; fr[8 * nc] = f.east.z;
-  float* o = D.cell_f32 + p;
+  double* fr = D.cell_frame + 9 * p;
+  fr[0] = f.normal.x; fr[1] = f.normal.y; fr[2] = f.normal.z;
+  fr[3] = f.north.x; fr[4] = f.north.y; fr[5] = f.north.z;
+  fr[6] = f.east.x; fr[7] = f.east.y; fr[8] = f.east.z;
   const float ox = (float)f.ox, oy = (float)f.oy, oz = (float)f.oz;
-  o[0] = ox; o[nc] = oy; o[2 * nc] = oz;
-  o[3 * nc] = (float)f.normal.x; o[4 * nc] = (float)f.normal.y; o[5 * nc] = (float)f.normal.z;
-  o[6 * nc] = (float)f.north.x; o[7 * nc] = (float)f.north.y; o[8 * nc] = (float)f.north.z;
-  o[9 * nc] = (float)f.east.x; o[10 * nc] = (float)f.east.y; o[11 * nc] = (float)f.east.z;
   const double dz = oz;
   const float fz = __fdiv_rn(kRf, (float)(dz + kEarthRadius));
-  o[12 * nc] = ox * fz;
-  o[13 * nc] = oy * fz;
   const double r2 = (double)ox * ox + (double)oy * oy + dz * (dz + 2.0 * kEarthRadius);
-  o[14 * nc] = __fdiv_rn((float)r2, sqrtf((float)(kEarthRadius * kEarthRadius + r2)) + kRf);
-  if (kPrecise) {
-    o[15 * nc] = (float)(f.ox - (double)ox);
-    o[16 * nc] = (float)(f.oy - (double)oy);
-    o[17 * nc] = (float)(f.oz - (double)oz);
-  }
+  const float height =
+      __fdiv_rn((float)r2, sqrtf((float)(kEarthRadius * kEarthRadius + r2)) + kRf);
+  float4* o = cell_rows<kPrecise>(D, p);
+  o[kFrameOrigin] = make_float4(ox, oy, oz, height);
+  o[kFrameNormal] =
+      make_float4((float)f.normal.x, (float)f.normal.y, (float)f.normal.z, 0.f);
+  o[kFrameNorth] = make_float4((float)f.north.x, (float)f.north.y, (float)f.north.z, ox * fz);
+  o[kFrameEast] = make_float4((float)f.east.x, (float)f.east.y, (float)f.east.z, oy * fz);
+  if (kPrecise)
+    o[kFrameRest] = make_float4((float)(f.ox - (double)ox), (float)(f.oy - (double)oy),
+                                (float)(f.oz - (double)oz), 0.f);
 }
 
 // Track of one (cell, azimuth) on the grid, in metres s along the gnomonic
@@ -619,6 +623,12 @@ __device__ __forceinline__ Track make_track(const GridDesc& g, float X0, float Y
   if (fabsf(t.dx) < 1e-12f) t.dx = t.dx < 0.f ? -1e-12f : 1e-12f;
   if (fabsf(t.dy) < 1e-12f) t.dy = t.dy < 0.f ? -1e-12f : 1e-12f;
   return t;
+}
+
+// First azimuth of a run of azimuths (of run D.runs: L); the first run_extra
+// runs hold one more than run_len.
+__device__ __forceinline__ int run_start(const DomainDesc& D, int run) {
+  return run * D.run_len + min(run, D.run_extra);
 }
 
 // ---------------------------------------------------------------------------
@@ -667,7 +677,6 @@ struct SweepShared {
   // elevation; elevation and flags from the triangle pass.
   int dom[kSweepBlock], cell[kSweepBlock], pos[kSweepBlock], az[kSweepBlock], az_end[kSweepBlock],
       prev[kSweepBlock], m[kSweepBlock], m_new[kSweepBlock], flags[kSweepBlock];
-  float reach[kSweepBlock];            // the search radius times cos(e)
   int2 entry[kSweepBlock];             // per list in order: thread, first entry - its number
   int2 queue[kWarps][64];              // (thread, triangle) to be cut with the plane
   float tan_m[kTanTable];
@@ -750,7 +759,8 @@ __device__ __forceinline__ int cut_triangle(const SweepShared<kPrecise>& sh, int
   const float e0 = kEps * (fabsf(a.x) + fabsf(a.y) + fabsf(a.z)),
               e1 = kEps * (fabsf(b.x) + fabsf(b.y) + fabsf(b.z)),
               e2 = kEps * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z));
-  const float ta = ray.w, ts = 1.f + fabsf(ta), xexit = along.w, reach = sh.reach[o];
+  const float ta = ray.w, ts = 1.f + fabsf(ta), xexit = along.w, tfar = sh.v[o][kRowUp].w,
+              reach = tfar * rsqrtf(__fmaf_rn(ta, ta, 1.f));  // the search radius along x
   const float* tm = sh.tan_m + kTanRange;
   const int m = sh.m[o];
   // Vertices in the plane within rounding: one of them is an end point of the
@@ -802,7 +812,7 @@ __device__ __forceinline__ int cut_triangle(const SweepShared<kPrecise>& sh, int
     // reach along x is that of the ray for rising ones, whose higher
     // neighbours reach less far, and the radius itself for falling ones.)
     if ((ah < -ea && bh < -eb) || fmaxf(ax, bx) < -xem || xmin > xexit ||
-        xmin > 1.00001f * (ta > 0.f ? reach : sh.v[o][kRowUp].w))
+        xmin > 1.00001f * (ta > 0.f ? reach : tfar))
       return 0;
     decided = ah > ea && bh > eb;
     if ((ah > ea && bh < -eb) || (ah < -ea && bh > eb)) {
@@ -823,7 +833,7 @@ __device__ __forceinline__ int cut_triangle(const SweepShared<kPrecise>& sh, int
         // Ray k is hidden where it passes the higher end below it by more than
         // the error te and within the radius (so do all between m and k then):
         // it meets the segment between ray m's crossing and that end.
-        const float far2 = 0.999f * sh.v[o][kRowUp].w * sh.v[o][kRowUp].w;
+        const float far2 = 0.999f * tfar * tfar;
         const float tx2 = fmaxf(tx, xc) * fmaxf(tx, xc);
         float v = 0.f, te = 0.f;
         const auto hides = [&](int k) {
@@ -878,7 +888,7 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
     k_sweep(const DomainDesc* __restrict__ doms, int ndom, const int* __restrict__ order,
             int total, int* __restrict__ work, int s_full, int* __restrict__ list,
             int* __restrict__ list_n, unsigned* __restrict__ listed, const SweepScene sc,
-            int* __restrict__ err) {
+            int lanes, int* __restrict__ err) {
   __shared__ SweepShared<kPrecise> sh;
   constexpr unsigned kFull = 0xffffffffu;
   constexpr int kUnknown = -30000, kFirst = -30001;
@@ -895,7 +905,9 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
   sh.dom[t] = 0;
   __syncthreads();
 
-  bool alive = true;
+  bool alive = lane < lanes;
+  const int walk_min = max(1, lanes * HZ_WALK_MIN >> 5),
+            adv_min = max(1, lanes * HZ_SWEEP_ADVANCE >> 5);
   int st = kLaneAdvance, fl = 0;
   int m = 0;
   int i = 0, j = 0, l = 0;
@@ -909,7 +921,6 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
     sh.v[t][kRowRay] = make_float4(__fmaf_rn(-ta, h.x, u.x), __fmaf_rn(-ta, h.y, u.y),
                                    __fmaf_rn(-ta, h.z, u.z), ta);
     sh.m[t] = m;
-    sh.reach[t] = u.w * rsqrtf(__fmaf_rn(ta, ta, 1.f));
   };
   // Height (as encoded in the lists) below which terrain between sa and sb
   // does not reach the ray: at distance x a ray of slope tan(e) is x (tan(e) +
@@ -929,7 +940,7 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
     const unsigned live = __ballot_sync(kFull, alive);
     if (live == 0u) break;
     const unsigned waiting = __ballot_sync(kFull, alive && st == kLaneAdvance);
-    if (waiting != 0u && (__popc(waiting) >= HZ_SWEEP_ADVANCE || waiting == live)) {
+    if (waiting != 0u && (__popc(waiting) >= adv_min || waiting == live)) {
       const bool mine = alive && st == kLaneAdvance;
       bool again = false;
       if (mine && sh.az[t] < sh.az_end[t]) {
@@ -982,7 +993,7 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
           if (take < nreq) {
             // Near the end of the queue a warp takes only what it needs.
             const int left = total - *(volatile int*)work;
-            const bool tail = left < (int)min(2147483647ll, (long long)gridDim.x * kWarps * 32);
+            const bool tail = left < (int)min(2147483647ll, (long long)gridDim.x * kWarps * lanes);
             const int grab = tail ? nreq - take : max(32, nreq - take);
             nb = atomicAdd(work, grab);
             sh.wq[0][wid] = nb + (nreq - take);
@@ -1001,25 +1012,24 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
             const int dom = domain_of_item(doms, ndom, item);
             const DomainDesc& D = doms[dom];
             const unsigned local = (unsigned)(item - D.item_begin);
+            // Quotient from FP32, off by one at most (fewer runs than 2^20).
             const unsigned run = local / (unsigned)D.ncell_traced;
             const int p = (int)(local - run * (unsigned)D.ncell_traced);
-            const long long nc = D.ncell;
-            const float* fr = D.cell_f32 + p;
-            sh.v[t][kRowOrigin] = make_float4(fr[0], fr[nc], fr[2 * nc], 0.f);
-            sh.v[t][kRowUp] = make_float4(fr[3 * nc], fr[4 * nc], fr[5 * nc], D.tfar);
-            if (kPrecise)
-              sh.v[t][kPrecise ? kRowRest : 0] =
-                  make_float4(fr[15 * nc], fr[16 * nc], fr[17 * nc], 0.f);
+            const float4* fr = cell_rows<kPrecise>(D, p);
+            const float4 fo = __ldg(fr + kFrameOrigin), fu = __ldg(fr + kFrameNormal);
+            sh.v[t][kRowOrigin] = make_float4(fo.x, fo.y, fo.z, 0.f);
+            sh.v[t][kRowUp] = make_float4(fu.x, fu.y, fu.z, D.tfar);
+            if (kPrecise) sh.v[t][kPrecise ? kRowRest : 0] = __ldg(fr + kFrameRest);
             const GridDesc& g = *D.grid;
-            sh.v[t][kRowHeight].w = (fr[14 * nc] - g.hpad - g.hlo) * g.iq;
+            sh.v[t][kRowHeight].w = (fo.w - g.hpad - g.hlo) * g.iq;
             sh.grid[t] = make_float4(g.unit, 2.f * g.pad, g.dadd + 2.f * __uint_as_float(g.lmax),
                                      __uint_as_float(D.ref_base));
             sh.size[t] = make_int4(g.W, g.H, g.L, D.cell_base);
             sh.dom[t] = dom;
             sh.cell[t] = (int)(order[D.k_begin + p] - D.cell_offset);
             sh.pos[t] = p;
-            sh.az[t] = (int)(run * (unsigned)D.L / (unsigned)D.runs);
-            sh.az_end[t] = (int)((run + 1) * (unsigned)D.L / (unsigned)D.runs);
+            sh.az[t] = run_start(D, (int)run);
+            sh.az_end[t] = run_start(D, (int)run + 1);
             sh.prev[t] = sh.az[t] == 0 ? 2 : kFirst;  // the search starts at 0 (cpp:511)
           }
         }
@@ -1043,17 +1053,17 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
           }
           const double2 cs64 = __ldg(&D.azim_cs[a]);
           const float c = (float)cs64.x, n = (float)cs64.y;
-          const long long nc = D.ncell;
-          const float* fr = D.cell_f32 + sh.pos[t];
-          const float hx = __fmaf_rn(c, fr[6 * nc], n * fr[9 * nc]);
-          const float hy = __fmaf_rn(c, fr[7 * nc], n * fr[10 * nc]);
-          const float hz = __fmaf_rn(c, fr[8 * nc], n * fr[11 * nc]);
+          const float4* fr = cell_rows<kPrecise>(D, sh.pos[t]);
+          const float4 fn = __ldg(fr + kFrameNorth), fe = __ldg(fr + kFrameEast);
+          const float hx = __fmaf_rn(c, fn.x, n * fe.x);
+          const float hy = __fmaf_rn(c, fn.y, n * fe.y);
+          const float hz = __fmaf_rn(c, fn.z, n * fe.z);
           const float4 u = sh.v[t][kRowUp];
           const float ux = u.x, uy = u.y, uz = u.z;
           sh.v[t][kRowAlong] = make_float4(hx, hy, hz, 0.f);
           sh.v[t][kRowSide] = make_float4(__fmaf_rn(hy, uz, -hz * uy), __fmaf_rn(hz, ux, -hx * uz),
                                           __fmaf_rn(hx, uy, -hy * ux), 0.f);
-          const Track tr = make_track(g, fr[12 * nc], fr[13 * nc], hx, hy, hz, ux, uy, uz);
+          const Track tr = make_track(g, fn.w, fe.w, hx, hy, hz, ux, uy, uz);
           sh.v[t][kRowTrack] = make_float4(tr.ox, tr.oy, tr.dx, tr.dy);
           sh.v[t][kRowHeight].x = tr.xlo * g.cmin * g.irlo;
           sh.v[t][kRowHeight].y = tr.xlo * g.iq;
@@ -1123,7 +1133,7 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
             st = kLaneAdvance;
         }
       }
-      if (__popc(__ballot_sync(kFull, st == kLaneWalk)) < HZ_WALK_MIN) break;
+      if (__popc(__ballot_sync(kFull, st == kLaneWalk)) < walk_min) break;
     }
     }
 
@@ -1326,7 +1336,7 @@ __global__ void k_sweep_runs(const DomainDesc* __restrict__ doms, int ndom, int 
   const int cell = (int)(gid - D.cell_offset);
   bool open = false;
   for (int r = 1; r < D.runs; r++) {
-    const int a = (int)((unsigned)r * (unsigned)D.L / (unsigned)D.runs);
+    const int a = run_start(D, r);
     const int16_t* c = D.codes + (long long)a * D.ncell + cell;
     open |= *c > kCodeAllMiss && c[-(long long)D.ncell] <= kRunStart + 1;
   }
@@ -1441,9 +1451,10 @@ __global__ void __launch_bounds__(128)
     const int cell = (int)(gid - D.cell_offset);
     const int p = list[w] - (int)D.k_begin;
     const long long nc = D.ncell;
-    const float* fr = D.cell_f32 + p;
-    const float ux = fr[3 * nc], uy = fr[4 * nc], uz = fr[5 * nc], X0 = fr[12 * nc],
-                Y0 = fr[13 * nc], ho = fr[14 * nc];
+    const float4* fr = cell_rows<kPrecise>(D, p);
+    const float4 fu = __ldg(fr + kFrameNormal), fn = __ldg(fr + kFrameNorth),
+                 fe = __ldg(fr + kFrameEast);
+    const float ho = __ldg(&fr[kFrameOrigin].w);
     const int safe = above_floor(D);
     int codes = 0;
     int m = 0, run = 0, before = 0;
@@ -1456,7 +1467,7 @@ __global__ void __launch_bounds__(128)
       int steps;
       // Where this azimuth's sweep began: the hits below that are not known.
       int from = s_full;
-      if ((int)((unsigned)run * (unsigned)D.L / (unsigned)D.runs) == a) {
+      if (run_start(D, run) == a) {
         from = a == 0 ? 0 : max(s_full, kRunStart);
         run++;
       } else if (before > kCodeAllMiss) {
@@ -1469,15 +1480,16 @@ __global__ void __launch_bounds__(128)
       }
       const double2 cs = __ldg(&D.azim_cs[a]);
       const float c = (float)cs.x, e = (float)cs.y;
-      const float hx = __fmaf_rn(c, fr[6 * nc], e * fr[9 * nc]);
-      const float hy = __fmaf_rn(c, fr[7 * nc], e * fr[10 * nc]);
-      const float hz = __fmaf_rn(c, fr[8 * nc], e * fr[11 * nc]);
+      const float hx = __fmaf_rn(c, fn.x, e * fe.x);
+      const float hy = __fmaf_rn(c, fn.y, e * fe.y);
+      const float hz = __fmaf_rn(c, fn.z, e * fe.z);
       auto ray_hits = [&](int mm) {
         double2 ecs;
         const Ray r = table_ray<kPrecise>(D, p, a, mm, ecs);
         // Beyond the zenith the ray runs along the opposite azimuth.
         const float sg = ecs.x < 0.0 ? -1.f : 1.f;
-        const Track tr = make_track(g, X0, Y0, sg * hx, sg * hy, sg * hz, ux, uy, uz);
+        const Track tr = make_track(g, fn.w, fe.w, sg * hx, sg * hy, sg * hz, fu.x,
+                                    fu.y, fu.z);
         const float c = fmaxf(fabsf((float)ecs.x), 1e-7f);
         return grid_ray<kPrecise>(D, g, r, tr, ho, __fdiv_rn((float)ecs.y, c));
       };
@@ -1612,7 +1624,7 @@ __global__ void k_sweep_finish(const DomainDesc* __restrict__ doms, int ndom, in
 
 long long sweep_cells_cap(long long n_tri) { return std::max(4096ll, 5 * n_tri / 2); }
 long long sweep_refs_cap(long long n_tri) { return 12 * n_tri + 4096; }
-size_t sweep_frame_floats() { return kFrameRows; }
+size_t sweep_frame_floats(bool precise) { return precise ? 20 : 16; }
 
 cudaError_t sweep_grid(const float* vert32, const float* vert_lo, const int* vot, int n_tri,
                        int n_vert, int tri_base, float tfar, const SweepBuffers& b, Tri* tris,
@@ -1647,18 +1659,46 @@ cudaError_t sweep_grid(const float* vert32, const float* vert_lo, const int* vot
   return cudaGetLastError();
 }
 
-// Resident blocks of the sweep over the device, at most one per kSweepBlock items.
-template <typename... P, typename... A>
-static cudaError_t launch_resident(void (*kernel)(P...), int block, long long most,
-                                   cudaStream_t s, A... args) {
+// Blocks of a kernel that are resident on the device at once; `wanted` per SM, for
+// which shared memory is set aside and the rest left to L1 (FP64 ray mode with the
+// share of six blocks where five run: 7.7 ms, with theirs 7.15).
+template <typename K>
+static long long resident_blocks(K kernel, int block, int wanted) {
   int dev = 0, sms = 0, per_sm = 0;
-  prefer_l1(kernel, HZ_SWEEP_MIN_BLOCKS);
+  prefer_l1(kernel, wanted);
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0);
-  long long blocks = (long long)sms * (per_sm > 0 ? per_sm : 1);
-  blocks = std::max(1ll, std::min(blocks, most));
-  kernel<<<(unsigned)blocks, block, 0, s>>>(args...);
+  return (long long)sms * (per_sm > 0 ? per_sm : 1);
+}
+
+template <bool kPrecise>
+static cudaError_t launch_search(const DomainDesc* doms, int ndom, const int32_t* order, int total,
+                                 int total_items, int s_full, int* work, int* list,
+                                 unsigned* listed, const SweepScene& sc, int* err,
+                                 cudaStream_t s) {
+  // Fewer items than resident threads go to all warps, a few lanes each: the
+  // lanes of a warp wait for one another's triangles and azimuths (500 cells x 24
+  // azimuths: 288 us in full warps, 187 with four lanes per warp).
+  const long long resident = resident_blocks(
+      k_sweep<kPrecise>, kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EXACT : HZ_SWEEP_MIN_BLOCKS);
+  const long long lanes = std::min(
+      32ll, std::max(1ll, ((long long)total_items + resident * kWarps - 1) / (resident * kWarps)));
+  const long long most = ((long long)total_items + lanes * kWarps - 1) / (lanes * kWarps);
+  k_sweep<kPrecise><<<(unsigned)std::min(resident, most), kSweepBlock, 0, s>>>(
+      doms, ndom, order, total_items, work, s_full, list, work + 1, listed, sc, (int)lanes, err);
+  note_launches(1);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  if (total_items > total) {
+    k_sweep_runs<<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, total, list, work + 1, listed,
+                                                      order, err);
+    note_launches(1);
+  }
+  const long long blocks = std::min(resident_blocks(k_sweep_repair<kPrecise>, 128, 4),
+                                    ((long long)total + 3) / 4);
+  k_sweep_repair<kPrecise><<<(unsigned)blocks, 128, 0, s>>>(doms, ndom, order, list, work + 1,
+                                                            work + 2, s_full, err);
   note_launches(1);
   return cudaGetLastError();
 }
@@ -1677,22 +1717,10 @@ cudaError_t sweep_search(const DomainDesc* doms, int ndom, const int32_t* order,
   else k_sweep_frames<false><<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, order, total);
   note_launches(1);
   const SweepScene sc{all.tris, all.tri_lo, all.refs, all.start, all.planes};
-  const long long most = ((long long)total_items + kSweepBlock - 1) / kSweepBlock;
-  e = precise ? launch_resident(k_sweep<true>, kSweepBlock, most, s, doms, ndom, order,
-                                total_items, work, s_full, list, work + 1, listed, sc, err)
-              : launch_resident(k_sweep<false>, kSweepBlock, most, s, doms, ndom, order,
-                                total_items, work, s_full, list, work + 1, listed, sc, err);
-  if (e != cudaSuccess) return e;
-  if (total_items > total) {
-    k_sweep_runs<<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, total, list, work + 1, listed,
-                                                      order, err);
-    note_launches(1);
-  }
-  const long long warps = ((long long)total + 3) / 4;
-  e = precise ? launch_resident(k_sweep_repair<true>, 128, warps, s, doms, ndom, order, list,
-                                work + 1, work + 2, s_full, err)
-              : launch_resident(k_sweep_repair<false>, 128, warps, s, doms, ndom, order, list,
-                                work + 1, work + 2, s_full, err);
+  e = precise ? launch_search<true>(doms, ndom, order, total, total_items, s_full, work, list,
+                                    listed, sc, err, s)
+              : launch_search<false>(doms, ndom, order, total, total_items, s_full, work, list,
+                                     listed, sc, err, s);
   if (e != cudaSuccess) return e;
   k_sweep_finish<<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, total, counters, err);
   note_launches(1);
