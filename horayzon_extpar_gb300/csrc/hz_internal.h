@@ -285,7 +285,10 @@ struct SweepAll {
   uint16_t* low;
   uint2* planes;
 };
-// Frames, sweep, repair and outputs of all domains (after cell_order and
+// Cell frames of all domains (after cell_order).
+cudaError_t sweep_frames(const DomainDesc* doms, int ndom, const int32_t* order, int total,
+                         bool precise, cudaStream_t s);
+// Sweep, repair and outputs of all domains (after sweep_frames and
 // trace_tables). s_full: the lowest lattice elevation a search can ask for.
 // work: 3 ints; list, listed: `total` work positions and bits.
 cudaError_t sweep_search(const DomainDesc* doms, int ndom, const int32_t* order, int total,

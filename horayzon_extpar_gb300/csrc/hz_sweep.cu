@@ -1703,6 +1703,15 @@ static cudaError_t launch_search(const DomainDesc* doms, int ndom, const int32_t
   return cudaGetLastError();
 }
 
+cudaError_t sweep_frames(const DomainDesc* doms, int ndom, const int32_t* order, int total,
+                         bool precise, cudaStream_t s) {
+  if (total <= 0 || ndom <= 0) return cudaSuccess;
+  if (precise) k_sweep_frames<true><<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, order, total);
+  else k_sweep_frames<false><<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, order, total);
+  note_launches(1);
+  return cudaGetLastError();
+}
+
 cudaError_t sweep_search(const DomainDesc* doms, int ndom, const int32_t* order, int total,
                          int total_items, int s_full, int* work, int* list, unsigned* listed,
                          const SweepAll& all, unsigned long long* counters, int* err,
@@ -1713,9 +1722,6 @@ cudaError_t sweep_search(const DomainDesc* doms, int ndom, const int32_t* order,
   if (e == cudaSuccess)
     e = cudaMemsetAsync(listed, 0, sizeof(unsigned) * ((size_t)total / 32 + 1), s);
   if (e != cudaSuccess) return e;
-  if (precise) k_sweep_frames<true><<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, order, total);
-  else k_sweep_frames<false><<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, order, total);
-  note_launches(1);
   const SweepScene sc{all.tris, all.tri_lo, all.refs, all.start, all.planes};
   e = precise ? launch_search<true>(doms, ndom, order, total, total_items, s_full, work, list,
                                     listed, sc, err, s)
