@@ -531,8 +531,17 @@ int resident_lanes(long long* lanes) {
 // Searches of more items than this many times the resident lanes queue the
 // border cells of each domain first (run_batch).
 constexpr long long kBorderFirstWaves = 4;
-// Sweep items per resident lane that a call aims at.
+// Sweep items per resident lane that a call aims at: a run's first azimuth
+// costs half an azimuth more, long runs leave lanes idle at the end. Half as many
+// where runs then still hold kTailAzimuths and the tail's are split (194k cells in
+// FP64 ray mode 6.65 -> 6.33 ms; 57k cells, runs of two azimuths, given starts: whole
+// call 1.38, with four 1.42).
 constexpr long long kSweepWaves = 4;
+// The last cells of the queue, one item per lane, go in up to kTailSplit times
+// as many runs of at least kTailAzimuths: the lanes finish together (194k cells x
+// 240 azimuths 41.4 -> 40.1 ms, 1.2M cells 42.6 -> 41.9; with the runs of two
+// azimuths 21k cells x 360 lost 4 %).
+constexpr int kTailSplit = 4, kTailAzimuths = 4;
 
 // Runs the pipeline for n domains whose arrays are device pointers in pr[].
 // With stop != kFull it ends after the mesh (or ENU) stage and leaves the
@@ -756,11 +765,12 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
     if (rl) return rl;
     const bool border_first = !sweep && items >= kBorderFirstWaves * lanes;
     // Sweep items: runs of consecutive azimuths per cell, enough of them to
-    // fill the lanes a few times over (the first azimuth of a run sweeps from
-    // the floor, 1.1 to 1.4 times the work of one that follows another).
+    // fill the lanes a few times over.
     long long cells_all = 0;
     for (int d = 0; d < n; d++) cells_all += pr[d].cell_count;
     const long long runs_wanted = (kSweepWaves * lanes + cells_all - 1) / std::max(1ll, cells_all);
+    const long long runs_half =
+        (kSweepWaves / 2 * lanes + cells_all - 1) / std::max(1ll, cells_all);
     // Queue order of the domains: least work (cells x azimuths) first, so
     // that the small domains of a batch complete early (shortest job first:
     // the lowest mean completion time for the same total work).
@@ -854,9 +864,20 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
         D.tris = bb.all.tris;
         D.tri_lo = bb.all.tri_lo;
       }
-      D.runs = (int)std::max(1ll, std::min<long long>(L, runs_wanted));
+      D.runs = (int)std::max(
+          1ll, std::min<long long>(L, L / runs_wanted >= kTailAzimuths ? runs_half : runs_wanted));
       D.run_len = L / D.runs;
       D.run_extra = L % D.runs;
+      D.tail_begin = P.cell_count;
+      D.tail_runs = D.runs;
+      if (j == n - 1 && D.run_len >= kTailAzimuths) {
+        D.tail_runs = std::max(D.runs, std::min(kTailSplit * D.runs, L / kTailAzimuths));
+        D.tail_begin -= (int)std::min<long long>(P.cell_count / 2, lanes / D.runs);
+      }
+      D.tail_run_len = L / D.tail_runs;
+      D.tail_run_extra = L % D.tail_runs;
+      D.items = (long long)D.tail_begin * D.runs +
+                (long long)(P.cell_count - D.tail_begin) * D.tail_runs;
       D.centre = frames[d].centre;
       D.pole = frames[d].pole;
       D.ray_org_elev = P.ray_org_elev;
@@ -875,7 +896,7 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
       D.tfar = (float)P.dist_search;
       desc[j] = D;  // in queue order: k_begin and item_begin increase with j
       total += P.cell_count;
-      total_items += (long long)P.cell_count * (sweep ? D.runs : P.groups);
+      total_items += sweep ? D.items : (long long)P.cell_count * P.groups;
     }
     const auto frames_on = [&](cudaStream_t to) {
       const cudaError_t e = cudaMemcpyAsync(bb.doms, desc, sizeof(DomainDesc) * (size_t)n,

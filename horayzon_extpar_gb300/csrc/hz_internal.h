@@ -196,7 +196,8 @@ struct DomainDesc {
   int occ_cache;
   // Profile sweep (hz_sweep.cu): grid, pyramid, list starts and lists; FP32
   // cell frames by work position; result codes [L][ncell]; items per cell (runs of
-  // consecutive azimuths: run_len each, the first run_extra one more).
+  // consecutive azimuths: run_len each, the first run_extra one more), the same for
+  // the cells from work position tail_begin on, and items of the domain.
   const GridDesc* grid;
   const uint2* planes;
   const uint16_t* low;
@@ -208,6 +209,8 @@ struct DomainDesc {
   unsigned ref_base;          // list entries, in the call's arrays (SweepAll)
   const float* tan_m;         // [kTanTable] tangents of (k - kTanTable / 2) * 0.5 deg
   int runs, run_len, run_extra;
+  int tail_begin, tail_runs, tail_run_len, tail_run_extra;
+  long long items;
   int16_t* raw_j;             // optional output: unclipped horizon j (h = j * 0.25 deg)
   double3 centre, pole;       // Earth centre / North Pole in ENU
   double ray_org_elev, hori_acc, elev_floor;

@@ -625,10 +625,11 @@ __device__ __forceinline__ Track make_track(const GridDesc& g, float X0, float Y
   return t;
 }
 
-// First azimuth of a run of azimuths (of run D.runs: L); the first run_extra
-// runs hold one more than run_len.
-__device__ __forceinline__ int run_start(const DomainDesc& D, int run) {
-  return run * D.run_len + min(run, D.run_extra);
+// First azimuth of a run of azimuths (of run D.runs: L) of the cell at position p;
+// the first `extra` runs hold one more than the others.
+__device__ __forceinline__ int run_start(const DomainDesc& D, int p, int run) {
+  const bool tail = p >= D.tail_begin;
+  return run * (tail ? D.tail_run_len : D.run_len) + min(run, tail ? D.tail_run_extra : D.run_extra);
 }
 
 // ---------------------------------------------------------------------------
@@ -906,8 +907,6 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
   __syncthreads();
 
   bool alive = lane < lanes;
-  const int walk_min = max(1, lanes * HZ_WALK_MIN >> 5),
-            adv_min = max(1, lanes * HZ_SWEEP_ADVANCE >> 5);
   int st = kLaneAdvance, fl = 0;
   int m = 0;
   int i = 0, j = 0, l = 0;
@@ -939,6 +938,9 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
   for (;;) {
     const unsigned live = __ballot_sync(kFull, alive);
     if (live == 0u) break;
+    // Shares of the lanes at work: few in small domains and at the queue's end.
+    const int walk_min = max(1, __popc(live) * HZ_WALK_MIN >> 5),
+              adv_min = max(1, __popc(live) * HZ_SWEEP_ADVANCE >> 5);
     const unsigned waiting = __ballot_sync(kFull, alive && st == kLaneAdvance);
     if (waiting != 0u && (__popc(waiting) >= adv_min || waiting == live)) {
       const bool mine = alive && st == kLaneAdvance;
@@ -973,7 +975,7 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
           sh.az[t] = a + 1;
           if (a + 1 == sh.az_end[t] && D.done) {
             const unsigned long long fin = atomicAdd(&D.done[0], 1ull) + 1ull;
-            if (fin == (unsigned long long)D.ncell_traced * (unsigned long long)D.runs) {
+            if (fin == (unsigned long long)D.items) {
               unsigned long long now;
               asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
               D.done[1] = now;
@@ -1013,8 +1015,13 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
             const DomainDesc& D = doms[dom];
             const unsigned local = (unsigned)(item - D.item_begin);
             // Quotient from FP32, off by one at most (fewer runs than 2^20).
-            const unsigned run = local / (unsigned)D.ncell_traced;
-            const int p = (int)(local - run * (unsigned)D.ncell_traced);
+            // Run by run over the cells; then over those of the tail.
+            const unsigned whole = (unsigned)D.tail_begin * (unsigned)D.runs;
+            const bool tail = local >= whole;
+            const unsigned rest = tail ? local - whole : local;
+            const unsigned cells = (unsigned)(tail ? D.ncell_traced - D.tail_begin : D.tail_begin);
+            const unsigned run = rest / cells;
+            const int p = (int)(rest - run * cells) + (tail ? D.tail_begin : 0);
             const float4* fr = cell_rows<kPrecise>(D, p);
             const float4 fo = __ldg(fr + kFrameOrigin), fu = __ldg(fr + kFrameNormal);
             sh.v[t][kRowOrigin] = make_float4(fo.x, fo.y, fo.z, 0.f);
@@ -1028,8 +1035,8 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
             sh.dom[t] = dom;
             sh.cell[t] = (int)(order[D.k_begin + p] - D.cell_offset);
             sh.pos[t] = p;
-            sh.az[t] = run_start(D, (int)run);
-            sh.az_end[t] = run_start(D, (int)run + 1);
+            sh.az[t] = run_start(D, p, (int)run);
+            sh.az_end[t] = run_start(D, p, (int)run + 1);
             sh.prev[t] = sh.az[t] == 0 ? 2 : kFirst;  // the search starts at 0 (cpp:511)
           }
         }
@@ -1335,8 +1342,9 @@ __global__ void k_sweep_runs(const DomainDesc* __restrict__ doms, int ndom, int 
   const DomainDesc& D = doms[domain_of(doms, ndom, gid)];
   const int cell = (int)(gid - D.cell_offset);
   bool open = false;
-  for (int r = 1; r < D.runs; r++) {
-    const int a = run_start(D, r);
+  const int p = (int)(k - D.k_begin), runs = p >= D.tail_begin ? D.tail_runs : D.runs;
+  for (int r = 1; r < runs; r++) {
+    const int a = run_start(D, p, r);
     const int16_t* c = D.codes + (long long)a * D.ncell + cell;
     open |= *c > kCodeAllMiss && c[-(long long)D.ncell] <= kRunStart + 1;
   }
@@ -1467,7 +1475,7 @@ __global__ void __launch_bounds__(128)
       int steps;
       // Where this azimuth's sweep began: the hits below that are not known.
       int from = s_full;
-      if (run_start(D, run) == a) {
+      if (run_start(D, p, run) == a) {
         from = a == 0 ? 0 : max(s_full, kRunStart);
         run++;
       } else if (before > kCodeAllMiss) {
