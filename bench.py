@@ -1,8 +1,8 @@
 """Benchmark: horizon evaluations/s of the HORAYZON horizon + SVF path.
 
 One step = one full pass of the hot path over one domain: triangle-mesh
-assembly, geodetic frames, LBVH build and the bracketing horizon search with
-the SVF epilogue (mo_lradtopo_horayzon.cpp:562-785), on the 500 m / 600 x 600
+assembly, geodetic frames, grid build and the horizon search with the SVF
+epilogue (mo_lradtopo_horayzon.cpp:562-785), on the 500 m / 600 x 600
 km / nhori 24 workload (~3.1M cells; grid_type 1, dist_search 40 km,
 ray_org_elev 0.2 m, refine_factor 1, svf_type 2). One horizon evaluation is
 one (cell, azimuth) of the output.
@@ -12,9 +12,9 @@ one (cell, azimuth) of the output.
   between steps, max over ranks.
 * ``e2e``: the public host entry (hz_horizon_svf) on pinned host buffers,
   host->device inputs and device->host outputs inside the timed region.
-* ``roofline``: the horizon-search kernel; algorithmic bytes per launch =
-  64 B per BVH node visit + 48 B per triangle test, counted on the device
-  over the same launch.
+* ``roofline``: the call against the bytes it cannot do without (every input
+  read once, every output written once); beside them the rays, node visits and
+  triangle tests of the same search by tree traversal, counted on the device.
 * ``cpu_baseline`` (rank 0, N=1): the CPU oracle on all host cores on a
   bounded sample (full mesh + BVH build, ray phase on a random cell subset,
   scaled to the full domain).
@@ -45,9 +45,6 @@ METRIC = ("horizon evals/s (cells×azimuths) 500 m nhori=24, learned vs plain GP
           "rays/s")
 WORKLOAD = "500 m ICON-like grid, 600x600 km, fBm(H=0.7)+ridged noise 200-4800 m, nhori=24"
 ARGS = (24, 1, 40000.0, 0.2, 1, 2)  # num_hori, grid_type, dist_search, ray_org_elev, refine, svf
-BYTES_PER_NODE = 64
-BYTES_PER_TRI = 48
-BUILD_BYTES_PER_TRI = 2 * 12 + 36 + 64
 EXTRAS = ("learned", "learned_small", "precision", "batch", "drop_in", "configs")
 
 
@@ -110,7 +107,7 @@ def l2_read_peak(dev) -> float | None:
 
 def traffic_from_profile():
     """DRAM bytes per launch of the search kernel from the committed ncu summary."""
-    path = os.path.join(ROOT, "profiles", "k_trace_warp_c3_500m.md")
+    path = os.path.join(ROOT, "profiles", "k_sweep_c3_300km.md")
     if not os.path.exists(path):
         return None
     for line in open(path):
@@ -632,11 +629,9 @@ def run_gpu(args):
                                        stream=stream, count_work=count, kernel=kernel,
                                        leaf_size=leaf_size)[2]
 
-    # Untimed: work counters. The algorithmic bytes are defined on the binary
-    # LBVH with leaves of <= 4 triangles (64 B per node visit, 48 B per
-    # triangle test), so they are counted by the same search on that tree;
-    # the counts of the timed kernel (4-wide tree, default leaves) are
-    # reported beside them.
+    # Untimed: work counters of the search by tree traversal, on the binary
+    # tree with leaves of <= 4 triangles and on the 4-wide one (the timed search
+    # is the profile sweep, which visits no tree; its rays are the same).
     st_count = step(count=True, kernel=_lib.HZ_KERNEL_PERSISTENT_BVH2, leaf_size=4)
     st_wide = step(count=True)
     l2_peak = l2_read_peak(dev)
@@ -745,13 +740,8 @@ def run_gpu(args):
     del sample
 
     peak, peak_kind = measured_peaks()
-    alg_bytes = BYTES_PER_NODE * st_count["node_visits"] + BYTES_PER_TRI * st_count["tri_tests"]
-    achieved = alg_bytes / (trace_ms * 1e-3) / 1e9
-    # LBVH build phase: 2 sort passes x 12 B + 36 B triangle + 64 B node per
-    # triangle, over the phase's CUDA-event time.
-    bvh_ms = float(np.mean([s["ms_bvh"] for s in stats]))
-    build_bytes = BUILD_BYTES_PER_TRI * st_count["n_tri"]
-    build_achieved = build_bytes / (bvh_ms * 1e-3) / 1e9
+    alg_bytes = h2d + d2h
+    achieved = alg_bytes / (ms * 1e-3) / 1e9
     traffic = traffic_from_profile()
 
     if rank != 0:
@@ -784,35 +774,27 @@ def run_gpu(args):
         "rays_per_s": world * rays / (ms * 1e-3),
         "rays_per_eval": rays / evals,
         "phase_ms": {"mesh": float(np.mean([s["ms_mesh"] for s in stats])),
-                     "bvh": float(np.mean([s["ms_bvh"] for s in stats])),
+                     "grid": float(np.mean([s["ms_bvh"] for s in stats])),
                      "trace": trace_ms},
         "e2e": {"value": world * evals / e2e_s, "unit": "evals/s",
                 "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
                 "wall_ms_per_step": 1e3 * e2e_s,
                 "phase_ms_last_step": {k: float(getattr(st, k)) for k in (
                     "ms_h2d", "ms_mesh", "ms_bvh", "ms_trace", "ms_d2h")}},
-        # The search reads its tree and triangles mostly from L1 / L2 (DRAM
-        # traffic is ~2 % of the algorithmic bytes): `frac` is the HBM-
-        # equivalent fraction of the measured copy bandwidth, `l2_frac` the
-        # fraction of the L2 read bandwidth measured by the project's probe;
-        # the measured limiter is L1/L2 latency and instruction issue.
-        "roofline": {"kernel": "k_trace_warp", "bound": "l1/l2 latency + issue",
+        # The sweep reads its grid and triangles from L1 / L2: what bounds it is
+        # instruction issue and the latency of those reads, not bytes.
+        "roofline": {"kernel": "k_sweep", "bound": "instruction issue + l1/l2 latency",
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
                      "frac_of": "measured HBM copy bandwidth (MEASURED_PEAKS.json hbm_gbs)",
+                     "alg_bytes_per_step": alg_bytes,
+                     "floor_ms": alg_bytes / (peak * 1e9) * 1e3,
                      "l2_peak": l2_peak,
-                     "l2_frac": achieved / l2_peak if l2_peak else None,
                      "l2_peak_kind": "measured (hz_l2_probe: 32 MiB, 300 passes, ld.global.cg)",
-                     "alg_bytes_per_launch": alg_bytes,
-                     "node_visits_per_ray": st_count["node_visits"] / rays,
-                     "tri_tests_per_ray": st_count["tri_tests"] / rays,
+                     "tree_node_visits_per_ray": st_count["node_visits"] / rays,
+                     "tree_tri_tests_per_ray": st_count["tri_tests"] / rays,
                      "bvh4_node_visits_per_ray": st_wide["node_visits"] / rays,
-                     "bvh4_tri_tests_per_ray": st_wide["tri_tests"] / rays,
-                     "build_bytes_per_triangle": BUILD_BYTES_PER_TRI,
-                     "build_bytes_per_launch": build_bytes, "build_ms": bvh_ms,
-                     "build_achieved": build_achieved, "build_frac": build_achieved / peak,
-                     "build_bound": "latency (bottom-up refit chains) and issue (Karras "
-                                    "splits)"},
+                     "bvh4_tri_tests_per_ray": st_wide["tri_tests"] / rays},
         "parity": parity,
         "cpu_baseline": cpu,
         "clocks": clk.summary(),

@@ -1,7 +1,9 @@
 """Autotuner for the launch knobs of the persistent horizon search.
 
 The knobs change speed, never results (the same rays are cast and every hit
-decision is the watertight test's):
+decision is the watertight test's). All of them 0 is the profile sweep, the
+library's choice wherever its grid can hold the domain; any other value selects
+the search by tree traversal with that setting:
 
 * ``leaf_size``: most triangles per BVH leaf (1..8);
 * ``advance_min``: lanes of a warp that must be waiting before the search
@@ -31,13 +33,13 @@ from .horizon_svf import horizon_svf_comp_device
 
 #: Candidate values per knob, in the order the descent visits them.
 GRID = {
-    "leaf_size": (2, 1, 3, 4, 6),
-    "advance_min": (16, 12, 20, 8, 24),
-    "leaf_min": (1, 2, 4, 8, 12),
-    "queue_chunk": (32, 16, 24, 48, 64),
+    "leaf_size": (0, 2, 1, 3, 4, 6),
+    "advance_min": (0, 16, 12, 20, 8, 24),
+    "leaf_min": (0, 1, 2, 4, 8, 12),
+    "queue_chunk": (0, 32, 16, 24, 48, 64),
     "kernel": (_lib.HZ_KERNEL_PERSISTENT, _lib.HZ_KERNEL_PERSISTENT_BVH2),
 }
-DEFAULTS = {"leaf_size": 2, "advance_min": 16, "leaf_min": 1, "queue_chunk": 32,
+DEFAULTS = {"leaf_size": 0, "advance_min": 0, "leaf_min": 0, "queue_chunk": 0,
             "kernel": _lib.HZ_KERNEL_PERSISTENT}
 _lock = threading.Lock()
 
@@ -50,12 +52,14 @@ def cache_path() -> str:
 
 def workload_key(ncell: int, args) -> str:
     """Cache key: GPU name, log2 bucket of the cell count and the arguments
-    that change the search (num_hori, grid_type, dist_search, refine_factor)."""
+    that change the search (num_hori, grid_type, dist_search, refine_factor).
+    Settings stored before the profile sweep was among the candidates have
+    keys without its name."""
     import torch
     num_hori, grid_type, dist_search, _, refine_factor, _ = args
-    return "%s|2^%d|%d|%d|%g|%d" % (torch.cuda.get_device_name(), int(math.log2(max(ncell, 1))),
-                                    int(num_hori), int(grid_type), float(dist_search),
-                                    int(refine_factor))
+    return "%s|2^%d|%d|%d|%g|%d|sweep" % (torch.cuda.get_device_name(), int(math.log2(max(ncell, 1))),
+                                          int(num_hori), int(grid_type), float(dist_search),
+                                          int(refine_factor))
 
 
 def _load_cache(path):
