@@ -53,6 +53,11 @@ def _same(inputs, args, **kw):
     (dict(edge_km=0.5, box_km=95.0, seed=10, hmax=3000.0), (77, 1, 6000.0, 0.2, 1, 2), {}),
     (dict(edge_km=0.5, box_km=95.0, seed=10, hmax=3000.0), (45, 1, 6000.0, 0.2, 2, 0),
      {"cells": (3001, 14003), "precision": 1}),
+    # azimuths close together, and starts one step below the one before
+    (dict(edge_km=0.5, box_km=40.0, seed=14, hmax=4000.0), (159, 1, 9000.0, 0.2, 1, 2), {}),
+    (dict(edge_km=0.5, box_km=40.0, seed=14, hmax=4000.0), (80, 1, 9000.0, 0.2, 2, 1), {}),
+    (dict(edge_km=0.2, box_km=8.0, seed=15, kind="eroded", hmax=3000.0),
+     (360, 0, 8000.0, 0.2, 1, 2), {"precision": 1}),
     # a triangle cut by many rays at the search radius, beyond it at the higher
     (dict(edge_km=0.24629858041449693, box_km=17.611548057004665, kind="eroded",
           hmin=268.98230903271724, hmax=9000, hurst=0.9368420793831944, n_features=6, seed=319,
