@@ -142,11 +142,12 @@ def horizon_svf_comp_py(clon, clat, hsurf, vlon, vlat, cells_of_vertex, num_hori
     [deg] and ``skyview`` (ncell) as new C-order float64 arrays. Keyword-only
     extras: CUDA ``device``, work counters, the downward-walk bound, a cell
     range ``cells=(begin, end)`` to trace (entries outside it are NaN), the
-    search ``kernel`` (0 persistent, 1 one thread per cell, 2 the
-    persistent search on the binary BVH), its ``advance_min`` / ``leaf_min``
-    knobs, the work-queue ``queue_chunk``, the BVH ``leaf_size``,
+    search ``kernel`` (0 persistent: the profile sweep, or the search on the
+    4-wide BVH where one of the following knobs or ``count_work`` asks for it;
+    1 one thread per cell, 2 the persistent search on the binary BVH), its
+    ``advance_min`` / ``leaf_min`` knobs, the work-queue ``queue_chunk``, the BVH ``leaf_size``,
     ``direct_launch`` (launch each kernel directly instead of replaying the
-    captured CUDA graph of the BVH build and search), ``bvh_treelets``
+    captured CUDA graph of the build and search), ``bvh_treelets``
     (treelet restructuring of the BVH: same results), ``elev_walk`` (1:
     bisection for the downward walk below the clip, see hz_options),
     ``occluder_cache`` (False: traverse the tree for every ray; same
