@@ -41,10 +41,14 @@
 // Against the tree search (GB300, whole call): one traversal of a bounding
 // volume tree per ray took 2.5 to 4 rays, 63 to 126 four-wide node visits and 38
 // to 76 triangle tests per evaluation; the sweep takes 40 to 66 eight-byte steps and
-// 15 to 23 tests. 500 m, 3.1M cells 132.9 -> 64.1 ms; 100 m, 1.2M cells 115.9 ->
-// 51.1 ms; 2.5 km, 57k cells 7.8 -> 1.8 ms; 500 cells 5.3 -> 1.0 ms; 360 azimuths,
-// 21k cells 56.3 -> 11.3 ms. The small domains gain most: a sweep from the floor
-// needs no other azimuth's result, so a cell's azimuths run side by side.
+// 15 to 23 tests. 500 m, 3.1M cells 132 -> 62 ms; 100 m, 1.2M cells 117 -> 39.9 ms; 2.5 km,
+// 57k cells 7.6 -> 1.36 ms; 500 cells 5.4 -> 0.7 ms; 360 azimuths, 21k cells 55.7 -> 9.7 ms.
+// The small domains gain most: a sweep from a low start needs no other azimuth's
+// result, so a cell's azimuths run side by side.
+//
+// What bounds it: instruction issue (62 % of the cycles at 17.8 of 32 lanes, 640 warp
+// instructions per evaluation) and L1/L2 latency with 24 resident warps per SM; DRAM
+// is idle (0.7 %).
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -66,17 +70,22 @@ constexpr int kSweepBlock = 128;
 #ifndef HZ_SWEEP_MIN_BLOCKS_EXACT
 #define HZ_SWEEP_MIN_BLOCKS_EXACT 5
 #endif
+// Pyramid steps per lane in one walk pass (6: +0.7 %, 11: the same); of 32 live
+// lanes, those that must still walk for the pass to go on (9: +0.6 %, 15: the same)
+// and those that must wait before azimuths are set up (57k cells: 3 1.08 ms, 5 1.06, 7
+// 1.03, 8 1.03; 1.2M cells 39.1, 38.7, 38.8, 39.0); a grid cell's area in mean triangle
+// areas (0.8 and 1.25 within 1 %, 2.2 +5 %).
 #ifndef HZ_WALK_STEPS
-#define HZ_WALK_STEPS 8  // pyramid steps per lane in one walk pass
+#define HZ_WALK_STEPS 8
 #endif
 #ifndef HZ_WALK_MIN
-#define HZ_WALK_MIN 12  // a walk pass ends when fewer lanes walk
-#endif
-#ifndef HZ_CELL_TRIS
-#define HZ_CELL_TRIS 1.0f  // cell area in mean triangle areas
+#define HZ_WALK_MIN 14
 #endif
 #ifndef HZ_SWEEP_ADVANCE
-#define HZ_SWEEP_ADVANCE 5  // lanes that must wait before azimuths are set up
+#define HZ_SWEEP_ADVANCE 7
+#endif
+#ifndef HZ_CELL_TRIS
+#define HZ_CELL_TRIS 1.0f
 #endif
 
 constexpr float kRf = 6371229.0f;         // kEarthRadius, exact in FP32
