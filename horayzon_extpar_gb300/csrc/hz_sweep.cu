@@ -118,6 +118,10 @@ __device__ __forceinline__ float height_magic(unsigned h16) {
 // ---------------------------------------------------------------------------
 // Grid build
 // ---------------------------------------------------------------------------
+// 9.4M triangles, ms: k_gnomonic 0.13, k_grid_count 0.37, k_grid_fill 0.60 (a scattered
+// atomic and an 8-byte store per list entry, 4.8 a triangle), k_grid_heights 0.55
+// (scattered vertex reads), k_grid_up 0.13; the tree build that this replaces
+// took 2.4 in all.
 
 // Gnomonic X, Y and height above the sphere of every mesh vertex, and their
 // bounds (ordered keys): min X, Y, H, z; max X, Y, H. The height is (r^2 -
@@ -567,6 +571,7 @@ __device__ __noinline__ bool exact_hit(const DomainDesc* D, int p, int a, int m,
   return test_tri<kPrecise>(D->tris, D->tri_lo, r, tri);
 }
 
+// FP64 pipe (square roots and divisions): 3.1M cells 0.75 ms, beside the grid build.
 template <bool kPrecise>
 __global__ void k_sweep_frames(const DomainDesc* __restrict__ doms, int ndom,
                                const int* __restrict__ order, int total) {
@@ -1477,7 +1482,10 @@ __device__ __forceinline__ void chain_start(const DomainDesc& D, int cell, int a
 }
 
 // A warp per listed cell: replays the cell's azimuths and searches the ones
-// left open by rays, 32 elevations at a time.
+// left open by rays, 32 elevations at a time. Latency of a few border cells: 20,000
+// to 70,000 cycles per round of 32 rays, whose grazing ones walk the whole track, 2.1
+// rounds per open azimuth (57k cells 0.18 ms, 1.2M cells at 100 m 1.3). Neither five to
+// eight blocks per SM nor list entries four at a time changed it.
 template <bool kPrecise>
 __global__ void __launch_bounds__(128)
     k_sweep_repair(const DomainDesc* __restrict__ doms, int ndom, const int* __restrict__ order,
