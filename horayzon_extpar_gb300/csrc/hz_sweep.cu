@@ -198,8 +198,11 @@ __global__ void k_grid_setup(const unsigned* __restrict__ b, int n_tri, long lon
   q.irlo = 1.f / q.rlo;
   const float s = fminf(tfar / q.rlo, 0.5f);
   q.tau_max = s / sqrtf(1.f - s * s) * 1.0001f;
+  // A ray's height over its origin's sphere gains x^2 times these over rlo.
   q.cmin = (q.rlo / q.rhi) * (1.f - 0.25f * q.tau_max * q.tau_max) * 0.5f;
-  q.cmax = (q.rhi / q.rlo) * 0.5f;
+  // x^2 / (r (1 + cos psi)), r >= rlo: at 500 km the cosine alone lifts a ray's
+  // height by 30 m against x^2 / 2 rlo.
+  q.cmax = (q.rhi / q.rlo) / (1.f + rsqrtf(1.f + 1.01f * q.tau_max * q.tau_max));
   q.W = W;
   q.H = H;
   q.L = L;

@@ -133,3 +133,24 @@ def test_gpu_sweep_given_starts(groups, every):
         out.append((h, s, raw, st["num_rays"]))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
     assert torch.equal(out[0][2], out[1][2]) and out[0][3] == out[1][3]
+
+
+@pytest.mark.parametrize("dkw,args,kw", [
+    (dict(edge_km=5.0, box_km=600.0, seed=3, hmax=3500.0), (4, 1, 500000.0, 80000.0, 1, 2), {}),
+])
+def test_gpu_sweep_of_far_rays_in_mid_air(dkw, args, kw):
+    """Origins high over the terrain: the rays that a search casts below its
+    horizon end in mid-air or meet terrain hundreds of kilometres away, where the
+    upper bound of a ray's height has to hold the curvature term's cosine too.
+    The horizons there are clipped to 0: the unclipped indices are compared."""
+    torch = pytest.importorskip("torch")
+    from horayzon_extpar_gb300 import horizon_svf_comp_device
+    d = synthetic.make_domain(**dkw)
+    t = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in d.inputs()]
+    out = []
+    for opt in ({"leaf_size": 2}, {}):
+        raw = torch.empty((args[0] * args[4], d.ncell), dtype=torch.int16, device="cuda")
+        h, s, st = horizon_svf_comp_device(*t, *args, raw_index=raw, **opt, **kw)
+        out.append((h, s, raw, st["num_rays"]))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    assert torch.equal(out[0][2], out[1][2]) and out[0][3] == out[1][3]
