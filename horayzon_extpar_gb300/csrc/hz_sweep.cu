@@ -628,9 +628,12 @@ __device__ __forceinline__ Track make_track(const GridDesc& g, float X0, float Y
   const float lambda = __fdividef(kRf, uz);  // |(X0, Y0, R)|, along u
   t.smax = __fdividef(g.tau_max * lambda, fmaxf(__fmaf_rn(-g.tau_max, gu, gh), 1e-3f)) * 1.0001f +
            2.f * g.pad;
-  const float a0 = __fdividef(gh, lambda);
-  const float a1 = __fdividef(gh, __fmaf_rn(t.smax, gu, lambda));
-  t.xlo = fminf(a0, a1) * (1.f - 4e-6f) * g.rlo;
+  // sin(psi) / s is gh over the distance of the line's point from the centre: the
+  // farther end has the lowest, tan(psi) / s of either end is no less than any.
+  const float a0 = __fdividef(gh, lambda), end = __fmaf_rn(t.smax, gu, lambda);
+  const float a1 = __fdividef(gh, end);
+  const float far = rsqrtf(__fmaf_rn(end, end, t.smax * gh * (t.smax * gh)));
+  t.xlo = fminf(a0, gh * far) * (1.f - 4e-6f) * g.rlo;
   t.xhi = fmaxf(a0, a1) * (1.f + 4e-6f) * g.rhi;
   t.ox = (X0 - g.x0) * g.inv_c;
   t.oy = (Y0 - g.y0) * g.inv_c;

@@ -137,11 +137,15 @@ def test_gpu_sweep_given_starts(groups, every):
 
 @pytest.mark.parametrize("dkw,args,kw", [
     (dict(edge_km=5.0, box_km=600.0, seed=3, hmax=3500.0), (4, 1, 500000.0, 80000.0, 1, 2), {}),
+    (dict(edge_km=10.0, box_km=1100.0, seed=207, hmax=2000.0), (5, 0, 500000.0, 100000.0, 1, 1),
+     {"precision": 1}),
+    (dict(edge_km=12.0, box_km=1100.0, seed=30, kind="eroded", hmax=5000.0),
+     (5, 0, 500000.0, 100000.0, 1, 0), {}),
 ])
 def test_gpu_sweep_of_far_rays_in_mid_air(dkw, args, kw):
     """Origins high over the terrain: the rays that a search casts below its
     horizon end in mid-air or meet terrain hundreds of kilometres away, where the
-    upper bound of a ray's height has to hold the curvature term's cosine too.
+    bounds of a ray's height have to hold the cosine of the angle at the centre.
     The horizons there are clipped to 0: the unclipped indices are compared."""
     torch = pytest.importorskip("torch")
     from horayzon_extpar_gb300 import horizon_svf_comp_device
