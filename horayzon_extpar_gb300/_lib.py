@@ -25,7 +25,10 @@ EXPORTED_SYMBOLS = ("hz_default_options", "horizon_svf_comp", "horizon_svf_comp_
                     "hz_last_error", "hz_version", "hz_release_workspace",
                     "hz_horizon_svf_device_static", "hz_horizon_svf_batch",
                     "hz_mlp_num_params", "hz_mlp_train_step", "hz_mlp_forward",
-                    "hz_distance_to_border", "hz_occluded32")
+                    "hz_distance_to_border", "hz_occluded32", "hz_last_search")
+
+#: hz_last_search in words (HZ_SEARCH_*).
+SEARCHES = ("none", "sweep", "tree", "sweep, then tree")
 
 
 class Domain(C.Structure):
@@ -68,7 +71,10 @@ class Stats(C.Structure):
                 ("ms_total", C.c_double), ("kernel_launches", C.c_int64)]
 
     def as_dict(self):
-        return {k: getattr(self, k) for k, _ in self._fields_}
+        """The members, and the search that this thread's last call ran."""
+        d = {k: getattr(self, k) for k, _ in self._fields_}
+        d["search"] = SEARCHES[load().hz_last_search()]
+        return d
 
 
 class HorizonError(RuntimeError):
@@ -105,6 +111,8 @@ def load(build_if_missing: bool = True):
         L.hz_last_error.restype = C.c_char_p
         L.hz_last_error.argtypes = []
         L.hz_version.restype = C.c_int
+        L.hz_last_search.restype = C.c_int
+        L.hz_last_search.argtypes = []
         L.hz_release_workspace.restype = C.c_int
         L.hz_release_workspace.argtypes = [C.c_int]
         common = [C.c_int, C.c_int, C.c_int, C.c_int, C.c_double, C.c_double, C.c_int,

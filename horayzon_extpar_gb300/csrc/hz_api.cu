@@ -34,6 +34,7 @@ thread_local std::string g_last_error;
 thread_local long long g_launches = 0;
 // Progress lines of the current call (the reference's std::cout lines).
 thread_local std::string g_log;
+thread_local int g_search = HZ_SEARCH_NONE;  // hz_last_search
 
 void log_line(const char* fmt, ...) {
   char buf[512];
@@ -1166,6 +1167,7 @@ bool use_sweep(const hz_domain* doms, int n, const hz_options& opt) {
 int run_entry(hz_domain* doms, int n, bool on_device, cudaStream_t user_stream,
               const hz_options& opt, hz_stats* stats) {
   auto t0 = std::chrono::steady_clock::now();
+  g_search = HZ_SEARCH_NONE;
   if (n < 1) return fail(HZ_ERR_VALUE, "no domains");
   // The search packs the domain index of a cell in 16 bits.
   if (n > 65535) return fail(HZ_ERR_VALUE, "at most 65535 domains per call");
@@ -1216,7 +1218,8 @@ int run_entry(hz_domain* doms, int n, bool on_device, cudaStream_t user_stream,
   };
   // The profile sweep where it can run; a domain its grid cannot hold (raised
   // on the device before any output is written) runs the tree search instead.
-  bool sweep = use_sweep(doms, n, opt);
+  const bool swept = use_sweep(doms, n, opt);
+  bool sweep = swept;
   std::vector<Buffers> b;
   std::vector<Problem> pr;
   double ms_h2d = 0.0;
@@ -1301,6 +1304,7 @@ int run_entry(hz_domain* doms, int n, bool on_device, cudaStream_t user_stream,
     sweep = false;
   }
   if (rc) return rc;
+  g_search = sweep ? HZ_SEARCH_SWEEP : swept ? HZ_SEARCH_SWEEP_THEN_TREE : HZ_SEARCH_TREE;
   for (int d = 0; d < n; d++) doms[d].latency_ms = out.latency_ms[d];
   const auto t_d2h = std::chrono::steady_clock::now();
   if (!on_device) {
@@ -1371,6 +1375,8 @@ void hz_default_options(hz_options* opt) {
 }
 
 const char* hz_last_error(void) { return g_last_error.c_str(); }
+
+int hz_last_search(void) { return g_search; }
 
 int hz_version(void) { return HZ_VERSION; }
 

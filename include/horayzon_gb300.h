@@ -377,6 +377,17 @@ const char* hz_last_error(void);
 /* HZ_VERSION of the loaded library. */
 int hz_version(void);
 
+enum {
+    HZ_SEARCH_NONE = 0,             /* no horizon search ran to its end */
+    HZ_SEARCH_SWEEP = 1,            /* profile sweep */
+    HZ_SEARCH_TREE = 2,             /* tree search */
+    HZ_SEARCH_SWEEP_THEN_TREE = 3   /* tree search, after the sweep turned the call down */
+};
+
+/* Which search the last horizon call on this thread ran (HZ_SEARCH_*; the results
+ * are the same). hz_horizon_svf_device_static, always the tree's, does not count. */
+int hz_last_search(void);
+
 /* Frees the cached device workspace of `device` (-1 = all devices) and
  * forgets the cached address of hz_horizon_svf_device_static's array there. */
 int hz_release_workspace(int device);

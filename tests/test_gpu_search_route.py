@@ -1,0 +1,103 @@
+"""Which search runs a call: the profile sweep by default, the tree search where
+an option of the tree asks for it, and the tree search after the sweep where its
+grid cannot hold the domain. Results are the same on every route; without these
+tests a sweep that turned every call down would pass the tests that compare it
+with the tree."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from horayzon_extpar_gb300 import _lib, horizon_svf_comp_py, synthetic
+from horayzon_extpar_gb300.horizon_svf import horizon_svf_comp_batch
+
+pytestmark = pytest.mark.gpu
+
+ARGS = (24, 1, 40000.0, 0.2, 1, 2)
+
+
+def _run(inputs, args=ARGS, **kw):
+    h, s, st = horizon_svf_comp_py(*inputs, *args, return_stats=True, **kw)
+    return h, s, st["num_rays"], st["search"]
+
+
+def _same(inputs, search, args=ARGS, **kw):
+    h0, s0, n0, by0 = _run(inputs, args, leaf_size=2, **kw)
+    h1, s1, n1, by1 = _run(inputs, args, **kw)
+    assert by0 == "tree" and by1 == search
+    np.testing.assert_array_equal(h1, h0)
+    np.testing.assert_array_equal(s1, s0)
+    assert n1 == n0
+
+
+@pytest.mark.parametrize("dkw,args,kw", [
+    (dict(edge_km=1.0, box_km=4.0, seed=1), ARGS, {}),
+    (dict(edge_km=0.1, box_km=8.0, seed=3, kind="eroded", hmin=0.0, hmax=3000.0),
+     (37, 1, 8000.0, 0.2, 1, 1), {}),
+    (dict(edge_km=0.1, box_km=5.0, seed=4, kind="eroded", hmin=0.0, hmax=2500.0),
+     (24, 0, 15000.0, 2.0, 2, 2), {"precision": 1}),
+    (dict(edge_km=40.0, box_km=2000.0, seed=5, hmax=6000.0, lat0_deg=70.0),
+     (24, 1, 500000.0, 0.2, 1, 2), {}),
+    (dict(edge_km=2.5, box_km=80.0, seed=8), ARGS, {"elev_floor_deg": 7.3}),
+    (dict(edge_km=0.5, box_km=95.0, seed=10, hmax=3000.0), (45, 1, 6000.0, 0.2, 2, 0),
+     {"cells": (3001, 14003)}),
+])
+def test_defaults_run_the_sweep(dkw, args, kw):
+    _same(synthetic.make_domain(**dkw).inputs(), "sweep", args, **kw)
+
+
+def test_a_batch_runs_the_sweep():
+    doms = [(d.inputs(), a) for d, a in synthetic.make_batch(n_domains=3, seed=3, min_cells=300,
+                                                             max_cells=3000)]
+    assert horizon_svf_comp_batch(doms, return_stats=True)[1]["search"] == "sweep"
+    assert horizon_svf_comp_batch(doms, return_stats=True, leaf_size=2)[1]["search"] == "tree"
+
+
+@pytest.mark.parametrize("kw", [
+    {"kernel": _lib.HZ_KERNEL_PER_CELL}, {"kernel": _lib.HZ_KERNEL_PERSISTENT_BVH2},
+    {"count_work": True}, {"elev_walk": 1}, {"advance_min": 16}, {"leaf_min": 1}, {"leaf_size": 4},
+    {"queue_chunk": 32}, {"bvh_treelets": True}, {"occluder_cache": False}])
+def test_options_of_the_tree_run_the_tree(kw):
+    d = synthetic.make_domain(edge_km=2.5, box_km=30.0, seed=2)
+    assert _run(d.inputs(), **kw)[3] == "tree"
+
+
+def test_a_wide_domain_falls_back():
+    d = synthetic.make_domain(edge_km=2.0, box_km=20.0, seed=13)
+    inputs = [np.array(a) for a in d.inputs()]
+    half = d.ncell // 2
+    inputs[0][half:] += 2.0  # 115 degrees: the mean direction shows it
+    _same(inputs, "sweep, then tree", (12, 1, 20000.0, 0.2, 1, 2))
+    inputs[0][half:] -= 0.7  # 75 degrees: the grid's bounds do
+    _same(inputs, "sweep, then tree", (12, 1, 20000.0, 0.2, 1, 2))
+
+
+def test_lists_beyond_their_capacity_fall_back():
+    """Triangles two to three cells across, twenty layers of them: more entries than
+    twelve per triangle, which the lists have room for."""
+    from scipy.spatial import cKDTree
+    d = synthetic.make_domain(edge_km=1.0, box_km=40.0, seed=21)
+    clon, clat, h, vlon, vlat, cov = (np.array(a) for a in d.inputs())
+    scale = np.cos(vlat.mean())
+    tree = cKDTree(np.stack([clon * scale, clat], 1))
+    ring = 2.6 / 6371.0
+    full = np.nonzero((cov != -2).all(axis=0))[0]
+    for k in range(6):
+        t = np.pi / 3 * k
+        at = np.stack([vlon[full] * scale + ring * np.sin(t), vlat[full] + ring * np.cos(t)], 1)
+        cov[k, full] = tree.query(at)[1]
+    distinct = np.sort(cov[:, full], axis=0)
+    cov[:, full[(distinct[1:] == distinct[:-1]).any(axis=0)]] = -2  # rings cut by the border
+    _same((clon, clat, h, vlon, vlat, cov), "sweep, then tree", (4, 1, 2000.0, 0.2, 1, 2))
+
+
+def test_a_failed_call_reports_no_search():
+    d = synthetic.make_domain(edge_km=2.5, box_km=30.0, seed=2)
+    _run(d.inputs())
+    assert _lib.load().hz_last_search() == 1
+    h = np.empty(4)
+    p = h.ctypes.data_as(C.POINTER(C.c_double))
+    i = np.empty(4, dtype=np.int32).ctypes.data_as(C.POINTER(C.c_int32))
+    assert _lib.load().hz_horizon_svf(p, p, p, p, p, i, p, p, 0, 0, 24, 1, 4e4, 0.2, 1, 2, None,
+                                      None) == _lib.HZ_ERR_VALUE
+    assert _lib.load().hz_last_search() == 0
