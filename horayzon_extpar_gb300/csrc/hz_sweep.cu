@@ -110,6 +110,7 @@ constexpr int kRunStart = -14;            // start of a run's first azimuth (-7 
 constexpr int kCodeAllMiss = -20000;      // no lattice ray meets the terrain
 constexpr int kCodeGap = -20001;          // left to k_sweep_repair
 constexpr int kCodeStop = 10000;          // + ((m + 2000) << 1 | up): the search's stop itself
+constexpr int kMaxStop = (32767 - kCodeStop) / 2 - 2000;  // highest m that 16 bits hold
 
 __device__ __forceinline__ float height_magic(unsigned h16) {
   return __uint_as_float(0x4B000000u | h16);
@@ -515,30 +516,6 @@ __device__ __forceinline__ CellFrame cell_frame64(const DomainDesc& D, int cell)
   return f;
 }
 
-// Ray of azimuth a and lattice elevation m: the direction of search_step.
-template <bool kPrecise>
-__device__ __forceinline__ Ray lattice_ray(const DomainDesc& D, const CellFrame& f, int a, int m,
-                                           double2& ecs) {
-  const double2 cs = __ldg(&D.azim_cs[a]);
-  const double hx = cs.x * f.north.x + cs.y * f.east.x;
-  const double hy = cs.x * f.north.y + cs.y * f.east.y;
-  const double hz = cs.x * f.north.z + cs.y * f.east.z;
-  if (m >= kElevMin && m < kElevMin + kElevTable) {
-    ecs = __ldg(&D.elev_cs[m - kElevMin]);
-  } else {
-    const double e = (double)m * D.two_ha;
-    ecs = make_double2(cos(e), sin(e));
-  }
-  const float dx = (float)(ecs.x * hx + ecs.y * f.normal.x);
-  const float dy = (float)(ecs.x * hy + ecs.y * f.normal.y);
-  const float dz = (float)(ecs.x * hz + ecs.y * f.normal.z);
-  const float ox = (float)f.ox, oy = (float)f.oy, oz = (float)f.oz;
-  if (kPrecise)
-    return make_ray(ox, oy, oz, dx, dy, dz, D.tfar, (float)(f.ox - (double)ox),
-                    (float)(f.oy - (double)oy), (float)(f.oz - (double)oz));
-  return make_ray(ox, oy, oz, dx, dy, dz, D.tfar);
-}
-
 // FP32 frame table by work position, quadruples of one cell together: origin
 // and its height, normal, north and the origin's gnomonic X, east and Y, and
 // (precise) the origin's FP32 residual. Lanes set up azimuths of scattered
@@ -555,12 +532,11 @@ __device__ __forceinline__ float4* cell_rows(const DomainDesc& D, long long p) {
 // The FP64 frame comes from its table: recomputing it (two square roots and
 // six divisions) took more of the FP64 pipe than the whole rest of the sweep.
 template <bool kPrecise>
-__device__ __forceinline__ Ray table_ray(const DomainDesc& D, int p, int a, int m, double2& ecs) {
+__device__ __forceinline__ Ray table_ray(const DomainDesc& D, int p, int a, double2 ecs) {
   const double* fr = D.cell_frame + 9ll * p;
   const float4* f32 = cell_rows<kPrecise>(D, p);
   const float4 o = __ldg(f32), q = kPrecise ? __ldg(f32 + kFrameRest) : o;
   const double2 cs = __ldg(&D.azim_cs[a]);
-  ecs = __ldg(&D.elev_cs[m - kElevMin]);
   const float dx = (float)(ecs.x * (cs.x * fr[3] + cs.y * fr[6]) + ecs.y * fr[0]);
   const float dy = (float)(ecs.x * (cs.x * fr[4] + cs.y * fr[7]) + ecs.y * fr[1]);
   const float dz = (float)(ecs.x * (cs.x * fr[5] + cs.y * fr[8]) + ecs.y * fr[2]);
@@ -569,8 +545,8 @@ __device__ __forceinline__ Ray table_ray(const DomainDesc& D, int p, int a, int 
 }
 template <bool kPrecise>
 __device__ __noinline__ bool exact_hit(const DomainDesc* D, int p, int a, int m, int tri) {
-  double2 ecs;
-  const Ray r = table_ray<kPrecise>(*D, p, a, m, ecs);
+  // Sweeps stay within kTanRange of the horizontal, well inside the table.
+  const Ray r = table_ray<kPrecise>(*D, p, a, __ldg(&D->elev_cs[m - kElevMin]));
   return test_tri<kPrecise>(D->tris, D->tri_lo, r, tri);
 }
 
@@ -1379,6 +1355,15 @@ __device__ bool grid_ray(const DomainDesc& D, const GridDesc& g, const Ray& r, c
   }
 }
 
+// Cosine and sine of lattice elevation m. Under a roof (a mesh folded over
+// itself) every ray of a turn hits, and each azimuth carries the search a turn
+// further, past the table.
+__device__ __forceinline__ double2 elevation(const DomainDesc& D, int m) {
+  if (m >= kElevMin && m < kElevMin + kElevTable) return __ldg(&D.elev_cs[m - kElevMin]);
+  const double e = (double)m * D.two_ha;
+  return make_double2(cos(e), sin(e));
+}
+
 // The first azimuth of every run but a cell's first was swept from kRunStart:
 // where the search can come to it from below that (the azimuth before has no
 // hits from there up, or is open), the cell goes to the repair.
@@ -1496,7 +1481,7 @@ template <bool kPrecise>
 __global__ void __launch_bounds__(128)
     k_sweep_repair(const DomainDesc* __restrict__ doms, int ndom, const int* __restrict__ order,
                    const int* __restrict__ list, const int* __restrict__ list_n,
-                   int* __restrict__ next, int s_full, const int* __restrict__ err) {
+                   int* __restrict__ next, int s_full, int* __restrict__ err) {
   constexpr unsigned kFull = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   if (*err & kErrGrid) return;
@@ -1545,8 +1530,8 @@ __global__ void __launch_bounds__(128)
       const float hy = __fmaf_rn(c, fn.y, e * fe.y);
       const float hz = __fmaf_rn(c, fn.z, e * fe.z);
       auto ray_hits = [&](int mm) {
-        double2 ecs;
-        const Ray r = table_ray<kPrecise>(D, p, a, mm, ecs);
+        const double2 ecs = elevation(D, mm);
+        const Ray r = table_ray<kPrecise>(D, p, a, ecs);
         // Beyond the zenith the ray runs along the opposite azimuth.
         const float sg = ecs.x < 0.0 ? -1.f : 1.f;
         const Track tr = make_track(g, fn.w, fe.w, sg * hx, sg * hy, sg * hz, fu.x,
@@ -1591,6 +1576,10 @@ __global__ void __launch_bounds__(128)
           have = 32;
           below = __ballot_sync(kFull, ray_hits(base - lane));
         }
+      }
+      if (m > kMaxStop) {  // many turns under a roof: the tree search carries on
+        if (lane == 0) atomicOr(err, kErrGrid);
+        break;
       }
       if (lane == 0) *slot = (int16_t)(kCodeStop + (((m + 2000) << 1) | (up ? 1 : 0)));
     }

@@ -158,3 +158,25 @@ def test_gpu_sweep_of_far_rays_in_mid_air(dkw, args, kw):
         out.append((h, s, raw, st["num_rays"]))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
     assert torch.equal(out[0][2], out[1][2]) and out[0][3] == out[1][3]
+
+
+@pytest.mark.parametrize("nh,search", [(4, "sweep"), (24, "sweep, then tree")])
+def test_gpu_sweep_under_a_roof(nh, search):
+    """A basin under a second sheet of cells: every ray of a full turn hits there,
+    and each azimuth starts where the last one ended, a turn of 720 elevations
+    further. The elevations leave the table (four azimuths), and the sweep's
+    16-bit codes (more than thirteen)."""
+    d = synthetic.make_domain(edge_km=0.5, box_km=15.0, seed=17)
+    clon, clat, h, vlon, vlat, cov = (np.array(a) for a in d.inputs())
+    x = (clon - clon.mean()) * np.cos(clat.mean()) * 6371.0
+    y = (clat - clat.mean()) * 6371.0
+    r = np.sqrt(x * x + y * y)
+    ground = 500.0 + 2500.0 * np.minimum(r / 6.0, 1.1) ** 4
+    n = clon.size
+    inputs = (np.concatenate([clon, clon]), np.concatenate([clat, clat]),
+              np.concatenate([ground, np.full(n, 1500.0)]), np.concatenate([vlon, vlon]),
+              np.concatenate([vlat, vlat]),
+              np.ascontiguousarray(np.concatenate([cov, np.where(cov == -2, -2, cov + n)], 1)))
+    st0, st1 = _same(inputs, (nh, 1, 20000.0, 0.2, 1, 2))
+    assert st0["num_rays"] > 700 * nh * np.sum(r < 3.0)  # full turns
+    assert st1["search"] == search
