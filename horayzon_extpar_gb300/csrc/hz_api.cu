@@ -292,6 +292,9 @@ BatchBuffers carve_batch(Carver& c, int n, long long total_cells, const SweepSiz
     b.all.top = c.take<uint16_t>(2 * sweep->cells);
     b.all.low = c.take<uint16_t>(2 * sweep->cells);
     b.all.planes = c.take<uint2>(2 * sweep->cells);
+    b.all.n_tri = sweep->tri;
+    b.all.n_cells = sweep->cells;
+    b.all.n_refs = sweep->refs;
   }
   b.counters = c.take<unsigned long long>(kCounterWords);
   b.done = c.take<unsigned long long>(2 * (size_t)n);
@@ -860,6 +863,7 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
       D.tan_m = b[d].tan_m;
       D.cell_base = b[d].cell_base;
       D.ref_base = b[d].ref_base;
+      D.tri_base = b[d].tri_base;
       if (sweep) {
         // Lists name triangles by their number in the call's array.
         D.tris = bb.all.tris;
@@ -941,7 +945,7 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
   unsigned long long* rb = pin;  // words 0..15 (descriptors live beyond word 64)
   HZ_CUDA(cudaMemcpyAsync(rb + 8, bb.counters, 3 * sizeof(unsigned long long),
                           cudaMemcpyDeviceToHost, s));
-  HZ_CUDA(cudaMemcpyAsync(rb + 12, bb.err, 3 * sizeof(int), cudaMemcpyDeviceToHost, s));
+  HZ_CUDA(cudaMemcpyAsync(rb + 12, bb.err, 4 * sizeof(int), cudaMemcpyDeviceToHost, s));
   HZ_CUDA(cudaMemcpyAsync(rb + 14, bb.t0, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
   unsigned long long* rb_done = pin + 64;  // the totals / error slots are no longer needed
   if (n > 1)
@@ -961,6 +965,9 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
 #endif
   const int* errw = reinterpret_cast<const int*>(rb + 12);  // bit word, check code, index
   const int err1 = errw[0];
+#if defined(HZ_CHECKED) && HZ_CHECKED
+  fprintf(stderr, "hz_checks %x\n", (unsigned)errw[3]);
+#endif
   if (err1 & kErrGrid) return kRetryWithTree;
   if (err1 & kErrStack) return fail(HZ_ERR_INTERNAL, "BVH traversal stack overflow");
   if (err1 & kErrBounds)

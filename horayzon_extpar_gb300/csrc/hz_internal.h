@@ -207,6 +207,7 @@ struct DomainDesc {
   int16_t* codes;
   int cell_base;              // of its cells in gstart (half of it: its pyramid) and of its
   unsigned ref_base;          // list entries, in the call's arrays (SweepAll)
+  int tri_base;               // and of its triangles
   const float* tan_m;         // [kTanTable] tangents of (k - kTanTable / 2) * 0.5 deg
   int runs, run_len, run_extra;
   int tail_begin, tail_runs, tail_run_len, tail_run_extra;
@@ -287,6 +288,7 @@ struct SweepAll {
   uint16_t* top;
   uint16_t* low;
   uint2* planes;
+  long long n_tri, n_cells, n_refs;  // sizes (the pyramids: twice the cells)
 };
 // Cell frames of all domains (after cell_order).
 cudaError_t sweep_frames(const DomainDesc* doms, int ndom, const int32_t* order, int total,

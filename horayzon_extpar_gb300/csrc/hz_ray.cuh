@@ -197,15 +197,22 @@ __device__ __forceinline__ V3 rotate3(V3 v, V3 k, double s, double c) {
 #ifndef HZ_CHECKED
 #define HZ_CHECKED 0  // 1: the search checks its indices and records violations (kErrBounds)
 #endif
-// What a checked build checks: a node reference against the tree's nodes, a
-// leaf's triangle range against its triangles, an output row / cell.
-enum : int { kCheckNode = 1, kCheckLeaf = 2, kCheckOutput = 3 };
+// What a checked build checks. Tree search: a node reference against the tree's
+// nodes, a leaf's triangle range against its triangles; both: an output row / cell.
+// Profile sweep: a triangle's number, a list (its start and its entries), a grid or
+// pyramid cell, a lattice elevation against its table, a slot of the warp's
+// triangle queue, a cell's work position, a result code's slot.
+enum : int { kCheckNode = 1, kCheckLeaf = 2, kCheckOutput = 3, kCheckTriangle = 4, kCheckList = 5,
+             kCheckGrid = 6, kCheckElevation = 7, kCheckQueue = 8, kCheckPosition = 9,
+             kCheckSlot = 10 };
 
 // In checked builds: records the first failed check (code, index) in err[1],
-// err[2] and raises kErrBounds; the caller then skips the access. Without
-// HZ_CHECKED every check passes and compiles away.
+// err[2] and raises kErrBounds; the caller then skips the access. err[3] holds a
+// bit for every kind of check made. Without HZ_CHECKED every check passes and
+// compiles away.
 __device__ __forceinline__ bool check_ok(bool ok, int code, long long index, int* err) {
 #if HZ_CHECKED
+  if (!(*(volatile int*)(err + 3) >> code & 1)) atomicOr(err + 3, 1 << code);
   if (!ok) {
     if (atomicCAS(err + 1, 0, code) == 0) err[2] = (int)index;
     atomicOr(err, kErrBounds);

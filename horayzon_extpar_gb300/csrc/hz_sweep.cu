@@ -286,7 +286,8 @@ __device__ __forceinline__ void for_cells(const GridDesc& g, float4 a, float4 b,
 __global__ void k_grid_count(const float* __restrict__ vert, const float* __restrict__ vert_lo,
                              const int* __restrict__ vot, int n, const float4* __restrict__ gv,
                              GridDesc* __restrict__ gd, uint32_t* __restrict__ count,
-                             Tri* __restrict__ tris, float4* __restrict__ tri_lo) {
+                             long long cap0, Tri* __restrict__ tris, float4* __restrict__ tri_lo,
+                             int* __restrict__ err) {
   __shared__ unsigned smax;
   if (threadIdx.x == 0) smax = 0u;
   __syncthreads();
@@ -314,7 +315,7 @@ __global__ void k_grid_count(const float* __restrict__ vert, const float* __rest
                                 len2(r.x.z - r.x.y, r.y.z - r.y.y, r.z.z - r.z.y)));
     atomicMax(&smax, __float_as_uint(sqrtf(e)));
     for_cells(g, gv[v0], gv[v1], gv[v2], [&](int cell, float, float) {
-      atomicAdd(&count[cell], 1u);
+      if (check_ok(cell >= 0 && cell < cap0, kCheckGrid, cell, err)) atomicAdd(&count[cell], 1u);
     });
   }
   __syncthreads();
@@ -325,14 +326,15 @@ __global__ void k_grid_count(const float* __restrict__ vert, const float* __rest
 // numbered through the domains of a call); count runs down from the cell's number of entries.
 __global__ void k_grid_fill(const int* __restrict__ vot, int n, int tri_base,
                             const float4* __restrict__ gv, const GridDesc* __restrict__ gd, uint32_t* __restrict__ count,
-                            const uint32_t* __restrict__ start, uint2* __restrict__ refs,
-                            long long cap_refs, int* __restrict__ err) {
+                            const uint32_t* __restrict__ start, long long cap0,
+                            uint2* __restrict__ refs, long long cap_refs, int* __restrict__ err) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n || !gd->ok) return;
   const GridDesc& g = *gd;
   bool over = false;
   for_cells(g, gv[vot[3LL * t]], gv[vot[3LL * t + 1]], gv[vot[3LL * t + 2]],
             [&](int cell, float up, float lo) {
+              if (!check_ok(cell >= 0 && cell < cap0, kCheckGrid, cell, err)) return;
               const long long pos = (long long)start[cell] + atomicSub(&count[cell], 1u) - 1;
               if (pos >= cap_refs) {
                 over = true;
@@ -376,13 +378,14 @@ __device__ __forceinline__ bool plane_fits(const GridDesc& g, float gx, float gy
 __global__ void k_grid_heights(const GridDesc* __restrict__ gd, const uint32_t* __restrict__ start,
                                const uint2* __restrict__ refs, long long cap_refs, int tri_base,
                                const int* __restrict__ vot, const float4* __restrict__ gv,
-                               uint16_t* __restrict__ top, uint16_t* __restrict__ low,
-                               uint2* __restrict__ planes) {
+                               long long cap0, uint16_t* __restrict__ top,
+                               uint16_t* __restrict__ low, uint2* __restrict__ planes,
+                               int* __restrict__ err) {
   if (!gd->ok) return;
   const GridDesc& g = *gd;
   const long long n0 = (long long)g.W * g.H;
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n0) return;
+  if (k >= n0 || !check_ok(k < cap0, kCheckGrid, k, err)) return;
   // Cell (i, j) of index k in the brick order.
   const int brick = (int)(k >> 4), wb = g.W >> 2;
   const int i = 4 * (brick % wb) + (int)(k & 3), j = 4 * (brick / wb) + (int)((k >> 2) & 3);
@@ -443,8 +446,9 @@ __global__ void k_grid_heights(const GridDesc* __restrict__ gd, const uint32_t* 
 // Level l of the pyramid from level l - 2: a cell's children are one brick.
 // Plane: gradient from the children's heights, the least height above every
 // child's plane or top within the child.
-__global__ void k_grid_up(const GridDesc* __restrict__ gd, int l, uint16_t* __restrict__ top,
-                          uint16_t* __restrict__ low, uint2* __restrict__ planes) {
+__global__ void k_grid_up(const GridDesc* __restrict__ gd, int l, long long cap0,
+                          uint16_t* __restrict__ top, uint16_t* __restrict__ low,
+                          uint2* __restrict__ planes, int* __restrict__ err) {
   if (!gd->ok || l > gd->L) return;
   const GridDesc& g = *gd;
   const int W = g.W, n2 = 2 * W * g.H;
@@ -453,6 +457,8 @@ __global__ void k_grid_up(const GridDesc* __restrict__ gd, int l, uint16_t* __re
   if (k >= (long long)w * h) return;
   const int b = (int)(k / w), a = (int)(k - (long long)b * w);
   const int from = grid_index(W, n2, 4 * a, 4 * b, l - 2), to = grid_index(W, n2, a, b, l);
+  if (!check_ok(from >= 0 && from + 16 <= 2 * cap0 && to >= 0 && to < 2 * cap0, kCheckGrid, to, err))
+    return;
   const float size = g.c * (float)(1 << (l - 2));  // of a child
   unsigned hi = 0u, lo = 0xFFFFu;
   float n = 0.f, mx = 0.f, my = 0.f, mh = 0.f, xx = 0.f, yy = 0.f, xh = 0.f, yh = 0.f;
@@ -678,7 +684,13 @@ struct SweepScene {
   const uint2* refs;
   const uint32_t* gstart;
   const uint2* planes;
+  long long n_tri, n_cells, n_refs;
 };
+
+// Grid cell at of a thread's domain and the one after it lie in the call's list starts.
+__device__ __forceinline__ bool size_ok(const int4 size, int at, const SweepScene& sc) {
+  return at >= 0 && at < size.x * size.y && size.w + (long long)at + 1 < sc.n_cells;
+}
 
 template <bool kPrecise>
 struct SweepShared {
@@ -764,7 +776,7 @@ __device__ __forceinline__ bool may_hide(const SweepShared<kPrecise>& sh, int o,
 template <bool kPrecise>
 __device__ __forceinline__ int cut_triangle(const SweepShared<kPrecise>& sh, int o,
                                             const SweepScene& sc, const DomainDesc* doms,
-                                            int tri, int& m_new) {
+                                            int tri, int& m_new, int* err) {
   float3 a, b, c;
   const float4 org = sh.v[o][kRowOrigin], side = sh.v[o][kRowSide], ray = sh.v[o][kRowRay],
                along = sh.v[o][kRowAlong];
@@ -779,6 +791,7 @@ __device__ __forceinline__ int cut_triangle(const SweepShared<kPrecise>& sh, int
               reach = tfar * rsqrtf(__fmaf_rn(ta, ta, 1.f));  // the search radius along x
   const float* tm = sh.tan_m + kTanRange;
   const int m = sh.m[o];
+  if (!check_ok(m >= -kTanRange && m <= kMaxM, kCheckElevation, m, err)) return kFlagAbove;
   // Vertices in the plane within rounding: one of them is an end point of the
   // segment whichever side it is taken to be on (the cell's own vertex, under
   // the ray origin, always is); two leave the segment open.
@@ -931,6 +944,7 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
 
   // Slope and plane normal of the ray at lattice elevation m.
   auto set_elevation = [&]() {
+    if (!check_ok(m > -kTanRange && m <= kMaxM + 1, kCheckElevation, m, err)) m = 0;
     ta = sh.tan_m[m + kTanRange];
     const float4 h = sh.v[t][kRowAlong], u = sh.v[t][kRowUp];
     sh.v[t][kRowRay] = make_float4(__fmaf_rn(-ta, h.x, u.x), __fmaf_rn(-ta, h.y, u.y),
@@ -981,7 +995,9 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
           code = kCodeAllMiss;
         }
         if (!again) {
-          D.codes[(long long)a * D.ncell + sh.cell[t]] = (int16_t)code;
+          if (check_ok(a >= 0 && a < D.L && sh.cell[t] >= 0 && sh.cell[t] < D.ncell, kCheckSlot,
+                       (long long)a * D.ncell + sh.cell[t], err))
+            D.codes[(long long)a * D.ncell + sh.cell[t]] = (int16_t)code;
           if (code == kCodeGap) {
             const long long q = D.k_begin + sh.pos[t];
             const unsigned bit = 1u << (q & 31);
@@ -1037,8 +1053,11 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
             const bool tail = local >= whole;
             const unsigned rest = tail ? local - whole : local;
             const unsigned cells = (unsigned)(tail ? D.ncell_traced - D.tail_begin : D.tail_begin);
-            const unsigned run = rest / cells;
-            const int p = (int)(rest - run * cells) + (tail ? D.tail_begin : 0);
+            unsigned run = rest / cells;
+            int p = (int)(rest - run * cells) + (tail ? D.tail_begin : 0);
+            if (!check_ok(p >= 0 && p < D.ncell_traced && run_start(D, p, (int)run + 1) <= D.L,
+                          kCheckPosition, item, err))
+              p = run = 0;
             const float4* fr = cell_rows<kPrecise>(D, p);
             const float4 fo = __ldg(fr + kFrameOrigin), fu = __ldg(fr + kFrameNormal);
             sh.v[t][kRowOrigin] = make_float4(fo.x, fo.y, fo.z, 0.f);
@@ -1132,6 +1151,9 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
       if (st == kLaneWalk) {
         const int a = i >> l, b = j >> l;
         at = grid_index(W, n2, a, b, l);
+        if (!check_ok(at >= 0 && at < n2 && 2 * (long long)size.w + at < 2 * sc.n_cells, kCheckGrid,
+                      at, err))
+          at = 0;
         const uint2 pl = __ldg(planes + at);
         const int bx = (a + 1 - nx) << l, by = (b + 1 - ny) << l;
         const float fx = (float)bx, fy = (float)by;
@@ -1184,6 +1206,9 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
       const float4 hc = sh.v[t][kRowHeight];
       const float xexit = s1 * hc.z * g.x;
       k0 = __float_as_uint(g.w) + k;
+      if (!check_ok(size_ok(sh.size[t], at, sc) && n >= 0 && (long long)k0 + n <= sc.n_refs,
+                    kCheckList, k0, err))
+        n = 0;
       sh.v[t][kRowOrigin].w = kEps * __fmaf_rn(1.1f, xexit, g.z);
       sh.v[t][kRowSide].w = threshold(hc, s, s1) + kMagic;
       sh.v[t][kRowAlong].w = xexit + g.y;
@@ -1206,7 +1231,7 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
       if (lane < count) {
         const int2 e = sh.queue[wid][lane];
         int m_new = 0;
-        const int r = cut_triangle<kPrecise>(sh, e.x, sc, doms, e.y, m_new);
+        const int r = cut_triangle<kPrecise>(sh, e.x, sc, doms, e.y, m_new, err);
         if (r == kFlagAbove) atomicOr(&sh.flags[e.x], kFlagAbove);
         else if (r != 0) {
           atomicMax(&sh.m_new[e.x], m_new);
@@ -1230,13 +1255,15 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
         o = e.x;
         const uint2 rf = __ldg(sc.refs + (unsigned)(e.y + x));
         const float4 side = sh.v[o][kRowSide];
-        if (height_magic(rf.y & 0xFFFFu) >= side.w) {
+        if (height_magic(rf.y & 0xFFFFu) >= side.w &&
+            check_ok((int)rf.x >= 0 && (int)rf.x < sc.n_tri, kCheckTriangle, (int)rf.x, err)) {
           tri = (int)rf.x;
           want = may_hide<kPrecise>(sh, o, side, sc, tri);
         }
       }
       const unsigned wants = __ballot_sync(kFull, want);
-      if (want) sh.queue[wid][queued + __popc(wants & below_me)] = make_int2(o, tri);
+      if (want && check_ok(queued + __popc(wants & below_me) < 64, kCheckQueue, queued, err))
+        sh.queue[wid][queued + __popc(wants & below_me)] = make_int2(o, tri);
       queued += __popc(wants);
       __syncwarp();
       if (queued >= 32) {
@@ -1289,7 +1316,7 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
 // Any-hit query of one lattice ray on the grid.
 template <bool kPrecise>
 __device__ bool grid_ray(const DomainDesc& D, const GridDesc& g, const Ray& r, const Track& tr,
-                         float ho, float slope) {
+                         float ho, float slope, int* err) {
   const int W = g.W, H = g.H, n2 = 2 * W * H;
   const float kl = tr.xlo * g.cmin / g.rlo, kh = tr.xhi * g.cmax / g.rlo;
   const float cl = (ho - g.hpad - g.hlo) * g.iq, ch = __fmaf_rn(ho + g.hpad - g.hlo, g.iq, 2.f);
@@ -1302,6 +1329,7 @@ __device__ bool grid_ray(const DomainDesc& D, const GridDesc& g, const Ray& r, c
   for (;;) {
     const int a = i >> l, b = j >> l;
     const int at = grid_index(W, n2, a, b, l);
+    if (!check_ok(at >= 0 && at < n2, kCheckGrid, at, err)) return false;
     const uint2 pl = __ldg(D.planes + at);
     const unsigned lo = __ldg(D.low + at);
     const bool sx = tr.dx > 0.f, sy = tr.dy > 0.f;
@@ -1332,7 +1360,10 @@ __device__ bool grid_ray(const DomainDesc& D, const GridDesc& g, const Ray& r, c
       for (unsigned k = D.gstart[at]; k < e; k++) {
         const uint2 rf = __ldg(D.refs + k);
         if ((float)(rf.y & 0xFFFFu) < tlo || (float)(rf.y >> 16) > thi) continue;
-        if (test_tri<kPrecise>(D.tris, D.tri_lo, r, (int)rf.x)) return true;
+        if (check_ok((int)rf.x >= D.tri_base && (int)rf.x < D.tri_base + D.n_tri, kCheckTriangle,
+                     (int)rf.x, err) &&
+            test_tri<kPrecise>(D.tris, D.tri_lo, r, (int)rf.x))
+          return true;
       }
       tested = true;
       continue;
@@ -1496,6 +1527,9 @@ __global__ void __launch_bounds__(128)
     const GridDesc& g = *D.grid;
     const int cell = (int)(gid - D.cell_offset);
     const int p = list[w] - (int)D.k_begin;
+    if (!check_ok(p >= 0 && p < D.ncell_traced && cell >= 0 && cell < D.ncell, kCheckPosition,
+                  list[w], err))
+      continue;
     const long long nc = D.ncell;
     const float4* fr = cell_rows<kPrecise>(D, p);
     const float4 fu = __ldg(fr + kFrameNormal), fn = __ldg(fr + kFrameNorth),
@@ -1537,7 +1571,7 @@ __global__ void __launch_bounds__(128)
         const Track tr = make_track(g, fn.w, fe.w, sg * hx, sg * hy, sg * hz, fu.x,
                                     fu.y, fu.z);
         const float c = fmaxf(fabsf((float)ecs.x), 1e-7f);
-        return grid_ray<kPrecise>(D, g, r, tr, ho, __fdiv_rn((float)ecs.y, c));
+        return grid_ray<kPrecise>(D, g, r, tr, ho, __fdiv_rn((float)ecs.y, c), err);
       };
       // Lanes 0-15: m .. m + 15; lanes 16-31: m - 1 .. m - 16.
       unsigned hits = __ballot_sync(kFull, ray_hits(lane < 16 ? m + lane : m - (lane - 15)));
@@ -1599,7 +1633,7 @@ __global__ void __launch_bounds__(128)
 // loop over them is not unrolled: eight times over it ran out of the
 // instruction cache.
 template <bool kRefine1>
-__device__ __forceinline__ unsigned finish_sweep(const DomainDesc& D, int cell) {
+__device__ __forceinline__ unsigned finish_sweep(const DomainDesc& D, int cell, int* err) {
   const long long nc = D.ncell;
   const float inv_ha = (float)(1.0 / D.hori_acc);
   const double ha = D.hori_acc, refine = (double)D.refine;
@@ -1628,12 +1662,14 @@ __device__ __forceinline__ unsigned finish_sweep(const DomainDesc& D, int cell) 
       if (h < 0.0) h = 0.0;
       if (kRefine1) {
         svf = svf + finish_svf_term(D, h, inv_ha);
-        D.horizon[(long long)a * nc + cell] = __dmul_rn(div_pi_rn(h), 180.0);
+        if (check_ok(cell >= 0 && cell < nc && a < D.nhori, kCheckOutput, a * nc + cell, err))
+          D.horizon[(long long)a * nc + cell] = __dmul_rn(div_pi_rn(h), 180.0);
       } else {
         part = part + lattice_svf_term(D, h, j);
         sector = sector + h;
         if (++in_sector == D.refine) {
-          D.horizon[(long long)row * nc + cell] = __dmul_rn(div_pi_rn(sector), 180.0) / refine;
+          if (check_ok(cell >= 0 && cell < nc && row < D.nhori, kCheckOutput, row * nc + cell, err))
+            D.horizon[(long long)row * nc + cell] = __dmul_rn(div_pi_rn(sector), 180.0) / refine;
           sector = 0.0;
           in_sector = 0;
           row++;
@@ -1652,7 +1688,7 @@ __device__ __forceinline__ unsigned finish_sweep(const DomainDesc& D, int cell) 
 
 __global__ void k_sweep_finish(const DomainDesc* __restrict__ doms, int ndom, int total,
                                unsigned long long* __restrict__ counters,
-                               const int* __restrict__ err) {
+                               int* __restrict__ err) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long rays = 0;
   if (k < total && !(*err & kErrGrid)) {
@@ -1664,7 +1700,7 @@ __global__ void k_sweep_finish(const DomainDesc* __restrict__ doms, int ndom, in
     }
     const DomainDesc& D = doms[lo];
     const int cell = D.cell_begin + (int)(k - D.k_begin);
-    rays = D.refine == 1 ? finish_sweep<true>(D, cell) : finish_sweep<false>(D, cell);
+    rays = D.refine == 1 ? finish_sweep<true>(D, cell, err) : finish_sweep<false>(D, cell, err);
   }
   rays = warp_sum_u64(rays);
   if ((threadIdx.x & 31) == 0 && rays) atomicAdd(&counters[0], rays);
@@ -1688,22 +1724,23 @@ cudaError_t sweep_grid(const float* vert32, const float* vert_lo, const int* vot
   note_launches(3);
   if (n_tri > 0) {
     k_grid_count<<<grid_for(n_tri, 256), 256, 0, s>>>(vert32, vert_lo, vot, n_tri, b.gv, b.grid,
-                                                      b.count, tris, vert_lo ? tri_lo : nullptr);
+                                                      b.count, cap0, tris, vert_lo ? tri_lo : nullptr, err);
     note_launches(1);
   }
   e = scan_exclusive_u32(b.count, b.start, cap0 + 1, b.total, b.partials, s);
   if (e != cudaSuccess) return e;
   if (n_tri > 0) {
     k_grid_fill<<<grid_for(n_tri, 256), 256, 0, s>>>(vot, n_tri, tri_base, b.gv, b.grid, b.count, b.start,
-                                                     b.refs, sweep_refs_cap(n_tri), err);
+                                                     cap0, b.refs, sweep_refs_cap(n_tri), err);
     note_launches(1);
   }
   k_grid_heights<<<grid_for(cap0, 256), 256, 0, s>>>(b.grid, b.start, b.refs,
-                                                     sweep_refs_cap(n_tri), tri_base, vot, b.gv, b.top,
-                                                     b.low, b.planes);
+                                                     sweep_refs_cap(n_tri), tri_base, vot, b.gv, cap0,
+                                                     b.top, b.low, b.planes, err);
   note_launches(1);
   for (int l = 2; l <= 8; l += 2) {
-    k_grid_up<<<grid_for(cap0 >> (2 * l), 128), 128, 0, s>>>(b.grid, l, b.top, b.low, b.planes);
+    k_grid_up<<<grid_for(cap0 >> (2 * l), 128), 128, 0, s>>>(b.grid, l, cap0, b.top, b.low,
+                                                             b.planes, err);
     note_launches(1);
   }
   return cudaGetLastError();
@@ -1772,7 +1809,8 @@ cudaError_t sweep_search(const DomainDesc* doms, int ndom, const int32_t* order,
   if (e == cudaSuccess)
     e = cudaMemsetAsync(listed, 0, sizeof(unsigned) * ((size_t)total / 32 + 1), s);
   if (e != cudaSuccess) return e;
-  const SweepScene sc{all.tris, all.tri_lo, all.refs, all.start, all.planes};
+  const SweepScene sc{all.tris,   all.tri_lo, all.refs,    all.start,
+                      all.planes, all.n_tri,  all.n_cells, all.n_refs};
   e = precise ? launch_search<true>(doms, ndom, order, total, total_items, s_full, work, list,
                                     listed, sc, err, s)
               : launch_search<false>(doms, ndom, order, total, total_items, s_full, work, list,
