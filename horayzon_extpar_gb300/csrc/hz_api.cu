@@ -686,8 +686,8 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
     for (int d = 0; d < n; d++) {
       if (sweep) {
         HZ_CUDA(sweep_grid(b[d].vert32, b[d].vert_lo, b[d].vot, out->n_tri[d], out->n_mv[d],
-                           b[d].tri_base, (float)pr[d].dist_search, b[d].sweep, b[d].tris,
-                           b[d].tri_lo, bb.err, fk.on(d)));
+                           b[d].tri_base, (float)pr[d].dist_search, (float)pr[d].ray_org_elev,
+                           b[d].sweep, b[d].tris, b[d].tri_lo, bb.err, fk.on(d)));
         if (b[d].rz)  // the learned start's raster is laid over these bounds
           HZ_CUDA(bvh_tri_bounds(b[d].vert32, b[d].vot, out->n_tri[d], b[d].bvh, fk.on(d)));
         continue;

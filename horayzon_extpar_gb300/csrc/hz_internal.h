@@ -152,7 +152,7 @@ struct GridDesc {
   float rlo, rhi, irlo;       // radii of the lowest and highest vertex, 1 / rlo
   float tau_max;              // tangent of the search radius' angle at the centre
   float cmin, cmax;           // bounds of the curvature term's factor
-  float dadd;                 // bound of a triangle's distance beyond the walk's
+  float dadd;                 // bound of a triangle's distance beyond the walk's and its edge's
   int W, H, L;                // cells; highest pyramid level
   unsigned lmax;              // longest edge (float bits)
   int ok;                     // 0: the grid cannot hold the domain (kErrGrid)
@@ -277,8 +277,8 @@ struct SweepBuffers {
 // Grid, lists and height pyramid of a domain, and its triangle records (mesh
 // order). Raises kErrGrid where the grid cannot hold the domain.
 cudaError_t sweep_grid(const float* vert32, const float* vert_lo, const int* vot, int n_tri,
-                       int n_vert, int tri_base, float tfar, const SweepBuffers& b, Tri* tris,
-                       float4* tri_lo, int* err, cudaStream_t s);
+                       int n_vert, int tri_base, float tfar, float org_elev, const SweepBuffers& b,
+                       Tri* tris, float4* tri_lo, int* err, cudaStream_t s);
 // The arrays of all domains of a call.
 struct SweepAll {
   Tri* tris;

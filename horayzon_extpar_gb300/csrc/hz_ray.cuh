@@ -201,10 +201,11 @@ __device__ __forceinline__ V3 rotate3(V3 v, V3 k, double s, double c) {
 // nodes, a leaf's triangle range against its triangles; both: an output row / cell.
 // Profile sweep: a triangle's number, a list (its start and its entries), a grid or
 // pyramid cell, a lattice elevation against its table, a slot of the warp's
-// triangle queue, a cell's work position, a result code's slot.
+// triangle queue, a cell's work position, a result code's slot; and that the error
+// bound of a cell's triangles covers each of their vertices.
 enum : int { kCheckNode = 1, kCheckLeaf = 2, kCheckOutput = 3, kCheckTriangle = 4, kCheckList = 5,
              kCheckGrid = 6, kCheckElevation = 7, kCheckQueue = 8, kCheckPosition = 9,
-             kCheckSlot = 10 };
+             kCheckSlot = 10, kCheckBound = 11 };
 
 // In checked builds: records the first failed check (code, index) in err[1],
 // err[2] and raises kErrBounds; the caller then skips the access. err[3] holds a

@@ -94,6 +94,11 @@ constexpr float kRf = 6371229.0f;         // kEarthRadius, exact in FP32
 // sweep's own (axes 5 u a component, coordinates u, sums 3 u) and 7 u of the
 // watertight test (sheared coordinates 6 u, direction 1 u).
 constexpr float kEps = 1.28e-6f;
+// The same over a bound of the distance: the 1-norm is up to sqrt(3) times the
+// length in the domain's axes. A vertex of a triangle in a cell that the walk
+// leaves at the horizontal distance x lies within (1 + tan(psi / 2)) x <= 1.04 x
+// (the axes turn by psi <= 0.08) and GridDesc::dadd + the longest edge.
+constexpr float kEpsCell = 1.7321f * kEps, kDropCell = 1.04f;
 constexpr float kMagic = 8388608.0f;      // 2^23: float(2^23 | n) = 2^23 + n
 constexpr int kTanRange = 180;            // lattice elevations with a tangent: |m| < 180
 constexpr int kMaxM = 177;                // sweeps stop below 89 deg
@@ -158,7 +163,7 @@ __global__ void k_grid_init(unsigned* b) {
 
 // Grid geometry: cells of HZ_CELL_TRIS times the mean triangle area.
 __global__ void k_grid_setup(const unsigned* __restrict__ b, int n_tri, long long cap0, float tfar,
-                             GridDesc* __restrict__ g, int* __restrict__ err) {
+                             float org_elev, GridDesc* __restrict__ g, int* __restrict__ err) {
   GridDesc q;
   const float x0 = ord2f(b[0]), y0 = ord2f(b[1]), h0 = ord2f(b[2]), z0 = ord2f(b[3]);
   const float x1 = ord2f(b[4]), y1 = ord2f(b[5]), h1 = ord2f(b[6]);
@@ -193,7 +198,7 @@ __global__ void k_grid_setup(const unsigned* __restrict__ b, int n_tri, long lon
   q.iq = 65000.f / (h1 - h0 + 1.f);
   q.unit = (h1 - h0 + 1.f) / 65000.f;
   q.hpad = 0.05f + 2e-6f * tfar;
-  q.dadd = 2.f * c + 4.f * pad + (h1 - h0) + 1.f;
+  q.dadd = 2.f * c + 4.f * pad + (h1 - h0) + org_elev + 1.f;
   q.rlo = kRf + h0;
   q.rhi = kRf + h1;
   q.irlo = 1.f / q.rlo;
@@ -746,10 +751,14 @@ __device__ __forceinline__ float dot3f(const float3 a, const float4 b) {
 // h1 |q0|) / (|q0| + |q1|).
 template <bool kPrecise>
 __device__ __forceinline__ bool may_hide(const SweepShared<kPrecise>& sh, int o,
-                                         const float4 side, const SweepScene& sc, int tri) {
+                                         const float4 side, const SweepScene& sc, int tri,
+                                         int* err) {
   float3 a, b, c;
   const float4 org = sh.v[o][kRowOrigin];
   load_relative(sh, o, org, sc, tri, a, b, c);
+  const auto norm1 = [](float3 v) { return fabsf(v.x) + fabsf(v.y) + fabsf(v.z); };
+  if (!check_ok(org.w >= kEps * fmaxf(norm1(a), fmaxf(norm1(b), norm1(c))), kCheckBound, tri, err))
+    return true;
   const float q0 = dot3f(a, side), q1 = dot3f(b, side), q2 = dot3f(c, side);
   const float mu = org.w;
   if (fminf(q0, fminf(q1, q2)) > mu || fmaxf(q0, fmaxf(q1, q2)) < -mu) return false;
@@ -1209,7 +1218,7 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
       if (!check_ok(size_ok(sh.size[t], at, sc) && n >= 0 && (long long)k0 + n <= sc.n_refs,
                     kCheckList, k0, err))
         n = 0;
-      sh.v[t][kRowOrigin].w = kEps * __fmaf_rn(1.1f, xexit, g.z);
+      sh.v[t][kRowOrigin].w = kEpsCell * __fmaf_rn(kDropCell, xexit, g.z);
       sh.v[t][kRowSide].w = threshold(hc, s, s1) + kMagic;
       sh.v[t][kRowAlong].w = xexit + g.y;
       sh.m_new[t] = m;
@@ -1258,7 +1267,7 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
         if (height_magic(rf.y & 0xFFFFu) >= side.w &&
             check_ok((int)rf.x >= 0 && (int)rf.x < sc.n_tri, kCheckTriangle, (int)rf.x, err)) {
           tri = (int)rf.x;
-          want = may_hide<kPrecise>(sh, o, side, sc, tri);
+          want = may_hide<kPrecise>(sh, o, side, sc, tri, err);
         }
       }
       const unsigned wants = __ballot_sync(kFull, want);
@@ -1713,14 +1722,14 @@ long long sweep_refs_cap(long long n_tri) { return 12 * n_tri + 4096; }
 size_t sweep_frame_floats(bool precise) { return precise ? 20 : 16; }
 
 cudaError_t sweep_grid(const float* vert32, const float* vert_lo, const int* vot, int n_tri,
-                       int n_vert, int tri_base, float tfar, const SweepBuffers& b, Tri* tris,
-                       float4* tri_lo, int* err, cudaStream_t s) {
+                       int n_vert, int tri_base, float tfar, float org_elev, const SweepBuffers& b,
+                       Tri* tris, float4* tri_lo, int* err, cudaStream_t s) {
   const long long cap0 = sweep_cells_cap(n_tri);
   cudaError_t e = cudaMemsetAsync(b.count, 0, sizeof(uint32_t) * (size_t)(cap0 + 1), s);
   if (e != cudaSuccess) return e;
   k_grid_init<<<1, 1, 0, s>>>(b.bounds);
   k_gnomonic<<<grid_for(n_vert, 256), 256, 0, s>>>(vert32, n_vert, b.gv, b.bounds);
-  k_grid_setup<<<1, 1, 0, s>>>(b.bounds, n_tri, cap0, tfar, b.grid, err);
+  k_grid_setup<<<1, 1, 0, s>>>(b.bounds, n_tri, cap0, tfar, org_elev, b.grid, err);
   note_launches(3);
   if (n_tri > 0) {
     k_grid_count<<<grid_for(n_tri, 256), 256, 0, s>>>(vert32, vert_lo, vot, n_tri, b.gv, b.grid,

@@ -1,9 +1,9 @@
 """The checked build (-DHZ_CHECKED=1) on the profile sweep: its triangles, lists,
-grid cells, elevations, queue slots, work positions and result slots are checked
-on the device, and parity cases run clean through it: runs of several azimuths,
-holes in the mesh (repair by rays), refined azimuths, the local-precision mode,
-given starts, a batch. The tree search's own checks run on the precise frame and
-a batch too, which name a tree option for it."""
+grid cells, elevations, queue slots, work positions, result slots and error bounds
+are checked on the device, and parity cases run clean through it: runs of several
+azimuths, holes in the mesh (repair by rays), refined azimuths, the local-precision
+mode, given starts, a batch. The tree search's own checks run on the precise frame
+and a batch too, which name a tree option for it."""
 import os
 import re
 import subprocess
@@ -45,6 +45,14 @@ SCRIPT = textwrap.dedent("""
     same("holes", (clon, clat, h, vlon, vlat, cov), (24, 0, 20000.0, 0.2, 3, 0))
     d = synthetic.make_domain(edge_km=0.2, box_km=8.0, seed=15, kind="eroded", hmax=3000.0)
     same("precise", d.inputs(), (60, 1, 8000.0, 0.2, 1, 2), precision=1)
+    # Rays far along the diagonals of the domain's axes, and origins far above flat
+    # terrain: where a bound by horizontal distance alone falls short.
+    d = synthetic.make_domain(edge_km=10.0, box_km=1200.0, seed=16, hmax=9000.0)
+    same("far", d.inputs(), (8, 1, 500000.0, 0.2, 1, 2))
+    d = synthetic.make_domain(edge_km=0.5, box_km=20.0, seed=7, hmin=100.0, hmax=100.0,
+                              n_features=0)
+    same("above", d.inputs(), (8, 1, 40000.0, 2000.0, 1, 2))
+    d = synthetic.make_domain(edge_km=0.2, box_km=8.0, seed=15, kind="eroded", hmax=3000.0)
     step("starts sweep")
     t = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in d.inputs()]
     g = torch.Generator().manual_seed(5)
@@ -63,9 +71,9 @@ SCRIPT = textwrap.dedent("""
 """)
 
 # Bits of hz_ray.cuh's kCheck*.
-NODE, LEAF, OUTPUT, TRIANGLE, LIST, GRID, ELEVATION, QUEUE, POSITION, SLOT = (
-    1 << k for k in range(1, 11))
-SWEEP = TRIANGLE | LIST | GRID | ELEVATION | QUEUE | POSITION | SLOT | OUTPUT
+NODE, LEAF, OUTPUT, TRIANGLE, LIST, GRID, ELEVATION, QUEUE, POSITION, SLOT, BOUND = (
+    1 << k for k in range(1, 12))
+SWEEP = BOUND | TRIANGLE | LIST | GRID | ELEVATION | QUEUE | POSITION | SLOT | OUTPUT
 
 
 def test_gpu_checked_build_checks_the_sweep(tmp_path):
@@ -82,7 +90,7 @@ def test_gpu_checked_build_checks_the_sweep(tmp_path):
     for part in r.stderr.split("case ")[1:]:
         made[part.split("\n", 1)[0]] = [int(m, 16) for m in
                                         re.findall(r"^hz_checks ([0-9a-f]+)$", part, re.M)]
-    assert len(made) == 12 and made.pop("end") == []
+    assert len(made) == 16 and made.pop("end") == []
     for name, masks in made.items():
         want = SWEEP if name.endswith("sweep") else NODE | LEAF
         assert masks and all(m & want == want for m in masks), (name, masks)
