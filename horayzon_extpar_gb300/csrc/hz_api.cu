@@ -400,9 +400,11 @@ struct Engine {
   int reserve(size_t bytes, cudaStream_t s) {
     if (bytes <= cap) return HZ_OK;
     // Failure injection for tests of the error path (no GPU fault involved):
-    // HZ_INJECT_ALLOC_FAILURE=1 makes every growth of the workspace fail.
+    // HZ_INJECT_ALLOC_FAILURE=N makes a growth of the workspace beyond N bytes fail (1: every
+    // growth).
     const char* inject = getenv("HZ_INJECT_ALLOC_FAILURE");
-    if (inject && inject[0] == '1')
+    const long long limit = inject ? atoll(inject) : 0;
+    if (limit > 0 && bytes > (size_t)limit)
       return fail(HZ_ERR_CUDA, "cudaMalloc of %zu bytes failed: injected failure", bytes);
     HZ_CUDA(cudaStreamSynchronize(s));
     if (arena) HZ_CUDA(cudaFree(arena));
@@ -1242,7 +1244,15 @@ int run_entry(hz_domain* doms, int n, bool on_device, cudaStream_t user_stream,
     if (sweep)
       for (int d = 0; d < n; d++) add_domain(sizes, doms[d].num_vertex, doms[d].grid_type);
     carve_batch(dry, n, total_cells, sweep ? &sizes : nullptr, precise);
+    const std::string message = g_last_error;
     rc = E->reserve(dry.off, s);
+    if (rc && sweep) {
+      // The sweep's result codes grow with the azimuths, the tree does not: a call
+      // that fits with the tree alone still runs.
+      g_last_error = message;
+      sweep = false;
+      continue;
+    }
     if (rc) return rc;
     Carver c(E->arena);
     b.assign(n, Buffers());
