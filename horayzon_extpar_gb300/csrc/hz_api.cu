@@ -1147,13 +1147,24 @@ int azimuth_groups(const hz_domain* doms, int n, const hz_options& opt, int* gro
 }
 
 // Whether a call runs the profile sweep (hz_sweep.cu) rather than the tree
-// search: wherever both can run it is the faster one, from 500 cells (1.9
-// against 5.3 ms) to 3.1M (102 against 136 ms), at every spacing and azimuth
-// count measured, with the same results. The tree search keeps what belongs to it: its own kernels and knobs,
-// work counters (they count its visits), the bisected walk (a ray sequence of
-// its own); and searches whose floor lies below 88 deg or whose result codes (2
-// bytes per cell and azimuth) would not fit beside the outputs.
+// search; the results are the same. From origins near the ground it is the faster
+// one at every spacing and azimuth count measured, from 500 cells (0.63 against 5.2 ms)
+// to 3.1M (63 against 132 ms). The tree search keeps what belongs to it: its own
+// kernels and knobs, work counters (they count its visits), the bisected walk (a ray
+// sequence of its own); searches whose floor lies below 88 deg or whose result codes
+// (2 bytes per cell and azimuth) would not fit beside the outputs; and high origins.
 constexpr long long kMaxCodeBytes = 16ll << 30;
+
+// From an origin high over the terrain the rays around the horizon end in mid-air,
+// with terrain below and beyond: azimuth after azimuth goes to the sweep's repair, a
+// warp per cell. Times of the tree over those of the sweep (radii of 1 to 500 km, spacings of 0.2
+// to 10 km, 24 azimuths), by origin height over search radius: 11,000 to 480,000 cells 1.1
+// to 5.0 at 0.02, 0.97 to 4.8 at 0.03, 0.1 to 2.3 at 0.1, 0.05 to 2.2 at 0.3; at 500 km the
+// line lies at 5 km instead (1.3 to 7 there, 0.8 to 6 at 10 km). Up to 4,000 cells, where the
+// tree search waits for its slowest cells, 1.1 to 7.7 up to 0.1 at radii to 40 km, and
+// 0.8 to 1.5 beyond it from origins above 5 km.
+constexpr double kHighOrigin = 0.03, kHighMetres = 5000.0, kHighSmall = 0.1;
+constexpr long long kSmallCells = 8192;
 
 bool use_sweep(const hz_domain* doms, int n, const hz_options& opt) {
   if (opt.kernel != HZ_KERNEL_PERSISTENT || opt.count_work ||
@@ -1161,12 +1172,18 @@ bool use_sweep(const hz_domain* doms, int n, const hz_options& opt) {
       opt.queue_chunk || opt.bvh_treelets || !opt.occluder_cache)
     return false;
   if (!(opt.elev_floor_deg >= -88.0 && opt.elev_floor_deg <= 88.0)) return false;
-  long long bytes = 0;
+  long long bytes = 0, high = 0;
+  bool very_high = false;
   SweepSizes all;
   for (int d = 0; d < n; d++) {
+    const double el = doms[d].ray_org_elev, dist = doms[d].dist_search;
+    if (el > kHighMetres || el > kHighOrigin * dist)
+      high += n == 1 && opt.cell_count > 0 ? opt.cell_count : doms[d].num_cell;
+    very_high |= el > kHighMetres && el > kHighSmall * dist;
     bytes += 2ll * doms[d].num_cell * doms[d].num_hori * doms[d].refine_factor;
     add_domain(all, doms[d].num_vertex, doms[d].grid_type);
   }
+  if (very_high || high > kSmallCells) return false;
   // 32-bit indices into the call's arrays.
   return bytes <= kMaxCodeBytes && all.tri < INT32_MAX && 2 * all.cells < INT32_MAX &&
          all.refs < UINT32_MAX;

@@ -101,3 +101,30 @@ def test_a_failed_call_reports_no_search():
     assert _lib.load().hz_horizon_svf(p, p, p, p, p, i, p, p, 0, 0, 24, 1, 4e4, 0.2, 1, 2, None,
                                       None) == _lib.HZ_ERR_VALUE
     assert _lib.load().hz_last_search() == 0
+
+
+@pytest.mark.parametrize("dkw,dist,elev,search", [
+    # 11,000 cells and more: up to 0.03 of the search radius, and to 5 km
+    (dict(edge_km=1.0, box_km=75.0, seed=31), 20000.0, 600.0, "sweep"),
+    (dict(edge_km=1.0, box_km=75.0, seed=31), 20000.0, 601.0, "tree"),
+    (dict(edge_km=10.0, box_km=750.0, seed=32), 400000.0, 5000.0, "sweep"),
+    (dict(edge_km=10.0, box_km=750.0, seed=32), 400000.0, 5001.0, "tree"),
+    (dict(edge_km=2.5, box_km=180.0, seed=34), 1000.0, 500.0, "tree"),
+    # a few cells: beyond a tenth of the radius from above 5 km only
+    (dict(edge_km=1.0, box_km=40.0, seed=33), 20000.0, 5000.0, "sweep"),
+    (dict(edge_km=1.0, box_km=40.0, seed=33), 49000.0, 5001.0, "tree"),
+    (dict(edge_km=1.0, box_km=40.0, seed=33), 60000.0, 5500.0, "sweep"),
+])
+def test_high_origins_run_the_tree(dkw, dist, elev, search):
+    """Where the tree search is the faster one (many times at a tenth of the radius
+    and 400,000 cells). With few cells traced the sweep runs again."""
+    d = synthetic.make_domain(**dkw)
+    args = (4, 1, dist, elev, 1, 2)
+    h0, s0, n0, by = _run(d.inputs(), args)
+    assert by == search
+    h1, s1, n1, by = _run(d.inputs(), args, **({} if by == "tree" else {"leaf_size": 2}))
+    assert by == "tree" and n1 == n0
+    np.testing.assert_array_equal(h1, h0)
+    np.testing.assert_array_equal(s1, s0)
+    if elev < 5000.0:
+        assert _run(d.inputs(), args, cells=(500, 3000))[3] == "sweep"
