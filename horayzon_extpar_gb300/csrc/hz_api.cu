@@ -299,7 +299,7 @@ BatchBuffers carve_batch(Carver& c, int n, long long total_cells, const SweepSiz
   b.counters = c.take<unsigned long long>(kCounterWords);
   b.done = c.take<unsigned long long>(2 * (size_t)n);
   b.t0 = c.take<unsigned long long>(2);
-  b.err = c.take<int>(4);
+  b.err = c.take<int>(8);
   return b;
 }
 
@@ -569,7 +569,7 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
   if (rc) return rc;
   unsigned long long* pin = E.pinned;
   for (int d = 0; d < n; d++) HZ_CUDA(cudaMemsetAsync(b[d].err, 0, 4 * sizeof(int), s));
-  HZ_CUDA(cudaMemsetAsync(bb.err, 0, 4 * sizeof(int), s));
+  HZ_CUDA(cudaMemsetAsync(bb.err, 0, 8 * sizeof(int), s));
   HZ_CUDA(cudaMemsetAsync(bb.counters, 0, kCounterWords * sizeof(unsigned long long), s));
 #ifdef HZ_DIAG
   HZ_CUDA(cudaMemsetAsync(bb.counters + 12, 0xFF, 2 * sizeof(unsigned long long), s));
@@ -687,8 +687,15 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
     HZ_CUDA(fk.begin());
     for (int d = 0; d < n; d++) {
       if (sweep) {
+        // A vertex inside a closed mesh of ncell cells has six (four) of its three (two)
+        // triangles per cell.
+        const Problem& P = pr[d];
+        const double vertices =
+            (double)std::max(0ll, (P.grid_type ? 3ll : 2ll) * P.ncell - out->n_tri[d]) /
+            (P.grid_type ? 6.0 : 4.0);
         HZ_CUDA(sweep_grid(b[d].vert32, b[d].vert_lo, b[d].vot, out->n_tri[d], out->n_mv[d],
-                           b[d].tri_base, (float)pr[d].dist_search, (float)pr[d].ray_org_elev,
+                           b[d].tri_base, (float)P.dist_search, (float)P.ray_org_elev,
+                           (float)P.cell_count, (float)(vertices * P.cell_count / P.ncell), n,
                            b[d].sweep, b[d].tris, b[d].tri_lo, bb.err, fk.on(d)));
         if (b[d].rz)  // the learned start's raster is laid over these bounds
           HZ_CUDA(bvh_tri_bounds(b[d].vert32, b[d].vot, out->n_tri[d], b[d].bvh, fk.on(d)));

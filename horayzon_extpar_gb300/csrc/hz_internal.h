@@ -275,10 +275,12 @@ struct SweepBuffers {
   uint2* refs;           // refs cap
 };
 // Grid, lists and height pyramid of a domain, and its triangle records (mesh
-// order). Raises kErrGrid where the grid cannot hold the domain.
+// order). Raises kErrGrid where the grid cannot hold the domain, or the call's ndom
+// domains have too many vertices missing in their meshes (`missing`) beside the cells searched.
 cudaError_t sweep_grid(const float* vert32, const float* vert_lo, const int* vot, int n_tri,
-                       int n_vert, int tri_base, float tfar, float org_elev, const SweepBuffers& b,
-                       Tri* tris, float4* tri_lo, int* err, cudaStream_t s);
+                       int n_vert, int tri_base, float tfar, float org_elev, float cells, float missing,
+                       int ndom, const SweepBuffers& b, Tri* tris, float4* tri_lo, int* err,
+                       cudaStream_t s);
 // The arrays of all domains of a call.
 struct SweepAll {
   Tri* tris;

@@ -161,15 +161,41 @@ __global__ void k_grid_init(unsigned* b) {
   for (int k = 4; k < 8; k++) b[k] = 0u;
 }
 
-// Grid geometry: cells of HZ_CELL_TRIS times the mean triangle area.
+// Holes: a cell beside an ICON vertex without its triangles looks under the
+// mesh's edge in half of its azimuths, and the repair searches those ray by ray, a
+// warp per cell. A domain without holes has few such cells, at its border. A vertex
+// missing inside costs 0.15 us (10 km spacing) to 2.3 us (0.2 km) at 24 azimuths; the
+// tree search takes 20 to 60 ns per cell more than the sweep and some 5 to 10 ms per
+// call. Times of the tree over those of the sweep, radius 40 km, vertices missing: 0.2 km,
+// 141k cells 1.7 at 2,100, 0.94 at 7,000, 0.5 at 21,000; 1.4M cells 1.5 at 7,100, 0.93 at
+// 21,000, 0.4 at 70,000; 1 km, 423k cells 1.65 at 6,300, 0.91 at 21,000; 1.4M cells 2.1 at
+// 21,000, 1.2 at 71,000; 2.5 km and more: 1.6 and more with a tenth of them missing. So the
+// tree search takes over where the missing vertices of a call are more than
+// kHolesCall and its cells over kHolesCells, those times the size of the grid's
+// cells over kHolesSize metres where that is larger.
+constexpr float kHolesCall = 6000.f, kHolesCells = 90.f, kHolesSize = 190.f;
+// Holes of the domains of a call, in err: their sum over what the cells allow, the
+// domains summed.
+enum : int { kErrHoles = 4, kErrHolesDomains = 5 };
+
+// Grid geometry: cells of HZ_CELL_TRIS times the mean triangle area. missing:
+// vertices missing beside the cells that are searched.
 __global__ void k_grid_setup(const unsigned* __restrict__ b, int n_tri, long long cap0, float tfar,
-                             float org_elev, GridDesc* __restrict__ g, int* __restrict__ err) {
+                             float org_elev, float cells, float missing, int ndom,
+                             GridDesc* __restrict__ g, int* __restrict__ err) {
   GridDesc q;
   const float x0 = ord2f(b[0]), y0 = ord2f(b[1]), h0 = ord2f(b[2]), z0 = ord2f(b[3]);
   const float x1 = ord2f(b[4]), y1 = ord2f(b[5]), h1 = ord2f(b[6]);
   const float ex = fmaxf(x1 - x0, 1.f), ey = fmaxf(y1 - y0, 1.f);
   const float big = fmaxf(fmaxf(fabsf(x0), fabsf(x1)), fmaxf(fabsf(y0), fabsf(y1)));
   float c = sqrtf(ex * ey * HZ_CELL_TRIS / (float)(n_tri > 0 ? n_tri : 1));
+  // (Sums of 65,535 domains stay within 32 bits.)
+  const float holes = missing - cells / kHolesCells * fmaxf(1.f, c / kHolesSize);
+  atomicAdd(&err[kErrHoles], (int)fminf(fmaxf(holes, -30000.f), 30000.f));
+  __threadfence();
+  if (atomicAdd(&err[kErrHolesDomains], 1) == ndom - 1 &&
+      (float)atomicAdd(&err[kErrHoles], 0) > kHolesCall)
+    atomicOr(err, kErrGrid);
   c = fminf(fmaxf(c, fmaxf(ex, ey) * 6e-5f), 1e6f);  // at most ~16,000 cells a side
   // Domains the projection cannot hold (a vertex 60 deg or more from the
   // centre's axis) or inputs that are not finite.
@@ -1722,14 +1748,16 @@ long long sweep_refs_cap(long long n_tri) { return 12 * n_tri + 4096; }
 size_t sweep_frame_floats(bool precise) { return precise ? 20 : 16; }
 
 cudaError_t sweep_grid(const float* vert32, const float* vert_lo, const int* vot, int n_tri,
-                       int n_vert, int tri_base, float tfar, float org_elev, const SweepBuffers& b,
-                       Tri* tris, float4* tri_lo, int* err, cudaStream_t s) {
+                       int n_vert, int tri_base, float tfar, float org_elev, float cells, float missing,
+                       int ndom, const SweepBuffers& b, Tri* tris, float4* tri_lo, int* err,
+                       cudaStream_t s) {
   const long long cap0 = sweep_cells_cap(n_tri);
   cudaError_t e = cudaMemsetAsync(b.count, 0, sizeof(uint32_t) * (size_t)(cap0 + 1), s);
   if (e != cudaSuccess) return e;
   k_grid_init<<<1, 1, 0, s>>>(b.bounds);
   k_gnomonic<<<grid_for(n_vert, 256), 256, 0, s>>>(vert32, n_vert, b.gv, b.bounds);
-  k_grid_setup<<<1, 1, 0, s>>>(b.bounds, n_tri, cap0, tfar, org_elev, b.grid, err);
+  k_grid_setup<<<1, 1, 0, s>>>(b.bounds, n_tri, cap0, tfar, org_elev, cells, missing, ndom, b.grid,
+                               err);
   note_launches(3);
   if (n_tri > 0) {
     k_grid_count<<<grid_for(n_tri, 256), 256, 0, s>>>(vert32, vert_lo, vot, n_tri, b.gv, b.grid,

@@ -128,3 +128,33 @@ def test_high_origins_run_the_tree(dkw, dist, elev, search):
     np.testing.assert_array_equal(s1, s0)
     if elev < 5000.0:
         assert _run(d.inputs(), args, cells=(500, 3000))[3] == "sweep"
+
+
+def _holes(d, share):
+    inputs = [np.array(a) for a in d.inputs()]
+    inputs[5][:, np.random.default_rng(1).random(d.nvertex) < share] = -2
+    return tuple(inputs)
+
+
+@pytest.mark.parametrize("share,grid_type,search", [
+    (0.0, 1, "sweep"), (0.1, 1, "sweep"), (0.1, 0, "sweep"), (0.3, 1, "sweep, then tree"),
+    (0.3, 0, "sweep, then tree")])
+def test_meshes_with_many_holes_run_the_tree(share, grid_type, search):
+    """59,000 cells, 30,000 ICON vertices: a tenth of them missing is repaired, of a third
+    the tree search is the faster one; a range of the cells has its share of them."""
+    d = synthetic.make_domain(edge_km=0.2, box_km=32.0, seed=41)
+    inputs, args = _holes(d, share), (4, grid_type, 3000.0, 0.2, 1, 2)
+    _same(inputs, search, args)
+    if share == 0.3 and grid_type == 1:
+        _same(inputs, "sweep", args, cells=(20000, 40000))
+
+
+def test_holes_of_a_batch_add_up():
+    d = synthetic.make_domain(edge_km=0.2, box_km=32.0, seed=41)
+    one = (_holes(d, 0.1), (4, 1, 3000.0, 0.2, 1, 2))
+    for n, search in ((2, "sweep"), (4, "sweep, then tree")):
+        outs, st = horizon_svf_comp_batch([one] * n, return_stats=True)
+        assert st["search"] == search
+        tree = horizon_svf_comp_batch([one] * n, leaf_size=2)
+        assert all(np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+                   for a, b in zip(outs, tree))
