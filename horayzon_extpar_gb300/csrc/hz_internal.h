@@ -155,6 +155,7 @@ struct GridDesc {
   float dadd;                 // bound of a triangle's distance beyond the walk's and its edge's
   int W, H, L;                // cells; highest pyramid level
   unsigned lmax;              // longest edge (float bits)
+  unsigned heavy;             // entries of lists longer than kHeavyList
   int ok;                     // 0: the grid cannot hold the domain (kErrGrid)
 };
 

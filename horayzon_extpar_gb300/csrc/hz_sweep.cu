@@ -239,6 +239,7 @@ __global__ void k_grid_setup(const unsigned* __restrict__ b, int n_tri, long lon
   q.H = H;
   q.L = L;
   q.lmax = 0u;
+  q.heavy = 0u;
   q.ok = ok ? 1 : 0;
   if (!ok) atomicOr(err, kErrGrid);
   *g = q;
@@ -353,15 +354,32 @@ __global__ void k_grid_count(const float* __restrict__ vert, const float* __rest
   if (threadIdx.x == 0 && smax) atomicMax(&gd->lmax, smax);
 }
 
+// Meshes that fill little of their bounds (patches far apart), or with triangles far
+// smaller than the mean (fine patches beside coarse ones): the grid's cells are
+// coarse against them, and every visit of one is a long list. Times of the tree over
+// those of the sweep by triangles per cell where the terrain is: two patches of 7,600
+// cells 3 to 20 deg apart 3.8 at 12, 2.4 at 48, 1.9 at 96, 1.2 at 190, 0.69 at 380 (of 1,200
+// cells 2.4 at 100, 1.2 at 210); two of
+// 350,000 cells 2.0 at 10, 1.6 at 40, 1.25 at 85, 0.94 at 145; half of 22,700 cells beside
+// cells 20 to 100 times as wide 1.8 at 30, 1.3 at 66, 0.94 at 115, 0.63 at 250, 0.27 at 690.
+// The tree search takes over where lists longer than this hold entries for more than
+// a quarter of the triangles.
+constexpr unsigned kHeavyList = 160;
+
 // (triangle, upper | lower height << 16) into each cell's list (triangles are
 // numbered through the domains of a call); count runs down from the cell's number of entries.
 __global__ void k_grid_fill(const int* __restrict__ vot, int n, int tri_base,
-                            const float4* __restrict__ gv, const GridDesc* __restrict__ gd, uint32_t* __restrict__ count,
-                            const uint32_t* __restrict__ start, long long cap0,
-                            uint2* __restrict__ refs, long long cap_refs, int* __restrict__ err) {
+                            const float4* __restrict__ gv, GridDesc* __restrict__ gd,
+                            uint32_t* __restrict__ count, const uint32_t* __restrict__ start,
+                            long long cap0, uint2* __restrict__ refs, long long cap_refs,
+                            int* __restrict__ err) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n || !gd->ok) return;
   const GridDesc& g = *gd;
+  for (long long k = t; k < (long long)g.W * g.H; k += n) {
+    const unsigned length = start[k + 1] - start[k];
+    if (length > kHeavyList) atomicAdd(&gd->heavy, length);
+  }
   bool over = false;
   for_cells(g, gv[vot[3LL * t]], gv[vot[3LL * t + 1]], gv[vot[3LL * t + 2]],
             [&](int cell, float up, float lo) {
@@ -409,11 +427,15 @@ __device__ __forceinline__ bool plane_fits(const GridDesc& g, float gx, float gy
 __global__ void k_grid_heights(const GridDesc* __restrict__ gd, const uint32_t* __restrict__ start,
                                const uint2* __restrict__ refs, long long cap_refs, int tri_base,
                                const int* __restrict__ vot, const float4* __restrict__ gv,
-                               long long cap0, uint16_t* __restrict__ top,
+                               long long cap0, int n_tri, uint16_t* __restrict__ top,
                                uint16_t* __restrict__ low, uint2* __restrict__ planes,
                                int* __restrict__ err) {
   if (!gd->ok) return;
   const GridDesc& g = *gd;
+  if (g.heavy > (unsigned)n_tri / 4u) {
+    if (threadIdx.x == 0) atomicOr(err, kErrGrid);
+    return;
+  }
   const long long n0 = (long long)g.W * g.H;
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n0 || !check_ok(k < cap0, kCheckGrid, k, err)) return;
@@ -1772,8 +1794,8 @@ cudaError_t sweep_grid(const float* vert32, const float* vert_lo, const int* vot
     note_launches(1);
   }
   k_grid_heights<<<grid_for(cap0, 256), 256, 0, s>>>(b.grid, b.start, b.refs,
-                                                     sweep_refs_cap(n_tri), tri_base, vot, b.gv, cap0,
-                                                     b.top, b.low, b.planes, err);
+                                                     sweep_refs_cap(n_tri), tri_base, vot, b.gv,
+                                                     cap0, n_tri, b.top, b.low, b.planes, err);
   note_launches(1);
   for (int l = 2; l <= 8; l += 2) {
     k_grid_up<<<grid_for(cap0 >> (2 * l), 128), 128, 0, s>>>(b.grid, l, cap0, b.top, b.low,

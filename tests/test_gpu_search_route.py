@@ -158,3 +158,35 @@ def test_holes_of_a_batch_add_up():
         tree = horizon_svf_comp_batch([one] * n, leaf_size=2)
         assert all(np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
                    for a, b in zip(outs, tree))
+
+
+def _beside(a, b):
+    """Two domains as one mesh without a triangle between them."""
+    n = a[0].size
+    return tuple(np.concatenate([x, y]) for x, y in zip(a[:5], b[:5])) + (
+        np.ascontiguousarray(np.concatenate([a[5], np.where(b[5] == -2, -2, b[5] + n)], 1)),)
+
+
+@pytest.mark.parametrize("deg,search", [(3, "sweep"), (20, "sweep, then tree"),
+                                        (40, "sweep, then tree")])
+def test_patches_far_apart_run_the_tree(deg, search):
+    """The grid spans the gap: its cells hold 12 triangles at 3 degrees, 380 at 20."""
+    a, b = ([np.array(x) for x in
+             synthetic.make_domain(edge_km=1.0, box_km=60.0, seed=s).inputs()] for s in (5, 6))
+    for k in (0, 3):
+        b[k] += np.radians(deg)
+        b[k + 1] += np.radians(deg / 2)
+    _same(_beside(a, b), search, (4, 1, 20000.0, 0.2, 1, 2))
+
+
+@pytest.mark.parametrize("ratio,search", [(10, "sweep"), (60, "sweep, then tree")])
+def test_fine_patches_beside_coarse_ones_run_the_tree(ratio, search):
+    """0.2 km cells beside cells 10 and 60 times as wide, the grid's cells between them."""
+    a = [np.array(x) for x in
+         synthetic.make_domain(edge_km=0.2, box_km=20.0, seed=7).inputs()]
+    b = [np.array(x) for x in
+         synthetic.make_domain(edge_km=0.2 * ratio, box_km=5.0 * ratio, seed=8).inputs()]
+    east = (a[0].max() - b[0].min()) * 1.001
+    b[0] += east
+    b[3] += east
+    _same(_beside(a, b), search, (4, 1, 20000.0, 0.2, 1, 2))
