@@ -682,20 +682,31 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
 
   // ---- BVH (cpp:395-432), or the profile sweep's grid ----
   const bool sweep = b[0].codes != nullptr;
+  // Vertices missing in the meshes beside the cells searched: one inside a closed
+  // mesh of ncell cells has six (four) of its three (two) triangles per cell.
+  std::vector<double> missing(n);
+  double missing_all = 0.0, traced = 0.0;
+  for (int d = 0; d < n; d++) {
+    const Problem& P = pr[d];
+    missing[d] = (double)std::max(0ll, (P.grid_type ? 3ll : 2ll) * P.ncell - out->n_tri[d]) /
+                 (P.grid_type ? 6.0 : 4.0) * P.cell_count / P.ncell;
+    missing_all += missing[d];
+    traced += P.cell_count;
+  }
+  const bool edges = sweep && missing_all > sweep_holes_allowed((float)traced);
   const auto build = [&]() -> int {
     Fork fk(E, s, n);
     HZ_CUDA(fk.begin());
     for (int d = 0; d < n; d++) {
       if (sweep) {
-        // A vertex inside a closed mesh of ncell cells has six (four) of its three (two)
-        // triangles per cell.
         const Problem& P = pr[d];
-        const double vertices =
-            (double)std::max(0ll, (P.grid_type ? 3ll : 2ll) * P.ncell - out->n_tri[d]) /
-            (P.grid_type ? 6.0 : 4.0);
+        if (edges)
+          HZ_CUDA(sweep_edge_cells(P.cov, P.nvert, P.ncell, P.cell_begin, P.cell_count,
+                                   reinterpret_cast<uint32_t*>(b[d].codes), b[d].err + 1,
+                                   fk.on(d)));
         HZ_CUDA(sweep_grid(b[d].vert32, b[d].vert_lo, b[d].vot, out->n_tri[d], out->n_mv[d],
                            b[d].tri_base, (float)P.dist_search, (float)P.ray_org_elev,
-                           (float)P.cell_count, (float)(vertices * P.cell_count / P.ncell), n,
+                           (float)P.cell_count, (float)missing[d], edges ? b[d].err + 1 : nullptr, n,
                            b[d].sweep, b[d].tris, b[d].tri_lo, bb.err, fk.on(d)));
         if (b[d].rz)  // the learned start's raster is laid over these bounds
           HZ_CUDA(bvh_tri_bounds(b[d].vert32, b[d].vot, out->n_tri[d], b[d].bvh, fk.on(d)));

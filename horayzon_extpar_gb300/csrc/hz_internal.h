@@ -275,13 +275,21 @@ struct SweepBuffers {
   uint2* planes;         // and of the upper bounds as planes
   uint2* refs;           // refs cap
 };
+// Counts the cells of [begin, begin + count) at an edge of the mesh into *edge (0 before):
+// some, not all, of their ICON vertices have all their cells. scratch: ncell words.
+cudaError_t sweep_edge_cells(const int* cov, int nvert, int ncell, int begin, int count,
+                             uint32_t* scratch, int* edge, cudaStream_t s);
 // Grid, lists and height pyramid of a domain, and its triangle records (mesh
 // order). Raises kErrGrid where the grid cannot hold the domain, or the call's ndom
-// domains have too many vertices missing in their meshes (`missing`) beside the cells searched.
+// domains have too many holes: `missing` vertices beside the cells searched, where *edge
+// is given at most a quarter of it.
 cudaError_t sweep_grid(const float* vert32, const float* vert_lo, const int* vot, int n_tri,
-                       int n_vert, int tri_base, float tfar, float org_elev, float cells, float missing,
-                       int ndom, const SweepBuffers& b, Tri* tris, float4* tri_lo, int* err,
-                       cudaStream_t s);
+                       int n_vert, int tri_base, float tfar, float org_elev, float cells,
+                       float missing, const int* edge, int ndom, const SweepBuffers& b, Tri* tris,
+                       float4* tri_lo, int* err, cudaStream_t s);
+// Vertices missing that a call's cells allow before the tree search is the faster
+// one, at least (on a fine grid; hz_sweep.cu).
+float sweep_holes_allowed(float cells);
 // The arrays of all domains of a call.
 struct SweepAll {
   Tri* tris;

@@ -172,17 +172,38 @@ __global__ void k_grid_init(unsigned* b) {
 // 21,000, 1.2 at 71,000; 2.5 km and more: 1.6 and more with a tenth of them missing. So the
 // tree search takes over where the missing vertices of a call are more than
 // kHolesCall and its cells over kHolesCells, those times the size of the grid's
-// cells over kHolesSize metres where that is larger.
+// cells over kHolesSize metres where that is larger. They are counted from the
+// triangles that the cells lack, at most a quarter of the cells at an edge of the
+// mesh (a hole has six, a third of all vertices missing four each): parts of a domain
+// without any triangles cost little.
 constexpr float kHolesCall = 6000.f, kHolesCells = 90.f, kHolesSize = 190.f;
 // Holes of the domains of a call, in err: their sum over what the cells allow, the
 // domains summed.
 enum : int { kErrHoles = 4, kErrHolesDomains = 5 };
 
+// ICON vertices of each cell with all their cells.
+__global__ void k_full_vertices(const int* __restrict__ cov, int nvert, uint32_t* __restrict__ full) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= nvert) return;
+  int c[6];
+  for (int k = 0; k < 6; k++) c[k] = cov[(long long)k * nvert + v];
+  for (int k = 0; k < 6; k++)
+    if (c[k] < 0) return;
+  for (int k = 0; k < 6; k++) atomicAdd(&full[c[k]], 1u);
+}
+__global__ void k_edge_cells(const uint32_t* __restrict__ full, int begin, int count,
+                             int* __restrict__ edge) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool at = k < count && full[begin + k] > 0u && full[begin + k] < 3u;
+  const unsigned n = __popc(__ballot_sync(0xffffffffu, at));
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(edge, (int)n);
+}
+
 // Grid geometry: cells of HZ_CELL_TRIS times the mean triangle area. missing:
 // vertices missing beside the cells that are searched.
 __global__ void k_grid_setup(const unsigned* __restrict__ b, int n_tri, long long cap0, float tfar,
-                             float org_elev, float cells, float missing, int ndom,
-                             GridDesc* __restrict__ g, int* __restrict__ err) {
+                             float org_elev, float cells, float missing, const int* __restrict__ edge,
+                             int ndom, GridDesc* __restrict__ g, int* __restrict__ err) {
   GridDesc q;
   const float x0 = ord2f(b[0]), y0 = ord2f(b[1]), h0 = ord2f(b[2]), z0 = ord2f(b[3]);
   const float x1 = ord2f(b[4]), y1 = ord2f(b[5]), h1 = ord2f(b[6]);
@@ -190,6 +211,7 @@ __global__ void k_grid_setup(const unsigned* __restrict__ b, int n_tri, long lon
   const float big = fmaxf(fmaxf(fabsf(x0), fabsf(x1)), fmaxf(fabsf(y0), fabsf(y1)));
   float c = sqrtf(ex * ey * HZ_CELL_TRIS / (float)(n_tri > 0 ? n_tri : 1));
   // (Sums of 65,535 domains stay within 32 bits.)
+  if (edge) missing = fminf(missing, (float)*edge * 0.25f);
   const float holes = missing - cells / kHolesCells * fmaxf(1.f, c / kHolesSize);
   atomicAdd(&err[kErrHoles], (int)fminf(fmaxf(holes, -30000.f), 30000.f));
   __threadfence();
@@ -1768,18 +1790,29 @@ __global__ void k_sweep_finish(const DomainDesc* __restrict__ doms, int ndom, in
 long long sweep_cells_cap(long long n_tri) { return std::max(4096ll, 5 * n_tri / 2); }
 long long sweep_refs_cap(long long n_tri) { return 12 * n_tri + 4096; }
 size_t sweep_frame_floats(bool precise) { return precise ? 20 : 16; }
+float sweep_holes_allowed(float cells) { return kHolesCall + cells / kHolesCells; }
+
+cudaError_t sweep_edge_cells(const int* cov, int nvert, int ncell, int begin, int count,
+                             uint32_t* scratch, int* edge, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * (size_t)ncell, s);
+  if (e != cudaSuccess || nvert <= 0) return e;
+  k_full_vertices<<<grid_for(nvert, 256), 256, 0, s>>>(cov, nvert, scratch);
+  k_edge_cells<<<grid_for(count, 256), 256, 0, s>>>(scratch, begin, count, edge);
+  note_launches(2);
+  return cudaGetLastError();
+}
 
 cudaError_t sweep_grid(const float* vert32, const float* vert_lo, const int* vot, int n_tri,
-                       int n_vert, int tri_base, float tfar, float org_elev, float cells, float missing,
-                       int ndom, const SweepBuffers& b, Tri* tris, float4* tri_lo, int* err,
-                       cudaStream_t s) {
+                       int n_vert, int tri_base, float tfar, float org_elev, float cells,
+                       float missing, const int* edge, int ndom, const SweepBuffers& b, Tri* tris,
+                       float4* tri_lo, int* err, cudaStream_t s) {
   const long long cap0 = sweep_cells_cap(n_tri);
   cudaError_t e = cudaMemsetAsync(b.count, 0, sizeof(uint32_t) * (size_t)(cap0 + 1), s);
   if (e != cudaSuccess) return e;
   k_grid_init<<<1, 1, 0, s>>>(b.bounds);
   k_gnomonic<<<grid_for(n_vert, 256), 256, 0, s>>>(vert32, n_vert, b.gv, b.bounds);
-  k_grid_setup<<<1, 1, 0, s>>>(b.bounds, n_tri, cap0, tfar, org_elev, cells, missing, ndom, b.grid,
-                               err);
+  k_grid_setup<<<1, 1, 0, s>>>(b.bounds, n_tri, cap0, tfar, org_elev, cells, missing, edge, ndom,
+                               b.grid, err);
   note_launches(3);
   if (n_tri > 0) {
     k_grid_count<<<grid_for(n_tri, 256), 256, 0, s>>>(vert32, vert_lo, vot, n_tri, b.gv, b.grid,

@@ -149,6 +149,19 @@ def test_meshes_with_many_holes_run_the_tree(share, grid_type, search):
         _same(inputs, "sweep", args, cells=(20000, 40000))
 
 
+@pytest.mark.parametrize("grid_type", [0, 1])
+def test_a_domain_without_triangles_in_parts_runs_the_sweep(grid_type):
+    """Only the south-west third of the vertices has its triangles: the triangles that
+    the cells lack are as many as with a third of the vertices missing, the cells
+    at an edge of the mesh are few."""
+    d = synthetic.make_domain(edge_km=0.2, box_km=32.0, seed=41)
+    inputs = [np.array(a) for a in d.inputs()]
+    lon, lat = inputs[3], inputs[4]
+    outside = ((lon - lon.min()) / np.ptp(lon) > 0.58) | ((lat - lat.min()) / np.ptp(lat) > 0.58)
+    inputs[5][:, outside] = -2
+    _same(inputs, "sweep", (4, grid_type, 3000.0, 0.2, 1, 2))
+
+
 def test_holes_of_a_batch_add_up():
     d = synthetic.make_domain(edge_km=0.2, box_km=32.0, seed=41)
     one = (_holes(d, 0.1), (4, 1, 3000.0, 0.2, 1, 2))
