@@ -156,6 +156,7 @@ struct GridDesc {
   int W, H, L;                // cells; highest pyramid level
   unsigned lmax;              // longest edge (float bits)
   unsigned heavy;             // entries of lists longer than kHeavyList
+  unsigned long long boxes;   // cells in the triangles' boxes
   int ok;                     // 0: the grid cannot hold the domain (kErrGrid)
 };
 

@@ -262,6 +262,7 @@ __global__ void k_grid_setup(const unsigned* __restrict__ b, int n_tri, long lon
   q.L = L;
   q.lmax = 0u;
   q.heavy = 0u;
+  q.boxes = 0ull;
   q.ok = ok ? 1 : 0;
   if (!ok) atomicOr(err, kErrGrid);
   *g = q;
@@ -283,6 +284,16 @@ __device__ __forceinline__ int grid_index(int W, int n2, int a, int b, int l) {
 // highest vertex. Between its vertices a plane triangle lies lower than the
 // linear interpolation of their heights above the sphere, by at most
 // edge^2 / 8 R.
+struct CellBox {
+  int i0, i1, j0, j1;
+};
+__device__ __forceinline__ CellBox cell_box(const GridDesc& g, float gx0, float gy0, float lx,
+                                            float hx, float ly, float hy) {
+  return {max(0, (int)floorf((gx0 + lx - g.pad) * g.inv_c)),
+          min(g.W - 1, (int)floorf((gx0 + hx + g.pad) * g.inv_c)),
+          max(0, (int)floorf((gy0 + ly - g.pad) * g.inv_c)),
+          min(g.H - 1, (int)floorf((gy0 + hy + g.pad) * g.inv_c))};
+}
 template <class F>
 __device__ __forceinline__ void for_cells(const GridDesc& g, float4 a, float4 b, float4 c, F f) {
   const float pad = g.pad;
@@ -292,10 +303,7 @@ __device__ __forceinline__ void for_cells(const GridDesc& g, float4 a, float4 b,
   const float ly = fminf(0.f, fminf(by, cy)), hy = fmaxf(0.f, fmaxf(by, cy));
   const float hmx = fmaxf(a.z, fmaxf(b.z, c.z)), hmn = fminf(a.z, fminf(b.z, c.z));
   const float gx0 = a.x - g.x0, gy0 = a.y - g.y0;
-  const int i0 = max(0, (int)floorf((gx0 + lx - pad) * g.inv_c));
-  const int i1 = min(g.W - 1, (int)floorf((gx0 + hx + pad) * g.inv_c));
-  const int j0 = max(0, (int)floorf((gy0 + ly - pad) * g.inv_c));
-  const int j1 = min(g.H - 1, (int)floorf((gy0 + hy + pad) * g.inv_c));
+  const CellBox box = cell_box(g, gx0, gy0, lx, hx, ly, hy);
   const float area = bx * cy - cx * by;
   const float e2 = fmaxf(fmaxf(bx * bx + by * by, cx * cx + cy * cy),
                          (cx - bx) * (cx - bx) + (cy - by) * (cy - by));
@@ -313,9 +321,9 @@ __device__ __forceinline__ void for_cells(const GridDesc& g, float4 a, float4 b,
   const float s0 = (fabsf(n0x) + fabsf(n0y)) * hw, s1 = (fabsf(n1x) + fabsf(n1y)) * hw,
               s2 = (fabsf(n2x) + fabsf(n2y)) * hw;
   const bool sat = fabsf(area) > 1e-6f * e2;  // else a sliver: its box
-  for (int j = j0; j <= j1; j++) {
+  for (int j = box.j0; j <= box.j1; j++) {
     const float y = ((float)j + 0.5f) * g.c - gy0;
-    for (int i = i0; i <= i1; i++) {
+    for (int i = box.i0; i <= box.i1; i++) {
       const float x = ((float)i + 0.5f) * g.c - gx0;
       if (sat && (n0x * x + n0y * y + s0 < 0.f ||
                   n1x * (x - bx) + n1y * (y - by) + s1 < 0.f ||
@@ -335,6 +343,21 @@ __device__ __forceinline__ void for_cells(const GridDesc& g, float4 a, float4 b,
   }
 }
 
+// Cells in a triangle's box.
+__device__ __forceinline__ unsigned box_cells(const GridDesc& g, float4 a, float4 b, float4 c) {
+  const CellBox box =
+      cell_box(g, a.x - g.x0, a.y - g.y0, fminf(0.f, fminf(b.x - a.x, c.x - a.x)),
+               fmaxf(0.f, fmaxf(b.x - a.x, c.x - a.x)), fminf(0.f, fminf(b.y - a.y, c.y - a.y)),
+               fmaxf(0.f, fmaxf(b.y - a.y, c.y - a.y)));
+  return (unsigned)max(0, box.i1 - box.i0 + 1) * (unsigned)max(0, box.j1 - box.j0 + 1);
+}
+
+// Most cells in the box of one triangle (a thread goes through them), and in the
+// boxes of all per triangle: a proper mesh has some ten, lists hold twelve. Beyond
+// them (vertices that join cells from all over the domain) the time of the build would
+// grow with the square of the triangles: the call is the tree search's.
+constexpr unsigned kMaxBox = 1u << 16, kMaxBoxes = 64u;
+
 // Triangles per cell; also the triangle records (identity order; precise:
 // the FP32 residuals too) and the longest edge.
 __global__ void k_grid_count(const float* __restrict__ vert, const float* __restrict__ vert_lo,
@@ -342,11 +365,30 @@ __global__ void k_grid_count(const float* __restrict__ vert, const float* __rest
                              GridDesc* __restrict__ gd, uint32_t* __restrict__ count,
                              long long cap0, Tri* __restrict__ tris, float4* __restrict__ tri_lo,
                              int* __restrict__ err) {
-  __shared__ unsigned smax;
-  if (threadIdx.x == 0) smax = 0u;
+  __shared__ unsigned smax, boxes, skip;
+  if (threadIdx.x == 0) {
+    smax = 0u;
+    boxes = 0u;
+    skip = 0u;
+  }
   __syncthreads();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n && gd->ok) {
+  const bool mine = t < n && gd->ok;
+  if (mine) {
+    const unsigned k = box_cells(*gd, gv[vot[3LL * t]], gv[vot[3LL * t + 1]], gv[vot[3LL * t + 2]]);
+    if (k > kMaxBox) skip = 1u;
+    atomicAdd(&boxes, min(k, kMaxBox));
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 &&
+      (skip || atomicAdd(&gd->boxes, (unsigned long long)boxes) + boxes >
+                   (unsigned long long)kMaxBoxes * n + kMaxBox)) {
+    skip = 1u;
+    gd->ok = 0;
+    atomicOr(err, kErrGrid);
+  }
+  __syncthreads();
+  if (mine && !skip) {
     const GridDesc& g = *gd;
     const int v0 = vot[3LL * t], v1 = vot[3LL * t + 1], v2 = vot[3LL * t + 2];
     const float* p0 = vert + 3LL * v0;

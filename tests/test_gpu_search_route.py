@@ -203,3 +203,25 @@ def test_fine_patches_beside_coarse_ones_run_the_tree(ratio, search):
     b[0] += east
     b[3] += east
     _same(_beside(a, b), search, (4, 1, 20000.0, 0.2, 1, 2))
+
+
+def test_vertices_that_join_far_cells_run_the_tree_at_once():
+    """Every triangle spans much of the domain: going through all grid cells of each
+    took the square of the mesh's size before the lists overflowed (here 40 ms, a
+    minute for a million cells)."""
+    d = synthetic.make_domain(edge_km=1.0, box_km=110.0, seed=15)
+    inputs = [np.array(a) for a in d.inputs()]
+    rng = np.random.default_rng(15)
+    full = np.nonzero((inputs[5] != -2).all(axis=0))[0]
+    for k in range(6):  # a cell per sextant of the domain: six different ones
+        part = np.arange(k * (d.ncell // 6), (k + 1) * (d.ncell // 6))
+        inputs[5][k, full] = rng.choice(part, full.size)
+    args, kw = (4, 1, 20000.0, 0.2, 1, 2), dict(cells=(0, 64))
+    _same(inputs, "sweep, then tree", args, **kw)
+
+    def lost():
+        st = horizon_svf_comp_py(*inputs, *args, return_stats=True, **kw)[2]
+        return st["ms_total"] - sum(st[k] for k in ("ms_h2d", "ms_mesh", "ms_bvh", "ms_trace",
+                                                    "ms_d2h"))
+
+    assert min(lost() for _ in range(3)) < 10.0
