@@ -244,6 +244,9 @@ Buffers carve_domain(Carver& c, long long ncell, long long nvert, long long nhor
   return b;
 }
 
+// Groups that a batch's domains are searched and finished in (profile sweep).
+constexpr int kMaxGroups = 4;
+
 // Device buffers shared by the domains of one call.
 struct BatchBuffers {
   DomainDesc* doms;
@@ -281,7 +284,7 @@ BatchBuffers carve_batch(Carver& c, int n, long long total_cells, const SweepSiz
   b.mlp = c.take<float>(kMlpParams);
   b.doms = c.take<DomainDesc>(n);
   b.order = c.take<int32_t>(total_cells);
-  b.work = c.take<int>(4);
+  b.work = c.take<int>(4 * kMaxGroups);
   if (sweep) {
     b.list = c.take<int>(total_cells);
     b.listed = c.take<unsigned>(total_cells / 32 + 1);
@@ -548,6 +551,14 @@ constexpr long long kSweepWaves = 4;
 // 240 azimuths 41.4 -> 40.1 ms, 1.2M cells 42.6 -> 41.9; with the runs of two
 // azimuths 21k cells x 360 lost 4 %).
 constexpr int kTailSplit = 4, kTailAzimuths = 4;
+// A domain is done when the repair and the outputs of its group are: all
+// domains of a call together, unless they go in groups, one after another. A group
+// more costs 0.2 to 0.9 ms (idle lanes at its end, its repair), so that they are made where little
+// is lost: a quarter of the work each in calls of kGroupWork evaluations (64 domains, 206M:
+// 136.9 -> 137.3 ms, half of the domains done after 36 ms; 14 domains, 13M: 11.3 -> 13.3, not cut), and
+// before a domain of kGroupGap times the work of all before it (a small domain beside
+// one of 6.9M: 8.3 -> 8.7 ms, the small one done after 0.5).
+constexpr double kGroupWork = 6e7, kGroupGap = 16.0, kGroupRest = 4e6;
 
 // Runs the pipeline for n domains whose arrays are device pointers in pr[].
 // With stop != kFull it ends after the mesh (or ENU) stage and leaves the
@@ -788,13 +799,6 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
     const int rl = resident_lanes(&lanes);
     if (rl) return rl;
     const bool border_first = !sweep && items >= kBorderFirstWaves * lanes;
-    // Sweep items: runs of consecutive azimuths per cell, enough of them to
-    // fill the lanes a few times over.
-    long long cells_all = 0;
-    for (int d = 0; d < n; d++) cells_all += pr[d].cell_count;
-    const long long runs_wanted = (kSweepWaves * lanes + cells_all - 1) / std::max(1ll, cells_all);
-    const long long runs_half =
-        (kSweepWaves / 2 * lanes + cells_all - 1) / std::max(1ll, cells_all);
     // Queue order of the domains: least work (cells x azimuths) first, so
     // that the small domains of a batch complete early (shortest job first:
     // the lowest mean completion time for the same total work).
@@ -804,9 +808,41 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
       return (long long)pr[x].cell_count * pr[x].nhori * pr[x].refine <
              (long long)pr[y].cell_count * pr[y].nhori * pr[y].refine;
     });
+    // Groups of domains of the sweep.
+    std::vector<SweepGroup> group(1);
+    std::vector<int> group_of(n, 0);
+    if (sweep && n > 1) {
+      const auto work_of = [&](int d) {
+        return (double)pr[d].cell_count * pr[d].nhori * pr[d].refine;
+      };
+      double all = 0.0, done = 0.0;
+      for (int d = 0; d < n; d++) all += work_of(d);
+      for (int j = 0; j < n; j++) {
+        const double w = work_of(queue[j]);
+        const bool quarter = all >= kGroupWork && done + w > all / kMaxGroups * group.size();
+        if (j > 0 && (int)group.size() < kMaxGroups &&
+            ((quarter && group.back().ndom > 0) || w >= std::max(kGroupGap * done, kGroupRest))) {
+          group.emplace_back();
+          group.back().first = j;
+        }
+        group_of[j] = (int)group.size() - 1;
+        group.back().ndom++;
+        done += w;
+      }
+    } else {
+      group[0].ndom = n;
+    }
+    for (int j = 0; j < n; j++) group[group_of[j]].total += pr[queue[j]].cell_count;
     Fork fk(E, s, n, beside);
     HZ_CUDA(fk.begin());
     for (int j = 0; j < n; j++) {
+      SweepGroup& gr = group[group_of[j]];
+      if (j == gr.first) gr.k_begin = (int)total;
+      // Sweep items: runs of consecutive azimuths per cell, enough of them in a group to
+      // fill the lanes a few times over.
+      const long long cells = std::max(1, gr.total);
+      const long long runs_wanted = (kSweepWaves * lanes + cells - 1) / cells,
+                      runs_half = (kSweepWaves / 2 * lanes + cells - 1) / cells;
       const int d = queue[j];
       const Problem& P = pr[d];
       const int L = P.nhori * P.refine;
@@ -870,7 +906,7 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
       D.groups = P.groups;
       D.deep_walk = opt.elev_walk == HZ_WALK_BISECT ? 1 : 0;
       D.occ_cache = opt.occluder_cache != 0 ? 1 : 0;
-      D.item_begin = total_items;
+      D.item_begin = sweep ? gr.items : total_items;
       D.svf_part = b[d].svf_part;
       D.raw_j = n == 1 ? opt.raw_index : nullptr;
       D.grid = b[d].sweep.grid;
@@ -895,14 +931,14 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
       D.run_extra = L % D.runs;
       D.tail_begin = P.cell_count;
       D.tail_runs = D.runs;
-      if (j == n - 1 && D.run_len >= kTailAzimuths) {
+      if (j == gr.first + gr.ndom - 1 && D.run_len >= kTailAzimuths) {
         D.tail_runs = std::max(D.runs, std::min(kTailSplit * D.runs, L / kTailAzimuths));
         D.tail_begin -= (int)std::min<long long>(P.cell_count / 2, lanes / D.runs);
       }
       D.tail_run_len = L / D.tail_runs;
       D.tail_run_extra = L % D.tail_runs;
-      D.items = (long long)D.tail_begin * D.runs +
-                (long long)(P.cell_count - D.tail_begin) * D.tail_runs;
+      const long long runs_all = (long long)D.tail_begin * D.runs +
+                                 (long long)(P.cell_count - D.tail_begin) * D.tail_runs;
       D.centre = frames[d].centre;
       D.pole = frames[d].pole;
       D.ray_org_elev = P.ray_org_elev;
@@ -921,7 +957,8 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
       D.tfar = (float)P.dist_search;
       desc[j] = D;  // in queue order: k_begin and item_begin increase with j
       total += P.cell_count;
-      total_items += sweep ? D.items : (long long)P.cell_count * P.groups;
+      total_items += sweep ? runs_all : (long long)P.cell_count * P.groups;
+      gr.items += runs_all;
     }
     const auto frames_on = [&](cudaStream_t to) {
       const cudaError_t e = cudaMemcpyAsync(bb.doms, desc, sizeof(DomainDesc) * (size_t)n,
@@ -951,8 +988,11 @@ int run_batch(Engine& E, const Problem* pr, const Buffers* b, int n, const Batch
     if (sweep) {
       // The lowest ray of a search: one step past the floor (cpp:538).
       const int s_full = std::min(-1, (int)floor(opt.elev_floor_deg * 2.0) - 1);
-      HZ_CUDA(sweep_search(bb.doms, n, bb.order, (int)total, (int)total_items, s_full, bb.work,
-                           bb.list, bb.listed, bb.all, bb.counters, bb.err, b[0].tri_lo != nullptr, s));
+      HZ_CUDA(cudaMemsetAsync(bb.work, 0, 4 * kMaxGroups * sizeof(int), s));
+      HZ_CUDA(cudaMemsetAsync(bb.listed, 0, sizeof(unsigned) * ((size_t)total / 32 + 1), s));
+      for (size_t k = 0; k < group.size(); k++)
+        HZ_CUDA(sweep_search(bb.doms, group[k], bb.order, s_full, bb.work + 4 * k, bb.list,
+                             bb.listed, bb.all, bb.counters, bb.err, b[0].tri_lo != nullptr, s));
     } else
     HZ_CUDA(trace_flat(bb.doms, n, bb.order, (int)total, (int)total_items, bb.work,
                        bb.counters, bb.err, knobs, opt.count_work != 0,

@@ -199,7 +199,7 @@ struct DomainDesc {
   // Profile sweep (hz_sweep.cu): grid, pyramid, list starts and lists; FP32
   // cell frames by work position; result codes [L][ncell]; items per cell (runs of
   // consecutive azimuths: run_len each, the first run_extra one more), the same for
-  // the cells from work position tail_begin on, and items of the domain.
+  // the cells from work position tail_begin on.
   const GridDesc* grid;
   const uint2* planes;
   const uint16_t* low;
@@ -213,7 +213,6 @@ struct DomainDesc {
   const float* tan_m;         // [kTanTable] tangents of (k - kTanTable / 2) * 0.5 deg
   int runs, run_len, run_extra;
   int tail_begin, tail_runs, tail_run_len, tail_run_extra;
-  long long items;
   int16_t* raw_j;             // optional output: unclipped horizon j (h = j * 0.25 deg)
   double3 centre, pole;       // Earth centre / North Pole in ENU
   double ray_org_elev, hori_acc, elev_floor;
@@ -305,11 +304,18 @@ struct SweepAll {
 // Cell frames of all domains (after cell_order).
 cudaError_t sweep_frames(const DomainDesc* doms, int ndom, const int32_t* order, int total,
                          bool precise, cudaStream_t s);
-// Sweep, repair and outputs of all domains (after sweep_frames and
-// trace_tables). s_full: the lowest lattice elevation a search can ask for.
-// work: 3 ints; list, listed: `total` work positions and bits.
-cudaError_t sweep_search(const DomainDesc* doms, int ndom, const int32_t* order, int total,
-                         int total_items, int s_full, int* work, int* list, unsigned* listed,
+// Domains of a call, next to one another in queue order, that are searched and finished
+// before the next group begins; their work positions and items.
+struct SweepGroup {
+  int first, ndom;
+  int k_begin, total;
+  long long items;
+};
+// Sweep, repair and outputs of one group (after sweep_frames and trace_tables).
+// s_full: the lowest lattice elevation a search can ask for. work: 3 ints, 0 before;
+// list, listed: work positions and bits of the call, the bits 0 before.
+cudaError_t sweep_search(const DomainDesc* doms, const SweepGroup& group, const int32_t* order,
+                         int s_full, int* work, int* list, unsigned* listed,
                          const SweepAll& all, unsigned long long* counters, int* err,
                          bool precise, cudaStream_t s);
 

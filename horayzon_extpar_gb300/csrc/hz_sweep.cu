@@ -1127,14 +1127,6 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
           sh.prev[t] = code > kCodeAllMiss ? code : kUnknown;
           if (code > kCodeAllMiss && a < kGuesses) sh.guess[wid][a] = (short)code;
           sh.az[t] = a + 1;
-          if (a + 1 == sh.az_end[t] && D.done) {
-            const unsigned long long fin = atomicAdd(&D.done[0], 1ull) + 1ull;
-            if (fin == (unsigned long long)D.items) {
-              unsigned long long now;
-              asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-              D.done[1] = now;
-            }
-          }
         }
       }
       // New items for the lanes whose azimuths are done.
@@ -1519,12 +1511,12 @@ __device__ __forceinline__ double2 elevation(const DomainDesc& D, int m) {
 // The first azimuth of every run but a cell's first was swept from kRunStart:
 // where the search can come to it from below that (the azimuth before has no
 // hits from there up, or is open), the cell goes to the repair.
-__global__ void k_sweep_runs(const DomainDesc* __restrict__ doms, int ndom, int total,
+__global__ void k_sweep_runs(const DomainDesc* __restrict__ doms, int ndom, int first, int total,
                              int* __restrict__ list, int* __restrict__ list_n,
                              unsigned* __restrict__ listed, const int* __restrict__ order,
                              const int* __restrict__ err) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= total || (*err & kErrGrid)) return;
+  const int k = first + blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= first + total || (*err & kErrGrid)) return;
   const long long gid = order[k];
   const DomainDesc& D = doms[domain_of(doms, ndom, gid)];
   const int cell = (int)(gid - D.cell_offset);
@@ -1807,13 +1799,16 @@ __device__ __forceinline__ unsigned finish_sweep(const DomainDesc& D, int cell, 
   return rays;
 }
 
-__global__ void k_sweep_finish(const DomainDesc* __restrict__ doms, int ndom, int total,
+// With D.done (a batch): the cells done of each domain, and the time of its last one.
+__global__ void k_sweep_finish(const DomainDesc* __restrict__ doms, int ndom, int first, int total,
                                unsigned long long* __restrict__ counters,
                                int* __restrict__ err) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int k = first + blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long rays = 0;
-  if (k < total && !(*err & kErrGrid)) {
-    int lo = 0, hi = ndom - 1;
+  const bool mine = k < first + total && !(*err & kErrGrid);
+  int lo = 0;
+  if (mine) {
+    int hi = ndom - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
       if (doms[mid].k_begin <= k) lo = mid;
@@ -1822,6 +1817,19 @@ __global__ void k_sweep_finish(const DomainDesc* __restrict__ doms, int ndom, in
     const DomainDesc& D = doms[lo];
     const int cell = D.cell_begin + (int)(k - D.k_begin);
     rays = D.refine == 1 ? finish_sweep<true>(D, cell, err) : finish_sweep<false>(D, cell, err);
+  }
+  if (doms[0].done) {
+    __threadfence();  // the outputs before the count
+    const unsigned peers = __match_any_sync(0xffffffffu, mine ? lo : -1);
+    if (mine && (int)(threadIdx.x & 31) == __ffs(peers) - 1) {
+      const DomainDesc& D = doms[lo];
+      const unsigned long long n = __popc(peers);
+      if (atomicAdd(&D.done[0], n) + n == (unsigned long long)D.ncell_traced) {
+        unsigned long long now;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        D.done[1] = now;
+      }
+    }
   }
   rays = warp_sum_u64(rays);
   if ((threadIdx.x & 31) == 0 && rays) atomicAdd(&counters[0], rays);
@@ -1894,8 +1902,8 @@ static long long resident_blocks(K kernel, int block, int wanted) {
 }
 
 template <bool kPrecise>
-static cudaError_t launch_search(const DomainDesc* doms, int ndom, const int32_t* order, int total,
-                                 int total_items, int s_full, int* work, int* list,
+static cudaError_t launch_search(const DomainDesc* doms, int ndom, const int32_t* order, int first,
+                                 int total, int total_items, int s_full, int* work, int* list,
                                  unsigned* listed, const SweepScene& sc, int* err,
                                  cudaStream_t s) {
   // Fewer items than resident threads go to all warps, a few lanes each: the
@@ -1912,7 +1920,7 @@ static cudaError_t launch_search(const DomainDesc* doms, int ndom, const int32_t
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (total_items > total) {
-    k_sweep_runs<<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, total, list, work + 1, listed,
+    k_sweep_runs<<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, first, total, list, work + 1, listed,
                                                       order, err);
     note_launches(1);
   }
@@ -1933,24 +1941,23 @@ cudaError_t sweep_frames(const DomainDesc* doms, int ndom, const int32_t* order,
   return cudaGetLastError();
 }
 
-cudaError_t sweep_search(const DomainDesc* doms, int ndom, const int32_t* order, int total,
-                         int total_items, int s_full, int* work, int* list, unsigned* listed,
-                         const SweepAll& all, unsigned long long* counters, int* err,
-                         bool precise, cudaStream_t s) {
-  if (total <= 0 || ndom <= 0) return cudaSuccess;
-  // work[0] is reset by cell_order; work[1]: listed cells, work[2]: taken by the repair.
-  cudaError_t e = cudaMemsetAsync(work + 1, 0, 2 * sizeof(int), s);
-  if (e == cudaSuccess)
-    e = cudaMemsetAsync(listed, 0, sizeof(unsigned) * ((size_t)total / 32 + 1), s);
-  if (e != cudaSuccess) return e;
+cudaError_t sweep_search(const DomainDesc* doms, const SweepGroup& group, const int32_t* order,
+                         int s_full, int* work, int* list, unsigned* listed, const SweepAll& all,
+                         unsigned long long* counters, int* err, bool precise, cudaStream_t s) {
+  if (group.total <= 0 || group.ndom <= 0) return cudaSuccess;
+  doms += group.first;
+  list += group.k_begin;
   const SweepScene sc{all.tris,   all.tri_lo, all.refs,    all.start,
                       all.planes, all.n_tri,  all.n_cells, all.n_refs};
-  e = precise ? launch_search<true>(doms, ndom, order, total, total_items, s_full, work, list,
-                                    listed, sc, err, s)
-              : launch_search<false>(doms, ndom, order, total, total_items, s_full, work, list,
-                                     listed, sc, err, s);
+  // work[0]: taken items, work[1]: listed cells, work[2]: taken by the repair.
+  const cudaError_t e =
+      precise ? launch_search<true>(doms, group.ndom, order, group.k_begin, group.total,
+                                    (int)group.items, s_full, work, list, listed, sc, err, s)
+              : launch_search<false>(doms, group.ndom, order, group.k_begin, group.total,
+                                     (int)group.items, s_full, work, list, listed, sc, err, s);
   if (e != cudaSuccess) return e;
-  k_sweep_finish<<<grid_for(total, 128), 128, 0, s>>>(doms, ndom, total, counters, err);
+  k_sweep_finish<<<grid_for(group.total, 128), 128, 0, s>>>(doms, group.ndom, group.k_begin,
+                                                            group.total, counters, err);
   note_launches(1);
   return cudaGetLastError();
 }

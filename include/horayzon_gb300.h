@@ -263,18 +263,26 @@ typedef struct hz_domain {
     int32_t num_cell, num_vertex, num_hori, grid_type;
     double dist_search, ray_org_elev;
     int32_t refine_factor, svf_type;
-    double latency_ms;       /* out: completion time of the domain's last cell,
-                                measured from the start of the search launch */
+    double latency_ms;       /* out: time at which the domain's last cell was done, measured
+                                from the start of the search. Profile sweep: its horizons
+                                and sky view factors are written on the device; tree
+                                search: its rays are cast, degrees and sky view factors
+                                follow for all domains together */
 } hz_domain;
 
 /*
- * Many independent domains in one call: mesh, frames and BVH per domain
- * (each BVH in its own slice of one device arena), then ONE persistent
- * search launch over the cells of all domains. Every domain carries its own
+ * Many independent domains in one call: mesh, frames and grid (or BVH) per
+ * domain, each in its own slice of one device arena, then one search over the
+ * cells of all domains. Every domain carries its own
  * arguments (num_hori, grid_type, ...); 1 <= n_domains <= 65535. on_device
  * = 0: host arrays (copied in and out); on_device = 1: device arrays, work
  * enqueued on `stream`. The search takes the domains in ascending order of
- * work (cells x azimuths), so small domains complete first (latency_ms).
+ * work (cells x azimuths). The profile sweep finishes them in up to four groups of
+ * that order, so that small domains complete first (latency_ms): a quarter of
+ * the work each from 60M (cell, azimuth) evaluations on, and what comes before a domain
+ * of at least 4M evaluations and 16 times the work of all before it; else all domains
+ * complete together. One domain that the sweep turns down takes the whole call to
+ * the tree search.
  * No reference counterpart: the reference computes one domain per call
  * (mo_lradtopo_horayzon.cpp:562-785).
  */

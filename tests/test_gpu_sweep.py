@@ -181,3 +181,40 @@ def test_gpu_sweep_under_a_roof(nh, search):
     st0, st1 = _same(inputs, (nh, 1, 20000.0, 0.2, 1, 2))
     assert st0["num_rays"] > 700 * nh * np.sum(r < 3.0)  # full turns
     assert st1["search"] == search
+
+
+def test_gpu_sweep_latency_holds_repair_and_outputs():
+    """A batch of meshes with holes, whose cells are repaired for most of the search:
+    their domains are done at its end, not when the sweep's last item is."""
+    batch = []
+    for seed in (51, 52):
+        d = synthetic.make_domain(edge_km=1.0, box_km=140.0, seed=seed)
+        inputs = [np.array(a) for a in d.inputs()]
+        inputs[5][:, np.random.default_rng(seed).random(d.nvertex) < 0.05] = -2
+        batch.append((inputs, (24, 1, 40000.0, 0.2, 1, 2)))
+    for _ in range(2):
+        _, st = horizon_svf_comp_batch(batch, return_stats=True)
+    assert st["search"] == "sweep"
+    assert all(0.85 * st["ms_trace"] < t < 1.05 * st["ms_trace"] for t in st["latency_ms"]), st
+
+
+def test_gpu_sweep_groups_of_a_large_batch():
+    """From 60M evaluations on the domains complete in groups of a quarter of the
+    work, in ascending order of their work; results are those of single calls."""
+    edges, boxes = [0.5] * 9, [40.0, 45.0, 160.0, 170.0, 180.0, 190.0, 200.0, 210.0, 220.0]
+    doms = [(synthetic.make_domain(edge_km=e, box_km=b, seed=60 + k).inputs(),
+             (36, 1, 4000.0, 0.2, 1, 2)) for k, (e, b) in enumerate(zip(edges, boxes))]
+    order = [4, 0, 8, 2, 6, 1, 7, 3, 5]
+    outs, st = horizon_svf_comp_batch([doms[k] for k in order], return_stats=True)
+    assert st["search"] == "sweep"
+    lat = np.empty(9)
+    lat[order] = st["latency_ms"]
+    assert sum(d[0][0].size for d in doms) * 36 >= 6e7
+    assert lat[0] < 0.4 * lat[8] and lat[4] < 0.7 * lat[8]
+    assert (np.diff(lat) > -0.1 * lat[8]).all()  # in order, within a group close together
+    rays = 0
+    for k, (h, s) in zip(order, outs):
+        h1, s1, st1 = horizon_svf_comp_py(*doms[k][0], *doms[k][1], return_stats=True)
+        assert np.array_equal(h, h1) and np.array_equal(s, s1)
+        rays += st1["num_rays"]
+    assert rays == st["num_rays"]
