@@ -13,8 +13,13 @@ one (cell, azimuth) of the output.
 * ``e2e``: the public host entry (hz_horizon_svf) on pinned host buffers,
   host->device inputs and device->host outputs inside the timed region.
 * ``roofline``: the call against the bytes it cannot do without (every input
-  read once, every output written once); beside them the rays, node visits and
-  triangle tests of the same search by tree traversal, counted on the device.
+  read once, every output written once); ``traffic`` is the sweep's DRAM traffic
+  where the committed profile is of the timed domain (``k_sweep_profile`` names its
+  size); beside them the node visits and triangle tests of the same search by tree
+  traversal, counted on the device.
+* untimed reports (learned start, precision, batch, drop-in, other
+  configurations) go to stderr, one JSON line each: stdout holds the result line
+  alone.
 * ``cpu_baseline`` (rank 0, N=1): the CPU oracle on all host cores on a
   bounded sample (full mesh + BVH build, ray phase on a random cell subset,
   scaled to the full domain).
@@ -105,18 +110,32 @@ def l2_read_peak(dev) -> float | None:
     return best
 
 
-def traffic_from_profile():
-    """DRAM bytes per launch of the search kernel from the committed ncu summary."""
+def traffic_from_profile(ncell: int):
+    """DRAM traffic of one launch of the sweep from the committed ncu summary:
+    (bytes if it was taken on a domain of ncell cells else None, bytes, its cells)."""
     path = os.path.join(ROOT, "profiles", "k_sweep_c3_300km.md")
-    if not os.path.exists(path):
-        return None
-    for line in open(path):
-        if line.startswith("traffic_bytes_per_launch:"):
-            try:
-                return float(line.split(":", 1)[1].strip())
-            except ValueError:
-                return None
-    return None
+    got = {}
+    if os.path.exists(path):
+        for line in open(path):
+            for key in ("traffic_bytes_per_launch", "traffic_cells"):
+                if line.startswith(key + ":"):
+                    got[key] = float(line.split(":", 1)[1])
+    if len(got) < 2:
+        return None, None, None
+    nbytes, cells = got["traffic_bytes_per_launch"], int(got["traffic_cells"])
+    return (nbytes if cells == ncell else None), nbytes, cells
+
+
+def emit(line: dict, reports: dict, path: str | None = None) -> None:
+    """The result as ONE JSON line on stdout, short enough to be read from the tail of a
+    log; the untimed reports beside it, one JSON line each, on stderr (and all in
+    `path`)."""
+    for name, report in reports.items():
+        print(json.dumps({"report": name, **report}), file=sys.stderr, flush=True)
+    if path:
+        with open(path, "w") as f:
+            json.dump({**line, **reports}, f, indent=1)
+    print(json.dumps(line), flush=True)
 
 
 class ClockSampler:
@@ -742,7 +761,7 @@ def run_gpu(args):
     peak, peak_kind = measured_peaks()
     alg_bytes = h2d + d2h
     achieved = alg_bytes / (ms * 1e-3) / 1e9
-    traffic = traffic_from_profile()
+    traffic, profiled, profiled_cells = traffic_from_profile(dom.ncell)
 
     if rank != 0:
         if world > 1:
@@ -783,14 +802,15 @@ def run_gpu(args):
                     "ms_h2d", "ms_mesh", "ms_bvh", "ms_trace", "ms_d2h")}},
         # The sweep reads its grid and triangles from L1 / L2: what bounds it is
         # instruction issue and the latency of those reads, not bytes.
-        "roofline": {"kernel": "k_sweep", "bound": "instruction issue + l1/l2 latency",
+        "roofline": {"kernel": "whole call (k_sweep: 90 % of it)",
+                     "bound": "instruction issue + l1/l2 latency",
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                     "frac_of": "measured HBM copy bandwidth (MEASURED_PEAKS.json hbm_gbs)",
+                     "frac": achieved / peak, "peak_kind": peak_kind,
                      "alg_bytes_per_step": alg_bytes,
                      "floor_ms": alg_bytes / (peak * 1e9) * 1e3,
+                     "traffic": traffic,
+                     "k_sweep_profile": {"traffic": profiled, "cells": profiled_cells},
                      "l2_peak": l2_peak,
-                     "l2_peak_kind": "measured (hz_l2_probe: 32 MiB, 300 passes, ld.global.cg)",
                      "tree_node_visits_per_ray": st_count["node_visits"] / rays,
                      "tree_tri_tests_per_ray": st_count["tri_tests"] / rays,
                      "bvh4_node_visits_per_ray": st_wide["node_visits"] / rays,
@@ -799,9 +819,9 @@ def run_gpu(args):
         "cpu_baseline": cpu,
         "clocks": clk.summary(),
         "gpu_launches": (launches * args.steps) if launches else None,
-        **extras,
+        "reports": sorted(extras),
     }
-    print(json.dumps(line), flush=True)
+    emit(line, extras, args.reports)
     if world > 1:
         torch.distributed.destroy_process_group()
     return 0
@@ -880,6 +900,8 @@ def main():
                     help="skip every untimed extra report")
     ap.add_argument("--extras", default="all",
                     help="comma-separated extra reports to run: " + ",".join(EXTRAS))
+    ap.add_argument("--reports", default=None, metavar="PATH",
+                    help="also write the result and the extra reports to this JSON file")
     ap.add_argument("--cpu-seconds", type=float, default=8.0,
                     help="target seconds of CPU ray work per CPU measurement")
     ap.add_argument("--parity-cells", type=int, default=20000,
