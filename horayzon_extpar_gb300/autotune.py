@@ -31,16 +31,20 @@ import threading
 from . import _lib
 from .horizon_svf import horizon_svf_comp_device
 
-#: Candidate values per knob, in the order the descent visits them.
+#: Candidate values of the tree search per knob, in the order the descent visits them.
 GRID = {
-    "leaf_size": (0, 2, 1, 3, 4, 6),
-    "advance_min": (0, 16, 12, 20, 8, 24),
-    "leaf_min": (0, 1, 2, 4, 8, 12),
-    "queue_chunk": (0, 32, 16, 24, 48, 64),
+    "leaf_size": (2, 1, 3, 4, 6),
+    "advance_min": (16, 12, 20, 8, 24),
+    "leaf_min": (1, 2, 4, 8, 12),
+    "queue_chunk": (32, 16, 24, 48, 64),
     "kernel": (_lib.HZ_KERNEL_PERSISTENT, _lib.HZ_KERNEL_PERSISTENT_BVH2),
 }
+#: The profile sweep: no knob of the tree set.
 DEFAULTS = {"leaf_size": 0, "advance_min": 0, "leaf_min": 0, "queue_chunk": 0,
             "kernel": _lib.HZ_KERNEL_PERSISTENT}
+#: Below this share of the tree search's time with its own defaults the sweep is not
+#: compared further: the knobs change that time by a fifth at most.
+ENOUGH = 0.6
 _lock = threading.Lock()
 
 
@@ -71,11 +75,12 @@ def _load_cache(path):
 
 
 def _time(inputs, args, cells, knobs, reps, stream):
+    """Best search time and the search that ran."""
     best = math.inf
     for _ in range(reps):
         _, _, st = horizon_svf_comp_device(*inputs, *args, cells=cells, stream=stream, **knobs)
         best = min(best, st["ms_trace"])
-    return best
+    return best, st["search"]
 
 
 def tune(inputs, args, sample_cells: int = 250_000, reps: int = 2, rounds: int = 2,
@@ -96,29 +101,38 @@ def tune(inputs, args, sample_cells: int = 250_000, reps: int = 2, rounds: int =
             hit = _load_cache(path).get(key)
         if hit:
             return dict(hit, cached=True)
+    built_in = grid is None
     grid = grid or GRID
     n = min(sample_cells, ncell)
     begin = (ncell - n) // 2
     cells = (begin, begin + n)
-    # Start from the first value of each knob in the grid (the library
-    # defaults head the built-in grid).
+    # The descent starts from the first value of each knob in the grid (the tree
+    # search's defaults head the built-in one).
     cur = {k: (grid[k][0] if k in grid else v) for k, v in DEFAULTS.items()}
     _time(inputs, args, cells, cur, 1, stream)  # warm-up (allocations, first launch)
-    best_ms = _time(inputs, args, cells, cur, reps, stream)
-    trials = 1
-    for _ in range(rounds):
+    best_ms, _ = _time(inputs, args, cells, cur, reps, stream)
+    trials, sweep_ms = 1, math.inf
+    if built_in:
+        _time(inputs, args, cells, DEFAULTS, 1, stream)
+        ms, search = _time(inputs, args, cells, DEFAULTS, reps, stream)
+        trials += 1
+        if search == "sweep":  # else the domain is the tree search's whatever is asked
+            sweep_ms = ms
+    for _ in range(rounds if sweep_ms > ENOUGH * best_ms else 0):
         changed = False
         for knob, values in grid.items():
             for v in values:
                 if v == cur[knob]:
                     continue
                 cand = dict(cur, **{knob: v})
-                ms = _time(inputs, args, cells, cand, reps, stream)
+                ms, _ = _time(inputs, args, cells, cand, reps, stream)
                 trials += 1
                 if ms < best_ms * 0.995:
                     best_ms, cur, changed = ms, cand, True
         if not changed:
             break
+    if sweep_ms <= best_ms:
+        best_ms, cur = sweep_ms, dict(DEFAULTS)
     result = dict(cur, ms_sample=best_ms, trials=trials, sample_cells=n)
     if use_cache:
         with _lock:
