@@ -540,13 +540,14 @@ int resident_lanes(long long* lanes) {
 // Searches of more items than this many times the resident lanes queue the
 // border cells of each domain first (run_batch).
 constexpr long long kBorderFirstWaves = 4;
-// Sweep items per resident lane that a call aims at: a run's first azimuth
+// Sweep items that a call aims at, in multiples of resident_lanes (1024 threads per SM: the
+// sweep keeps 768 of them, 640 in FP64 ray mode): a run's first azimuth
 // costs half an azimuth more, long runs leave lanes idle at the end. Half as many
 // where runs then still hold kTailAzimuths and the tail's are split (194k cells in
 // FP64 ray mode 6.65 -> 6.33 ms; 57k cells, runs of two azimuths, given starts: whole
 // call 1.38, with four 1.42).
 constexpr long long kSweepWaves = 4;
-// The last cells of the queue, one item per lane, go in up to kTailSplit times
+// The last cells of the queue, resident_lanes items, go in up to kTailSplit times
 // as many runs of at least kTailAzimuths: the lanes finish together (194k cells x
 // 240 azimuths 41.4 -> 40.1 ms, 1.2M cells 42.6 -> 41.9; with the runs of two
 // azimuths 21k cells x 360 lost 4 %).

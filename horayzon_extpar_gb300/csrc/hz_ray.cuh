@@ -322,7 +322,7 @@ __device__ __forceinline__ int domain_of_item(const DomainDesc* __restrict__ dom
 // Shared memory is carved out of the SM's 256 KB of L1: ask for just what
 // `resident` blocks need, so the rest caches the tree.
 template <typename K>
-inline void prefer_l1(K kernel, int resident, size_t dynamic = 0) {
+inline void prefer_l1(K kernel, int resident) {
 #if HZ_CARVEOUT
   cudaFuncAttributes fa;
   int dev = 0, smem_sm = 0, reserved = 0;
@@ -335,7 +335,7 @@ inline void prefer_l1(K kernel, int resident, size_t dynamic = 0) {
     (void)cudaGetLastError();
     return;
   }
-  const long long need = (long long)resident * ((long long)fa.sharedSizeBytes + (long long)dynamic + reserved);
+  const long long need = (long long)resident * ((long long)fa.sharedSizeBytes + reserved);
   const int pct = (int)std::min<long long>(100, (need * 100 + smem_sm - 1) / smem_sm);
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct) !=
       cudaSuccess)

@@ -270,7 +270,8 @@ __global__ void k_grid_setup(const unsigned* __restrict__ b, int n_tri, long lon
 
 // Index of cell (a, b) of level l (even; a = i >> l of level 0's i): a level is
 // stored in bricks of 4 x 4 cells, the children of one cell of the level
-// above, so that a walk reads 16 neighbours with one 32-byte access; level l
+// above, so that 16 neighbours' planes are one 128-byte line (their level bounds
+// 32 bytes); level l
 // begins at n2 - (n2 >> l / 2), n2 twice the cells of level 0.
 __device__ __forceinline__ int grid_index(int W, int n2, int a, int b, int l) {
   return n2 - (n2 >> (l >> 1)) + ((((b >> 2) * (W >> (l + 2)) + (a >> 2)) << 4) | ((b & 3) << 2) |
@@ -1160,7 +1161,6 @@ __global__ void __launch_bounds__(kSweepBlock, kPrecise ? HZ_SWEEP_MIN_BLOCKS_EX
             const int dom = domain_of_item(doms, ndom, item);
             const DomainDesc& D = doms[dom];
             const unsigned local = (unsigned)(item - D.item_begin);
-            // Quotient from FP32, off by one at most (fewer runs than 2^20).
             // Run by run over the cells; then over those of the tail.
             const unsigned whole = (unsigned)D.tail_begin * (unsigned)D.runs;
             const bool tail = local >= whole;

@@ -143,9 +143,11 @@ def horizon_svf_comp_py(clon, clat, hsurf, vlon, vlat, cells_of_vertex, num_hori
     extras: CUDA ``device``, work counters, the downward-walk bound, a cell
     range ``cells=(begin, end)`` to trace (entries outside it are NaN), the
     search ``kernel`` (0 persistent: the profile sweep, or the search on the
-    4-wide BVH where one of the following knobs or ``count_work`` asks for it;
-    1 one thread per cell, 2 the persistent search on the binary BVH), its
-    ``advance_min`` / ``leaf_min`` knobs, the work-queue ``queue_chunk``, the BVH ``leaf_size``,
+    4-wide BVH where one of the following knobs or ``count_work`` asks for it or
+    the sweep cannot run or is slower; 1 one thread per cell, 2 the persistent
+    search on the binary BVH; ``stats["search"]`` names what ran), its
+    ``advance_min`` / ``leaf_min`` knobs, the work-queue ``queue_chunk``, the BVH
+    ``leaf_size`` (these select the tree search by any value but 0),
     ``direct_launch`` (launch each kernel directly instead of replaying the
     captured CUDA graph of the build and search), ``bvh_treelets``
     (treelet restructuring of the BVH: same results), ``elev_walk`` (1:
@@ -333,14 +335,15 @@ def horizon_svf_comp_batch(domains, *, device=-1, count_work=False, elev_floor_d
                            mlp_every_azimuth=False, kernel=0, leaf_min=0, leaf_size=0,
                            queue_chunk=0, direct_launch=False, mlp_azimuth_groups=0,
                            bvh_treelets=False, elev_walk=0, occluder_cache=True):
-    """Many independent domains in one call (one persistent search launch).
+    """Many independent domains in one call.
 
     ``domains``: sequence of ``(inputs, args)`` with ``inputs`` the six arrays
     of :func:`horizon_svf_comp_py` and ``args`` its six scalar arguments
     ``(num_hori, grid_type, dist_search, ray_org_elev, refine_factor,
     svf_type)``; each domain has its own. Returns a list of ``(horizon,
     skyview)`` and, with ``return_stats``, the call statistics plus the
-    per-domain completion latency in ms (from the start of the search).
+    per-domain completion time in ms from the start of the search (small
+    domains first where the call's work is large, see hz_horizon_svf_batch).
     """
     keep, structs, outs = [], [], []
     for inputs, args in domains:

@@ -16,8 +16,8 @@
  * Every entry point except horizon_svf_comp returns a status (HZ_OK = 0) and
  * leaves a message for hz_last_error(). No entry point aborts the process.
  * Calls on one device are serialised by the library; the caller owns all
- * buffers. Internally each call builds the triangle mesh, the LBVH and runs
- * the horizon search on one GPU.
+ * buffers. Internally each call builds the triangle mesh and the search's
+ * structure over it (a regular grid, or an LBVH) and runs the horizon search on one GPU.
  */
 #ifndef HORAYZON_GB300_H
 #define HORAYZON_GB300_H
@@ -56,8 +56,11 @@ typedef struct hz_options {
                                 azimuth), and the tree search with the same results where
                                 an option of the tree is set (count_work, advance_min,
                                 leaf_min, leaf_size, queue_chunk, bvh_treelets, elev_walk,
-                                occluder_cache 0) or the domain is too wide for the
-                                sweep's projection */
+                                occluder_cache 0), where the sweep cannot run (a domain
+                                too wide for its projection, a workspace that does not
+                                fit) and where it is the slower one (origins high over the
+                                terrain, many holes in the mesh, patches far apart);
+                                hz_last_search tells which ran */
     int32_t advance_min;     /* persistent kernel: lanes of a warp that must wait before
                                 the search state advances (1..32; 0 = library default) */
     int32_t precision;       /* HZ_PRECISION_REFERENCE (default) or HZ_PRECISION_LOCAL */
@@ -78,11 +81,12 @@ typedef struct hz_options {
     int32_t leaf_min;        /* persistent kernel: lanes of a warp that must hold a
                                 postponed leaf before a triangle pass (1..32; 0 =
                                 library default) */
-    int32_t leaf_size;       /* most triangles per BVH leaf (1..8; 0 = 2) */
+    int32_t leaf_size;       /* most triangles per BVH leaf (1..8; 0 = 2, the only value
+                                that leaves the choice of the search to the library) */
     int32_t queue_chunk;     /* persistent kernel: consecutive cells (curve order) a
                                 warp takes from the work queue at a time (0 = 32) */
     int32_t direct_launch;   /* 1: launch every kernel directly instead of replaying a
-                                captured CUDA graph of the BVH build and search */
+                                captured CUDA graph of the build and search */
     /* Learned warm start: search items per cell. 0 or 1: one item runs the
        cell's azimuths as the reference's chain, the MLP's proposal starting
        the first one. G > 1 (a divisor of num_hori): G items of num_hori / G
@@ -160,7 +164,7 @@ typedef struct hz_stats {
      * of the call's graph, or the caller's stream when launched directly). */
     double ms_h2d;           /* host->device copies (host entry points) */
     double ms_mesh;          /* mesh assembly + geodetic frames */
-    double ms_bvh;           /* LBVH build */
+    double ms_bvh;           /* build of the sweep's grid, or of the LBVH */
     double ms_trace;         /* learned start if any, frames, search, outputs */
     double ms_d2h;           /* device->host copies (host entry points) */
     double ms_total;         /* whole call, wall clock */
