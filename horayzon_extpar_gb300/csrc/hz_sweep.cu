@@ -1632,7 +1632,7 @@ __global__ void __launch_bounds__(128)
   const int n = *list_n;
   for (;;) {
     int w = 0;
-    if (lane == 0) w = atomicAdd(next, 1);
+    if (lane == 0) w = *(volatile int*)err & kErrGrid ? n : atomicAdd(next, 1);
     w = __shfl_sync(kFull, w, 0);
     if (w >= n) return;
     const long long gid = order[list[w]];

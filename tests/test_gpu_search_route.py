@@ -225,3 +225,14 @@ def test_vertices_that_join_far_cells_run_the_tree_at_once():
                                                     "ms_d2h"))
 
     assert min(lost() for _ in range(3)) < 10.0
+
+
+def test_occluder_cache_of_the_tree_search_in_a_batch():
+    """Both settings on the 4-wide tree (the default with the cache on is the sweep)."""
+    doms = [(d.inputs(), a) for d, a in synthetic.make_batch(n_domains=3, seed=5, min_cells=300,
+                                                             max_cells=3000)]
+    off, st0 = horizon_svf_comp_batch(doms, leaf_size=2, occluder_cache=False, return_stats=True)
+    on, st1 = horizon_svf_comp_batch(doms, leaf_size=2, return_stats=True)
+    assert st0["search"] == st1["search"] == "tree" and st0["num_rays"] == st1["num_rays"]
+    assert all(np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+               for a, b in zip(off, on))
