@@ -540,25 +540,25 @@ int resident_lanes(long long* lanes) {
 // Searches of more items than this many times the resident lanes queue the
 // border cells of each domain first (run_batch).
 constexpr long long kBorderFirstWaves = 4;
-// Sweep items that a call aims at, in multiples of resident_lanes (1024 threads per SM: the
-// sweep keeps 768 of them, 640 in FP64 ray mode): a run's first azimuth
-// costs half an azimuth more, long runs leave lanes idle at the end. Half as many
-// where runs then still hold kTailAzimuths and the tail's are split (194k cells in
-// FP64 ray mode 6.65 -> 6.33 ms; 57k cells, runs of two azimuths, given starts: whole
-// call 1.38, with four 1.42).
+// Sweep items that a call aims at, in multiples of resident_lanes (1024 threads per
+// SM: the sweep keeps 768 of them, 640 in FP64 ray mode): a run's first azimuth costs
+// half an azimuth more, long runs leave lanes idle at the end. Half as many where runs
+// then still hold kTailAzimuths and the tail's are split (194k cells in FP64 ray mode
+// 6.65 -> 6.33 ms; 57k cells, runs of two azimuths, given starts: whole call 1.38,
+// with four 1.42).
 constexpr long long kSweepWaves = 4;
 // The last cells of the queue, resident_lanes items, go in up to kTailSplit times
 // as many runs of at least kTailAzimuths: the lanes finish together (194k cells x
 // 240 azimuths 41.4 -> 40.1 ms, 1.2M cells 42.6 -> 41.9; with the runs of two
 // azimuths 21k cells x 360 lost 4 %).
 constexpr int kTailSplit = 4, kTailAzimuths = 4;
-// A domain is done when the repair and the outputs of its group are: all
-// domains of a call together, unless they go in groups, one after another. A group
-// more costs 0.2 to 0.9 ms (idle lanes at its end, its repair), so that they are made where little
-// is lost: a quarter of the work each in calls of kGroupWork evaluations (64 domains, 206M:
-// 136.9 -> 137.3 ms, half of the domains done after 36 ms; 14 domains, 13M: 11.3 -> 13.3, not cut), and
-// before a domain of kGroupGap times the work of all before it (a small domain beside
-// one of 6.9M: 8.3 -> 8.7 ms, the small one done after 0.5).
+// A domain is done when the repair and the outputs of its group are: all domains of
+// a call together, unless they go in groups, one after another. A group more costs
+// 0.2 to 0.9 ms (idle lanes at its end, its repair), so that they are made where
+// little is lost: a quarter of the work each in calls of kGroupWork evaluations (64
+// domains, 206M: 136.9 -> 137.3 ms, half of the domains done after 36 ms; 14 domains,
+// 13M: 11.3 -> 13.3, not cut), and before a domain of kGroupGap times the work of all
+// before it (a small domain beside one of 6.9M: 8.3 -> 8.7 ms, the small one done after 0.5).
 constexpr double kGroupWork = 6e7, kGroupGap = 16.0, kGroupRest = 4e6;
 
 // Runs the pipeline for n domains whose arrays are device pointers in pr[].
@@ -1207,8 +1207,8 @@ int azimuth_groups(const hz_domain* doms, int n, const hz_options& opt, int* gro
 
 // Whether a call runs the profile sweep (hz_sweep.cu) rather than the tree
 // search; the results are the same. From origins near the ground it is the faster
-// one at every spacing and azimuth count measured, from 500 cells (0.63 against 5.2 ms)
-// to 3.1M (63 against 132 ms). The tree search keeps what belongs to it: its own
+// one at every spacing and azimuth count measured, from 500 cells (0.64 against 5.2 ms)
+// to 3.1M (61 against 132 ms). The tree search keeps what belongs to it: its own
 // kernels and knobs, work counters (they count its visits), the bisected walk (a ray
 // sequence of its own); searches whose floor lies below 88 deg or whose result codes
 // (2 bytes per cell and azimuth) would not fit beside the outputs; and high origins.
@@ -1216,12 +1216,12 @@ constexpr long long kMaxCodeBytes = 16ll << 30;
 
 // From an origin high over the terrain the rays around the horizon end in mid-air,
 // with terrain below and beyond: azimuth after azimuth goes to the sweep's repair, a
-// warp per cell. Times of the tree over those of the sweep (radii of 1 to 500 km, spacings of 0.2
-// to 10 km, 24 azimuths), by origin height over search radius: 11,000 to 480,000 cells 1.1
-// to 5.0 at 0.02, 0.97 to 4.8 at 0.03, 0.1 to 2.3 at 0.1, 0.05 to 2.2 at 0.3; at 500 km the
-// line lies at 5 km instead (1.3 to 7 there, 0.8 to 6 at 10 km). Up to 4,000 cells, where the
-// tree search waits for its slowest cells, 1.1 to 7.7 up to 0.1 at radii to 40 km, and
-// 0.8 to 1.5 beyond it from origins above 5 km.
+// warp per cell. Times of the tree over those of the sweep (radii of 1 to 500 km,
+// spacings of 0.2 to 10 km, 24 azimuths), by origin height over search radius: 11,000 to
+// 480,000 cells 1.1 to 5.0 at 0.02, 0.97 to 4.8 at 0.03, 0.1 to 2.3 at 0.1, 0.05 to 2.2 at
+// 0.3; at 500 km the line lies at 5 km instead (1.3 to 7 there, 0.8 to 6 at 10 km). Up to
+// 4,000 cells, where the tree search waits for its slowest cells, 1.1 to 7.7 up to 0.1 at
+// radii to 40 km, and 0.8 to 1.5 beyond it from origins above 5 km.
 constexpr double kHighOrigin = 0.03, kHighMetres = 5000.0, kHighSmall = 0.1;
 constexpr long long kSmallCells = 8192;
 

@@ -41,12 +41,12 @@
 // Against the tree search (GB300, whole call): one traversal of a bounding
 // volume tree per ray took 2.5 to 4 rays, 63 to 126 four-wide node visits and 38
 // to 76 triangle tests per evaluation; the sweep takes 40 to 66 eight-byte steps and
-// 15 to 23 tests. 500 m, 3.1M cells 132 -> 62 ms; 100 m, 1.2M cells 117 -> 39.9 ms; 2.5 km,
-// 57k cells 7.6 -> 1.36 ms; 500 cells 5.4 -> 0.7 ms; 360 azimuths, 21k cells 55.7 -> 9.7 ms.
+// 15 to 23 tests. 500 m, 3.1M cells 132 -> 60.7 ms; 100 m, 1.2M cells 117 -> 39.2 ms; 2.5 km,
+// 57k cells 7.7 -> 1.38 ms; 500 cells 5.2 -> 0.64 ms; 360 azimuths, 21k cells 56.0 -> 10.0 ms.
 // The small domains gain most: a sweep from a low start needs no other azimuth's
 // result, so a cell's azimuths run side by side.
 //
-// What bounds it: instruction issue (62 % of the cycles at 17.8 of 32 lanes, 640 warp
+// What bounds it: instruction issue (63 % of the cycles at 18.0 of 32 lanes, 640 warp
 // instructions per evaluation) and L1/L2 latency with 24 resident warps per SM; DRAM
 // is idle (0.7 %).
 #include <cuda_fp16.h>
@@ -124,7 +124,7 @@ __device__ __forceinline__ float height_magic(unsigned h16) {
 // ---------------------------------------------------------------------------
 // Grid build
 // ---------------------------------------------------------------------------
-// 9.4M triangles, ms: k_gnomonic 0.13, k_grid_count 0.37, k_grid_fill 0.60 (a scattered
+// 9.4M triangles, ms: k_gnomonic 0.15, k_grid_count 0.47, k_grid_fill 0.63 (a scattered
 // atomic and an 8-byte store per list entry, 4.8 a triangle), k_grid_heights 0.55
 // (scattered vertex reads), k_grid_up 0.13; the tree build that this replaces
 // took 2.4 in all.
@@ -182,7 +182,8 @@ constexpr float kHolesCall = 6000.f, kHolesCells = 90.f, kHolesSize = 190.f;
 enum : int { kErrHoles = 4, kErrHolesDomains = 5 };
 
 // ICON vertices of each cell with all their cells.
-__global__ void k_full_vertices(const int* __restrict__ cov, int nvert, uint32_t* __restrict__ full) {
+__global__ void k_full_vertices(const int* __restrict__ cov, int nvert,
+                                uint32_t* __restrict__ full) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= nvert) return;
   int c[6];
@@ -202,8 +203,8 @@ __global__ void k_edge_cells(const uint32_t* __restrict__ full, int begin, int c
 // Grid geometry: cells of HZ_CELL_TRIS times the mean triangle area. missing:
 // vertices missing beside the cells that are searched.
 __global__ void k_grid_setup(const unsigned* __restrict__ b, int n_tri, long long cap0, float tfar,
-                             float org_elev, float cells, float missing, const int* __restrict__ edge,
-                             int ndom, GridDesc* __restrict__ g, int* __restrict__ err) {
+                             float org_elev, float cells, float missing,
+                             const int* __restrict__ edge, int ndom, GridDesc* __restrict__ g, int* __restrict__ err) {
   GridDesc q;
   const float x0 = ord2f(b[0]), y0 = ord2f(b[1]), h0 = ord2f(b[2]), z0 = ord2f(b[3]);
   const float x1 = ord2f(b[4]), y1 = ord2f(b[5]), h1 = ord2f(b[6]);
@@ -271,8 +272,7 @@ __global__ void k_grid_setup(const unsigned* __restrict__ b, int n_tri, long lon
 // Index of cell (a, b) of level l (even; a = i >> l of level 0's i): a level is
 // stored in bricks of 4 x 4 cells, the children of one cell of the level
 // above, so that 16 neighbours' planes are one 128-byte line (their level bounds
-// 32 bytes); level l
-// begins at n2 - (n2 >> l / 2), n2 twice the cells of level 0.
+// 32 bytes); level l begins at n2 - (n2 >> l / 2), n2 twice the cells of level 0.
 __device__ __forceinline__ int grid_index(int W, int n2, int a, int b, int l) {
   return n2 - (n2 >> (l >> 1)) + ((((b >> 2) * (W >> (l + 2)) + (a >> 2)) << 4) | ((b & 3) << 2) |
                                   (a & 3));
@@ -575,7 +575,8 @@ __global__ void k_grid_up(const GridDesc* __restrict__ gd, int l, long long cap0
   if (k >= (long long)w * h) return;
   const int b = (int)(k / w), a = (int)(k - (long long)b * w);
   const int from = grid_index(W, n2, 4 * a, 4 * b, l - 2), to = grid_index(W, n2, a, b, l);
-  if (!check_ok(from >= 0 && from + 16 <= 2 * cap0 && to >= 0 && to < 2 * cap0, kCheckGrid, to, err))
+  if (!check_ok(from >= 0 && from + 16 <= 2 * cap0 && to >= 0 && to < 2 * cap0, kCheckGrid, to,
+                err))
     return;
   const float size = g.c * (float)(1 << (l - 2));  // of a child
   unsigned hi = 0u, lo = 0xFFFFu;
