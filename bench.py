@@ -505,7 +505,7 @@ def drop_in_report(dom, steps):
 
 
 def batch_report(args, mlp_params=None):
-    """64 uneven independent domains in one call (one persistent search);
+    """64 uneven independent domains in one call;
     with mlp_params also the same batch with the learned start (the
     library's choice of azimuth groups)."""
     from horayzon_extpar_gb300 import synthetic
